@@ -12,6 +12,7 @@
 // synchronisation.  A device-resident batch of small jobs is captured as a
 // CUDA graph and replayed when the same batch comes again.
 #include <algorithm>
+#include <cmath>
 #include <numeric>
 #include <vector>
 
@@ -55,6 +56,11 @@ int plan_batch(int sm_count, int njobs, const siting_params *params, const sitin
   std::vector<Job> &jobs = bp->jobs;
   jobs.assign(njobs, Job{});
   size_t ws = 0, tab_bytes = 0;
+  // small jobs' VIX tiles share a grid (run_batch merges waves of up to 2^18
+  // cells a job), whose tile size is chosen for all of their cells
+  double cells = 0;
+  for (int j = 0; j < njobs; j++) cells += (double)params[j].nrows * params[j].nrows;
+  const bool shared_grid = cells <= njobs * 262144.0;
   for (int j = 0; j < njobs; j++) {
     Job &J = jobs[j];
     J.p = params[j];
@@ -67,7 +73,8 @@ int plan_batch(int sm_count, int njobs, const siting_params *params, const sitin
     J.nwpr = (J.nr + 63) / 64;
     J.per = (size_t)J.nr * J.nwpr;
     const siting_plan *pl = plans ? &plans[j] : nullptr;
-    J.vp = vix_plan_for(J.n, J.p.roi, J.p.ntests, pl ? pl->vix_tile : 0, pl ? pl->vix_smem : -1);
+    const int grid_rows = shared_grid ? (int)std::min(std::sqrt(cells), 20000.0) : J.n;
+    J.vp = vix_plan_for(grid_rows, J.p.roi, J.p.ntests, pl ? pl->vix_tile : 0, pl ? pl->vix_smem : -1);
     J.sp = shed_plan_for(J.p.roi, pl ? pl->shed_smem : -1);
     J.G = (pl && pl->site_ctas > 0) ? std::min(pl->site_ctas, sm_count)
                                      : batch_site_ctas(J.g.nwanted, sm_count);

@@ -63,6 +63,12 @@ __device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsig
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+// Each half rounded toward zero.
+__device__ __forceinline__ unsigned long long f2_add_rz(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 // copysign(pred(0.5), v): the addend of round_i for v's sign
 __device__ __forceinline__ float round_addend(float v) {
   return __uint_as_float((__float_as_uint(v) & 0x80000000u) | 0x3effffffu);

@@ -34,7 +34,7 @@ bool make_dem_tensor_map(CUtensorMap *map, const DemView &dem, int box_w, int bo
 struct VixPlan {
   int tile;       // cells per tile side
   int threads;    // threads per CTA
-  bool use_smem;  // stage the halo tile in shared memory by TMA
+  bool use_smem;  // stage the whole halo by TMA (else the cells within 64 of the tile)
 };
 // Device tables of the VIX stage (host-computed with the reference's
 // expressions): jump[2k], jump[2k+1] = LCG multiplier/increment of k+1 steps

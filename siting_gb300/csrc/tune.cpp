@@ -77,7 +77,7 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
   int *err = static_cast<int *>(d_err);
 
   siting_plan out{0, -1, -1, 0};
-  // VIX: tile 16/32/64, halo staged or read through L1 (plans the kernel
+  // VIX: tile 16/32/64, whole halo or near window staged (plans the kernel
   // cannot take are mapped to the nearest one it can, then deduplicated)
   std::vector<VixPlan> seen;
   float bt = 1e30f;

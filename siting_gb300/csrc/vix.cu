@@ -5,21 +5,32 @@
 // major axis) rises above the sight line.  VIX = min(255, (int)(nvis/ntests *
 // 255.999f)).
 //
-// GB300 mapping: one CTA per T x T cell tile.  The tile's halo (T+2roi rows,
-// T+2roi+7 columns rounded to 8) is loaded into shared memory by TMA
-// bulk-tensor copies, so every line-of-sight sample is a shared-memory gather.
-// Each thread keeps one cell per pass and takes every L-th of its targets
-// (L threads a cell); the target of item (cell, t) comes from the LCG state
-// after 2t+1 steps from the seed, obtained by an affine jump-ahead table
-// instead of a serial chain.  Per-cell hit counts accumulate in shared memory
-// and become VIX bytes through a host-computed table.  When the halo does not
-// fit in shared memory (large roi) the same code reads the DEM through the
-// read-only L1 path instead.
+// GB300 mapping: one CTA per T x T cell tile.  A window of the DEM around the
+// tile is loaded into shared memory by TMA bulk-tensor copies: the whole halo
+// (T+2roi rows) while it fits, so that every line-of-sight sample is a
+// shared-memory gather, else (large roi) the cells within 64 of the tile, which
+// hold the samples at offsets 1..64, and the target itself and the samples at
+// offsets 128, 256, ... are read through L1.  Each thread keeps one cell per
+// pass and takes every L-th of its targets (L threads a cell); the target of
+// item (cell, t) comes from the LCG state after 2t+1 steps from the seed,
+// obtained by an affine jump-ahead table instead of a serial chain.  The counts
+// become VIX bytes through a host-computed table.
 //
-// Bit-exactness: every FP32 operation is separately rounded (no FMA), the
-// reference's drecip = (float)(1.0/d) comes from a host table, and C's
-// truncating integer division and round-half-away-from-zero are kept.
+// Bound by instruction issue (92-95% of the slots at roi 100).  2048^2, roi
+// 100, 100 targets: 157 -> 139 thread instructions a target and 1.894 -> 1.473
+// ms (285 G targets/s) with offsets as magnitudes whose signs go with the
+// strides (one rounding addend, no sign handling a sample), the samples unrolled
+// with one FMA for each scaled sum, the draws doubled modulo 2^32, and 32x32
+// instead of 16x16 tiles now that no per-cell table shares the window's memory.
+// roi 200, 64 targets: all samples through L1 1.688 ms, the near window staged
+// 1.262 ms.
+//
+// Bit-exactness: every FP32 operation rounds once where the reference's does (an
+// FMA only where its product is exact), the reference's drecip = (float)(1.0/d)
+// comes from a host table, and C's truncating integer division and
+// round-half-away-from-zero are kept.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -27,11 +38,15 @@
 namespace siting {
 namespace {
 
+// Staged samples of the far form.
+constexpr int kFarNear = 7;
+
 struct VixArgs {
   const uint16_t *dem;
   int pitch, n, roi, oht, tht, ntests;
   uint8_t *vix;
   int tile, tiles_per_row;
+  int halo;  // cells staged around the tile
   int halo_w, box_rows, nboxes;
   const uint32_t *jump;  // ntests pairs: LCG map of 2t+1 steps
   const float *rtab;     // roi+1
@@ -39,231 +54,254 @@ struct VixArgs {
   int *err;
 };
 
-// DEM accessors by linear offset: `base` is the observer cell's offset, a cell
-// (dx, dy) away is at base + dx*stride + dy.
-struct SmemDem {
-  static constexpr bool kShared = true;
-  const uint16_t *s;
-  int w, x0, y0;
-  __device__ __forceinline__ int base(int x, int y) const { return (x - x0) * w + (y - y0); }
-  __device__ __forceinline__ int stride() const { return w; }
-  __device__ __forceinline__ int at(int o) const { return s[o]; }
-};
+// The staged samples of a sight line, at offsets id = 1, 2, 4, ...: a sample
+// rounds slope*id to the minor offset, forms the sight line's height
+// oz + id*zslope and takes the cell's height above it; the line is clear when
+// the largest of these is not positive (a difference of floats has the exact
+// difference's sign).  A lane whose target is nearer than id keeps the
+// previous sample's difference, which is counted already.  The offset is at
+// least 0 here (signs go with the strides), so adding 2^23 toward zero leaves
+// its floor in the low bits, on an idler pipe than a conversion's; the strides'
+// share of 2^23's own bits is taken out of the base address.  Scaling by a power
+// of two is exact, so one FMA rounds once, as the reference's sum with the
+// scaled product does.  Written as one asm statement for its predicated
+// subtraction: as comparisons combined in a predicate the compiler spends 13
+// instructions a sample instead of 10.
+#define VIX_SAMPLE(D, ID, FID)            \
+  "setp.gt.s32 p, %1, " ID ";\n\t"       \
+  "fma.rn.f32 f, %2, " FID ", %5;\n\t"   \
+  "fma.rn.f32 h, %3, " FID ", %4;\n\t"   \
+  "add.rz.f32 f, f, 0f4B000000;\n\t"    \
+  "mov.b32 o, f;\n\t"                   \
+  "mad.lo.s32 t, %7, " ID ", z;\n\t"    \
+  "mad.lo.s32 t, o, %8, t;\n\t"         \
+  "@p ld.shared.u16 e, [t];\n\t"        \
+  "cvt.rn.f32.s32 g, e;\n\t"            \
+  "@p sub.rn.f32 " D ", g, h;\n\t"
+#define VIX_MAX "max.f32 m, m, d0, d1;\n\t"
+#define VIX_SAMPLES(BODY)                                                           \
+  asm("{\n\t.reg .pred p;\n\t.reg .f32 f, h, g, m, d0, d1;\n\t.reg .s32 o, t, e, z;\n\t" \
+      "mad.lo.s32 z, %8, 0xB5000000, %6;\n\tmov.s32 e, 0;\n\tmov.f32 d0, 0fBF800000;\n\tmov.f32 d1, 0fBF800000;\n\t"      \
+      "mov.f32 m, 0fBF800000;\n\t" BODY "max.f32 %0, m, d0, d1;\n\t}"                 \
+      : "=f"(over)                                                                  \
+      : "r"(ad), "f"(slope), "f"(zslope), "f"(foz), "f"(0x1.fffffep-2f), "r"(ob2), \
+        "r"(smaj), "r"(smin))
+#define VIX_S5                                                                        \
+  VIX_SAMPLE("d0", "1", "0f3F800000") VIX_SAMPLE("d1", "2", "0f40000000") VIX_MAX       \
+  VIX_SAMPLE("d0", "4", "0f40800000") VIX_SAMPLE("d1", "8", "0f41000000") VIX_MAX       \
+  VIX_SAMPLE("d0", "16", "0f41800000")
+#define VIX_S6 VIX_S5 VIX_SAMPLE("d1", "32", "0f42000000")
+#define VIX_S7 VIX_S6 VIX_MAX VIX_SAMPLE("d0", "64", "0f42800000")
+#define VIX_S8 VIX_S7 VIX_SAMPLE("d1", "128", "0f43000000")
 
-struct GlobalDem {
-  static constexpr bool kShared = false;
-  const uint16_t *g;
-  int pitch;
-  __device__ __forceinline__ int base(int x, int y) const { return x * pitch + y; }
-  __device__ __forceinline__ int stride() const { return pitch; }
-  __device__ __forceinline__ int at(int o) const { return __ldg(g + o); }
+template <int kNear>
+__device__ __forceinline__ int near_samples(int ad, float slope, float zslope, float foz,
+                                            uint32_t ob2, int smaj, int smin) {
+  float over;
+  if constexpr (kNear == 5) VIX_SAMPLES(VIX_S5);
+  if constexpr (kNear == 6) VIX_SAMPLES(VIX_S6);
+  if constexpr (kNear == 7) VIX_SAMPLES(VIX_S7);
+  if constexpr (kNear == 8) VIX_SAMPLES(VIX_S8);
+  return !(over > 0.f);
+}
+
+// What a thread keeps of its cell.
+struct VixCell {
+  uint32_t ob2;  // shared-memory byte address of the cell in the window
+  int ctz;       // tht - observer height
+  float foz;     // observer height
+  uint32_t seed;
+  int ox, oy, gbase;  // DEM coordinates and element offset
 };
 
 // One random target of one cell (siting.cpp:155-175 and 54-135).  kInterior:
 // every cell of the tile is at least roi from the DEM edge, so no target can
-// fall outside it and the bounds test is dropped.
-template <bool kInterior, class Dem>
-__device__ __forceinline__ int vix_target(const Dem &dem, int obase, int n, int roi, int roi2,
-                                          int tht, unsigned long long span2, int ox, int oy,
-                                          int oz, float foz, uint32_t r1,
-                                          const unsigned long long *rtab2) {
-  const uint32_t r2 = lcg_step(r1);
+// fall outside it and the bounds test is dropped.  kNear: samples at offsets
+// 1 .. 2^(kNear-1) are read from the staged window.  kFar: the target itself
+// and the samples beyond are read from the DEM through L1.
+template <int kNear, bool kFar, bool kInterior>
+__device__ __forceinline__ int vix_target(const VixArgs &a, const VixCell &c, int W2, int roi2,
+                                          unsigned long long span2, uint2 j, const float *rtab) {
+  // Both draws (siting.cpp:29-33) are carried doubled, modulo 2^32: the
+  // reference's modulus 2^31 then needs no masking, and a float of the doubled
+  // draw is twice the draw's (span arrives scaled by 2^-32).
+  const uint32_t r1 = j.x * c.seed + j.y;
+  const uint32_t r2 = 1103515245u * r1 + 2u * 12345u;
   // (int)((2*roi+0.99999f)*r/RANDOM_MAX): the divisor is 2^31, and scaling
   // by a power of two commutes with rounding (no overflow or underflow
-  // here), so RN(span*r)/2^31 = RN((span*2^-31)*r): span arrives pre-scaled,
-  // paired with itself, and both draws are scaled by one packed multiply.
-  const unsigned long long dd = f2_mul(span2, f2_pack(i2f((int)r1), i2f((int)r2)));
-  int dx = f2i(f2_lo(dd)) - roi;
-  int dy = f2i(f2_hi(dd)) - roi;
-  if (dx * dx + dy * dy > roi2) {  // fold into the circle (siting.cpp:162-166)
-    dx /= 3;
-    dy /= 3;
-  }
-  if (!kInterior &&
-      ((unsigned)(ox + dx) >= (unsigned)n || (unsigned)(oy + dy) >= (unsigned)n))
-    return 0;
-  const int adx = abs(dx), ady = abs(dy);
-  if (adx <= 1 && ady <= 1) return 1;
-  const int W = dem.stride();
-  const int tz = dem.at(obase + dx * W + dy) + tht;
-  const bool mx = adx >= ady;
-  const int d = mx ? dx : dy, m = mx ? dy : dx, ad = mx ? adx : ady;
-  // Sample offsets are id = +-1, 2, 4, ... along the major axis (the sign of
-  // d).  slope*id = m*drecip*id = (m*|drecip|)*|id| exactly (negation and
-  // scaling by a power of two are exact in FP32), likewise id*zslope, so both
-  // are carried by doubling from m*|drecip| and (tz-oz)*|drecip|, bit-identical
-  // to the reference's products.  They travel as one pair P = {slope*|id|,
-  // zslope*|id|}: one packed add doubles both, and one packed add with
-  // C = {copysign(pred(0.5), slope), oz} gives the rounding sum of the minor
-  // offset and the sight-line height oz + id*zslope.  The sample's offset
-  // from the observer is id*(major stride) + round(slope*id)*(minor stride).
-  unsigned long long P = f2_mul(f2_pack(i2f(m), i2f(tz - oz)), rtab2[ad]);  // |drecip|, siting.cpp:91
-  const unsigned long long C = f2_pack(round_addend(f2_lo(P)), foz);  // the sign never changes
-  const int smin = mx ? 1 : W;
-  int q = obase + (mx ? (d > 0 ? W : -W) : (d > 0 ? 1 : -1));  // observer + id*(major stride)
-  if constexpr (Dem::kShared) {
-    // With the halo in shared memory every sample is tested: a blocked
-    // target's lane would idle until its warp's other lanes finish anyway, and
-    // no branch is left for the lanes to diverge on.  (Through L1 the extra
-    // loads cost more than the branch.)
-    bool vis = true;
-    // the sample's shared-memory byte address, doubled about the observer's
-    // (no scaling of an element offset at every sample)
-    const uint32_t sb = smem_u32(dem.s);
-    uint32_t qb = sb + 2u * (uint32_t)q;
-    const uint32_t ob2 = sb + 2u * (uint32_t)obase;
-    const int sminb = 2 * smin;
-    for (int step = 1; step < ad; step <<= 1) {
-      const unsigned long long Q = f2_add(P, C);
-      const int off = f2i(f2_lo(Q));  // round(slope*id), half away from zero
-      unsigned short ev;
-      asm("ld.shared.u16 %0, [%1];" : "=h"(ev) : "r"(qb + off * sminb));
-      vis &= !(i2f(ev) > f2_hi(Q));
-      P = f2_add(P, P);
-      qb = 2u * qb - ob2;  // id doubles
+  // here), so RN(span*r)/2^31 = RN((span*2^-31)*r).  The products are in
+  // [0, 2^23): adding 2^23 toward zero leaves their floor in the low bits.
+  const unsigned long long dd = f2_mul(span2, f2_pack(__uint2float_rn(r1), __uint2float_rn(r2)));
+  const unsigned long long fl = f2_add_rz(dd, f2_pack(8388608.f, 8388608.f));
+  const int dx = __float_as_int(f2_lo(fl)) - (0x4b000000 + a.roi);
+  const int dy = __float_as_int(f2_hi(fl)) - (0x4b000000 + a.roi);
+  const bool fold = dx * dx + dy * dy > roi2;  // fold into the circle (siting.cpp:162-166)
+  unsigned adx = abs(dx), ady = abs(dy);
+  if (kFar) {
+    if (fold) {
+      adx /= 3u;
+      ady /= 3u;
     }
-    return vis;
+  } else {  // |v| / 3 = |v| * 43691 >> 17 for |v| < 2^16 (a staged window's roi is far smaller)
+    const unsigned m = fold ? 43691u : 131072u;
+    adx = (adx * m) >> 17;
+    ady = (ady * m) >> 17;
+  }
+  if (!kInterior) {
+    const int x = c.ox + (dx < 0 ? -(int)adx : (int)adx), y = c.oy + (dy < 0 ? -(int)ady : (int)ady);
+    if ((unsigned)x >= (unsigned)a.n || (unsigned)y >= (unsigned)a.n) return 0;
+  }
+  // From here on offsets are magnitudes and the signs go with the strides:
+  // slope, rounding and products are symmetric about zero.
+  const int sx = dx < 0 ? -W2 : W2, sy = dy < 0 ? -2 : 2;
+  int ev;
+  if constexpr (kFar) {
+    const int gx = dx < 0 ? -(int)adx : (int)adx, gy = dy < 0 ? -(int)ady : (int)ady;
+    ev = __ldg(a.dem + (c.gbase + gx * a.pitch + gy));
   } else {
-    for (int step = 1; step < ad; step <<= 1) {
-      const unsigned long long Q = f2_add(P, C);
-      const int off = f2i(f2_lo(Q));  // round(slope*id), half away from zero
-      if (i2f(dem.at(q + off * smin)) > f2_hi(Q)) return 0;
-      P = f2_add(P, P);
-      q = 2 * q - obase;  // id doubles
-    }
-    return 1;
+    asm("ld.shared.u16 %0, [%1];"
+        : "=r"(ev)
+        : "r"(c.ob2 + (uint32_t)((int)adx * sx) + (uint32_t)((int)ady * sy)));
   }
+  const bool mx = adx >= ady;
+  const int ad = mx ? adx : ady, am = mx ? ady : adx;
+  const int smaj = mx ? sx : sy, smin = mx ? sy : sx;
+  // Sample offsets are id = 1, 2, 4, ... along the major axis.  slope*id =
+  // m*drecip*id = (m*drecip)*id exactly (scaling by a power of two), likewise
+  // id*zslope, so both start from m*|drecip| and (tz-oz)*|drecip| and are
+  // bit-identical to the reference's products (siting.cpp:91).
+  const float r = rtab[ad];
+  const float slope = fmul(i2f(am), r), zslope = fmul(i2f(ev + c.ctz), r);
+  // every staged sample is tested: a blocked target's lane would idle until
+  // its warp's other lanes finish anyway
+  const int vis = near_samples<kNear>(ad, slope, zslope, c.foz, c.ob2, smaj, smin);
+  if constexpr (kFar) {
+    if (ad > (1 << kNear) && vis) {
+      const int P = a.pitch;
+      const int gmaj = mx ? (dx < 0 ? -P : P) : (dy < 0 ? -1 : 1);
+      const int gmin = mx ? (dy < 0 ? -1 : 1) : (dx < 0 ? -P : P);
+      for (int id = 1 << kNear; id < ad; id <<= 1) {
+        const float fid = i2f(id);
+        const float f = __fmaf_rn(slope, fid, 0x1.fffffep-2f);
+        const float h = __fmaf_rn(zslope, fid, c.foz);
+        if (i2f(__ldg(a.dem + (c.gbase + id * gmaj + f2i(f) * gmin))) > h) return 0;
+      }
+    }
+  }
+  return vis;
 }
 
 // The tile's (cell, target) items: L = blockDim/T^2 consecutive threads share
 // a cell (T = 16: 4) and take every L-th of its targets, so a thread keeps one
 // cell for the whole pass (no per-item bookkeeping) and a warp's lanes run the
 // same number of targets; the L partial counts are summed by shuffles.
-template <bool kInterior, class Dem>
-__device__ __forceinline__ void vix_tile_work(const Dem &dem, const VixArgs &a,
-                                              const int4 *cinfo, const uint2 *jump,
-                                              const unsigned long long *rtab2, int *cnt) {
-
-  const int ncell = a.tile * a.tile;
+template <int kNear, bool kFar, bool kInterior>
+__device__ __forceinline__ void vix_tile_work(const VixArgs &a, const uint16_t *halo, int tx0,
+                                              int ty0, int hx0, int hy0, const uint2 *jump,
+                                              const float *rtab, const uint8_t *vtab) {
+  const int T = a.tile, ncell = T * T;
   const int L = max(1, (int)blockDim.x / ncell);  // a power of two: tiles are 16, 32, 64
   const int per_pass = blockDim.x / L;
-  const float span = fmul(fadd(i2f(2 * a.roi), 0.99999f), 0x1p-31f);  // scaled by 2^-31
+  const float span = fmul(fadd(i2f(2 * a.roi), 0.99999f), 0x1p-32f);  // of doubled draws
   const unsigned long long span2 = f2_pack(span, span);
   const int roi2 = a.roi * a.roi;
+  const int W2 = 2 * a.halo_w;
   const int sub = threadIdx.x & (L - 1);
+  const uint32_t win = smem_u32(halo);
   for (int c0 = 0; c0 < ncell; c0 += per_pass) {
     const int cell = c0 + threadIdx.x / L;
+    const int lx = cell / T, ly = cell - lx * T;
+    VixCell c;
+    c.ox = tx0 + lx;
+    c.oy = ty0 + ly;
+    const bool in = cell < ncell && c.ox < a.n && c.oy < a.n;
     int acc = 0;
-    if (cell < ncell) {
-      const int4 ci = cinfo[cell];
-      if (ci.w >= 0) {
-        const int obase = ci.x, oz = ci.y, ox = ci.w >> 16, oy = ci.w & 0xffff;
-        const float foz = i2f(oz);
-        const uint32_t seed = (uint32_t)ci.z;
-        for (int t = sub; t < a.ntests; t += L) {
-          const uint2 j = jump[t];
-          const uint32_t r1 = (j.x * seed + j.y) & 0x7fffffffu;
-          acc += vix_target<kInterior>(dem, obase, a.n, a.roi, roi2, a.tht, span2, ox, oy, oz,
-                                       foz, r1, rtab2);
-        }
-      }
+    if (in) {
+      const int at = (c.ox - hx0) * a.halo_w + (c.oy - hy0);
+      const int oz = halo[at] + a.oht;
+      c.ob2 = win + 2u * (uint32_t)at;
+      c.ctz = a.tht - oz;
+      c.foz = i2f(oz);
+      c.seed = (uint32_t)(c.ox * a.n + c.oy);  // the cell index (siting.cpp:150, r = tid)
+      c.gbase = c.ox * a.pitch + c.oy;
+#pragma unroll 1  // unrolled, the copies crowd the 32 registers (4096^2: 7.24 vs 7.02 ms)
+      for (int t = sub; t < a.ntests; t += L)
+        acc += vix_target<kNear, kFar, kInterior>(a, c, W2, roi2, span2, jump[t], rtab);
     }
     for (int o = 1; o < L; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (sub == 0 && cell < ncell) cnt[cell] = acc;
+    if (in && sub == 0) a.vix[c.ox * a.n + c.oy] = vtab[acc];
   }
 }
 
-// One T x T tile of cells: `map` is the halo's tensor map (kSmem), `tile` the
+// One T x T tile of cells: `map` is the window's tensor map, `tile` the
 // tile's index (row-major over tiles_per_row^2), `sm` the CTA's dynamic
-// shared memory (vix_smem_bytes), `mbar` the halo's mbarrier (shared
+// shared memory (vix_smem_bytes), `mbar` the window's mbarrier (shared
 // memory).  Every thread of the CTA calls it.
-template <bool kSmem>
+template <bool kFar>
 __device__ __forceinline__ void vix_tile(const CUtensorMap *map, const VixArgs &a, int tile,
                                          unsigned char *sm, uint64_t *mbar) {
   const int T = a.tile;
   const int tx0 = (tile / a.tiles_per_row) * T;
   const int ty0 = (tile % a.tiles_per_row) * T;
-  const int hx0 = tx0 - a.roi;
-  const int hy0 = (ty0 - a.roi) & ~7;  // TMA inner coordinate: 16-byte aligned
+  const int hx0 = tx0 - a.halo;
+  const int hy0 = (ty0 - a.halo) & ~7;  // TMA inner coordinate: 16-byte aligned
   size_t off = 0;
   uint16_t *halo = reinterpret_cast<uint16_t *>(sm);
-  const uint32_t halo_bytes = kSmem ? (uint32_t)a.nboxes * a.box_rows * a.halo_w * 2u : 0u;
+  const uint32_t halo_bytes = (uint32_t)a.nboxes * a.box_rows * a.halo_w * 2u;
   off += halo_bytes + 16;  // (the per-tile kernel's mbarrier)
   uint2 *jump = reinterpret_cast<uint2 *>(sm + off);
   off += (size_t)a.ntests * 8;
-  unsigned long long *rtab2 = reinterpret_cast<unsigned long long *>(sm + off);  // {r, r} pairs
-  off += (size_t)(a.roi + 1) * 8;
-  int *cnt = reinterpret_cast<int *>(sm + off);
-  off += (size_t)T * T * 4;
-  off = (off + 15) & ~(size_t)15;
-  int4 *cinfo = reinterpret_cast<int4 *>(sm + off);  // per cell: base, oz, seed, row<<16|col
-  off += (size_t)T * T * 16;
+  float *rtab = reinterpret_cast<float *>(sm + off);
+  off += (size_t)(a.roi + 1) * 4;
   uint8_t *vtab = sm + off;
 
-  if (kSmem && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     mbar_init(mbar, 1);
     mbar_expect_tx(mbar, halo_bytes);
     for (int b = 0; b < a.nboxes; b++)
       tma_load_window(halo + (size_t)b * a.box_rows * a.halo_w, map, hy0, hx0 + b * a.box_rows,
                       mbar);
   }
-  for (int i = threadIdx.x; i < a.ntests; i += blockDim.x)
-    jump[i] = make_uint2(a.jump[2 * i], a.jump[2 * i + 1]);
-  for (int i = threadIdx.x; i <= a.roi; i += blockDim.x) rtab2[i] = f2_pack(a.rtab[i], a.rtab[i]);
+  for (int i = threadIdx.x; i < a.ntests; i += blockDim.x)  // doubled draws (vix_target)
+    jump[i] = make_uint2(2u * a.jump[2 * i], 2u * a.jump[2 * i + 1]);
+  for (int i = threadIdx.x; i <= a.roi; i += blockDim.x) rtab[i] = a.rtab[i];
   for (int i = threadIdx.x; i <= a.ntests; i += blockDim.x) vtab[i] = a.vtab[i];
   __syncthreads();
 
   // targets lie within roi of their cell (after the fold, |dx|,|dy| <= roi)
   const bool interior = tx0 >= a.roi && ty0 >= a.roi && tx0 + T + a.roi <= a.n &&
                         ty0 + T + a.roi <= a.n;
-  // per-cell constants, once per tile (rows and columns are below 2^16)
-  auto fill_cells = [&](const auto &dem) {
-    for (int i = threadIdx.x; i < T * T; i += blockDim.x) {
-      const int x = tx0 + i / T, y = ty0 + i % T;
-      int4 ci = make_int4(0, 0, 0, -1);
-      if (x < a.n && y < a.n) {
-        ci.x = dem.base(x, y);
-        ci.y = dem.at(ci.x) + a.oht;
-        ci.z = x * a.n + y;  // the LCG seed is the cell index (siting.cpp:150, r = tid)
-        ci.w = (x << 16) | y;
-      }
-      cinfo[i] = ci;
-    }
-    __syncthreads();
-  };
-  if (kSmem) {
-    if (!mbar_wait(mbar, 0)) {
-      if (threadIdx.x == 0) atomicOr(a.err, kErrTmaTimeout);
-      return;
-    }
-    const SmemDem dem{halo, a.halo_w, hx0, hy0};
-    fill_cells(dem);
-    if (interior)
-      vix_tile_work<true>(dem, a, cinfo, jump, rtab2, cnt);
-    else
-      vix_tile_work<false>(dem, a, cinfo, jump, rtab2, cnt);
-  } else {
-    const GlobalDem dem{a.dem, a.pitch};
-    fill_cells(dem);
-    if (interior)
-      vix_tile_work<true>(dem, a, cinfo, jump, rtab2, cnt);
-    else
-      vix_tile_work<false>(dem, a, cinfo, jump, rtab2, cnt);
+  if (!mbar_wait(mbar, 0)) {
+    if (threadIdx.x == 0) atomicOr(a.err, kErrTmaTimeout);
+    return;
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < T * T; i += blockDim.x) {
-    const int lx = i / T;
-    const int x = tx0 + lx, y = ty0 + (i - lx * T);
-    if (x < a.n && y < a.n) a.vix[x * a.n + y] = vtab[cnt[i]];
+  auto work = [&](auto near) {
+    constexpr int kNear = decltype(near)::value;
+    if (interior)
+      vix_tile_work<kNear, kFar, true>(a, halo, tx0, ty0, hx0, hy0, jump, rtab, vtab);
+    else
+      vix_tile_work<kNear, kFar, false>(a, halo, tx0, ty0, hx0, hy0, jump, rtab, vtab);
+  };
+  if constexpr (kFar) {
+    work(std::integral_constant<int, kFarNear>());
+  } else {  // the fewest samples that reach offsets below roi
+    if (a.roi <= 32)
+      work(std::integral_constant<int, 5>());
+    else if (a.roi <= 64)
+      work(std::integral_constant<int, 6>());
+    else if (a.roi <= 128)
+      work(std::integral_constant<int, 7>());
+    else
+      work(std::integral_constant<int, 8>());
   }
 }
 
-template <bool kSmem>
-__global__ void __launch_bounds__(1024) vix_kernel(const __grid_constant__ CUtensorMap map,
-                                                  const VixArgs a) {
+template <bool kFar>
+__global__ void __launch_bounds__(1024, 2) vix_kernel(const __grid_constant__ CUtensorMap map,
+                                                     const VixArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
-  const uint32_t halo_bytes = kSmem ? (uint32_t)a.nboxes * a.box_rows * a.halo_w * 2u : 0u;
-  vix_tile<kSmem>(&map, a, blockIdx.x, sm, reinterpret_cast<uint64_t *>(sm + halo_bytes));
+  const uint32_t halo_bytes = (uint32_t)a.nboxes * a.box_rows * a.halo_w * 2u;
+  vix_tile<kFar>(&map, a, blockIdx.x, sm, reinterpret_cast<uint64_t *>(sm + halo_bytes));
 }
 
 // ---- VIX of many jobs in one launch (batched form) ---------------------------
@@ -274,7 +312,7 @@ __global__ void __launch_bounds__(1024) vix_kernel(const __grid_constant__ CUten
 // all threads and is read from the constant bank, as in the one-job kernel.
 
 struct VixQJob {
-  CUtensorMap map;  // halo map of a staged job
+  CUtensorMap map;  // window map
   VixArgs a;
   unsigned first;   // grid index of the job's first tile
 };
@@ -285,10 +323,10 @@ struct VixQTable {
 };
 static_assert(sizeof(VixQTable) <= 32000, "kernel parameters are limited to 32 KB");
 
-// One CTA per (job, tile) item.  kSmem: every job of the launch has its halo
-// staged (else none has): one kernel per staging keeps each within 32
-// registers a thread.
-template <bool kSmem>
+// One CTA per (job, tile) item.  kFar: every job of the launch reads its far
+// targets through L1 (else none does): one kernel per form keeps each within
+// 32 registers a thread.
+template <bool kFar>
 __global__ void __launch_bounds__(1024, 2) vixq_kernel(const __grid_constant__ VixQTable tab) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ __align__(8) uint64_t mbar;
@@ -302,30 +340,49 @@ __global__ void __launch_bounds__(1024, 2) vixq_kernel(const __grid_constant__ V
       hi = mid - 1;
   }
   const VixQJob &J = tab.jobs[lo];
-  vix_tile<kSmem>(&J.map, J.a, (int)(it - J.first), sm, &mbar);
+  vix_tile<kFar>(&J.map, J.a, (int)(it - J.first), sm, &mbar);
 }
 
 int round8(int v) { return (v + 7) & ~7; }
 
+// Samples of the near window of the far form: offsets 1..64, so the window
+// reaches kFarHalo cells around the tile.
+constexpr int kFarHalo = 1 << (kFarNear - 1);
+
+// Two 1024-thread CTAs share an SM when each takes at most half of its 228 KB
+// shared memory (at most 32 registers a thread); the second CTA fills the
+// issue slots that the first leaves while its warps drain at the end of a tile.
+constexpr size_t kVixTwoCtaSmem = 112 * 1024;
+constexpr size_t kVixMaxSmem = 220 * 1024;
+
 struct HaloGeom {
   int w, box_rows, nboxes;
+  size_t bytes() const { return (size_t)nboxes * box_rows * w * 2; }
 };
 
-HaloGeom halo_geom(int tile, int roi) {
-  HaloGeom g;
-  g.w = round8(tile + 2 * roi + 7);
-  const int h = tile + 2 * roi;
-  g.nboxes = (h + 255) / 256;
-  g.box_rows = round8((h + g.nboxes - 1) / g.nboxes);
-  return g;
+// mbarrier, jump table, reciprocals, VIX bytes
+size_t tables_tail_bytes(int roi, int ntests) {
+  return 16 + (size_t)ntests * 8 + (size_t)(roi + 1) * 4 + ntests + 1;
 }
 
-size_t tables_tail_bytes(int tile, int roi, int ntests) {
-  // mbarrier, jump table, reciprocal pairs, counts, then the int4 cell table
-  // (16-byte aligned: the offsets before it are multiples of 4), VIX bytes
-  size_t b = 16 + (size_t)ntests * 8 + (size_t)(roi + 1) * 8 + (size_t)tile * tile * 4;
-  b = (b + 15) & ~(size_t)15;
-  return b + (size_t)tile * tile * 16 + ntests + 1;
+int plan_halo(const VixPlan &p, int roi) { return p.use_smem ? roi : kFarHalo; }
+
+// The window of a tile: its columns start at a multiple of 8 at or before the
+// halo's first (tiles start at multiples of 16).
+HaloGeom halo_geom(const VixPlan &p, int roi, int ntests) {
+  const int halo = plan_halo(p, roi), h = p.tile + 2 * halo;
+  HaloGeom g;
+  g.w = round8(h + (-halo & 7));
+  g.nboxes = (h + 255) / 256;
+  // boxes after the first start on 128 bytes
+  g.box_rows = g.nboxes == 1 ? h : round8((h + g.nboxes - 1) / g.nboxes);
+  // A row pitch of an odd multiple of 4 words starts nearby rows in distinct
+  // banks (2048^2, roi 100: 387 M -> 310 M shared-memory wavefronts), unless
+  // the wider rows cost the second CTA of an SM.
+  HaloGeom o = g;
+  o.w |= 8;
+  const size_t tail = tables_tail_bytes(roi, ntests);
+  return g.bytes() + tail <= kVixTwoCtaSmem && o.bytes() + tail > kVixTwoCtaSmem ? g : o;
 }
 
 }  // namespace
@@ -356,32 +413,24 @@ void vix_fill_tables(void *host_buf, int roi, int ntests) {
 }
 
 size_t vix_smem_bytes(const VixPlan &p, int roi, int ntests) {
-  size_t b = tables_tail_bytes(p.tile, roi, ntests);
-  if (p.use_smem) {
-    const HaloGeom g = halo_geom(p.tile, roi);
-    b += (size_t)g.nboxes * g.box_rows * g.w * 2;
-  }
-  return b;
+  return tables_tail_bytes(roi, ntests) + halo_geom(p, roi, ntests).bytes();
 }
 
-// Two 1024-thread CTAs share an SM when each takes at most half of its 228 KB
-// shared memory (at most 32 registers a thread); the second CTA fills the
-// issue slots that the first leaves while its warps drain at the end of a tile.
-constexpr size_t kVixTwoCtaSmem = 112 * 1024;
-constexpr size_t kVixMaxSmem = 220 * 1024;
-
+// 32x32 tiles (one cell a thread) with the whole halo staged are fastest where
+// two CTAs share an SM, then 16x16 (four threads a cell), whose halo takes
+// longer to load for a quarter of the cells: 2048^2, roi 96, staged 16x16 takes
+// 0.32 ms + 12.2 us a target, 32x32 with the near window alone 0.04 ms + 16.1
+// us, so few targets take the far form.  64x64 tiles (four cells a thread)
+// never won.  A grid of 32x32 tiles that is not two waves of the 152 SMs' CTA
+// pairs leaves SMs idle: 16x16 tiles then (us at 32 and 16, 256^2 roi 20: 23,
+// 15; 400^2 roi 200: 100, 69; 700^2 roi 200: 198, 176; 1000^2 roi 50: 187, 207).
 VixPlan vix_default_plan(int nrows, int roi, int ntests) {
-  (void)nrows;
-  // 32x32 tiles (one cell a thread) are fastest wherever their halo fits two
-  // CTAs per SM, then 16x16 (four threads a cell); else the L1 path, where
-  // the halo costs nothing.  64x64 tiles (four cells a thread) never won.
-  for (int tile : {32, 16}) {
-    VixPlan q{tile, 1024, true};
-    if (vix_smem_bytes(q, roi, ntests) <= kVixTwoCtaSmem) return q;
-  }
-  VixPlan p{32, 1024, false};
-  if (vix_smem_bytes(p, roi, ntests) > kVixMaxSmem) p.tile = 16;
-  return p;
+  const int t32 = (nrows + 31) / 32;
+  const bool few = t32 * t32 < 4 * 152;
+  const VixPlan s32{32, 1024, true}, s16{16, 1024, true};
+  if (!few && vix_smem_bytes(s32, roi, ntests) <= kVixTwoCtaSmem) return s32;
+  if ((few || ntests >= 72) && vix_smem_bytes(s16, roi, ntests) <= kVixTwoCtaSmem) return s16;
+  return VixPlan{few ? 16 : 32, 1024, false};
 }
 
 VixPlan vix_plan_for(int nrows, int roi, int ntests, int tile, int smem) {
@@ -389,9 +438,9 @@ VixPlan vix_plan_for(int nrows, int roi, int ntests, int tile, int smem) {
   if (tile == 16 || tile == 32 || tile == 64) {
     p.tile = tile;
     p.use_smem = smem != 0;
-    const HaloGeom g = halo_geom(tile, roi);
-    if (p.use_smem && (g.w > 2048 || vix_smem_bytes(p, roi, ntests) > kVixMaxSmem)) p.use_smem = false;
-    if (!p.use_smem && vix_smem_bytes(p, roi, ntests) > kVixMaxSmem) p = vix_default_plan(nrows, roi, ntests);
+    if (p.use_smem &&
+        (halo_geom(p, roi, ntests).w > 2048 || vix_smem_bytes(p, roi, ntests) > kVixMaxSmem))
+      p.use_smem = false;
   } else if (smem == 0) {
     p.use_smem = false;
   }
@@ -403,7 +452,9 @@ namespace {
 // Kernel arguments and halo map of one job; false if the map cannot be made.
 bool vix_args(const DemView &dem, int roi, int oht, int tht, int ntests, uint8_t *vix,
               const void *d_tables, const VixPlan &plan, int *d_err, VixArgs *out,
-              CUtensorMap *map, bool *smem) {
+              CUtensorMap *map) {
+  // the radii whose tables of 8 bytes an entry fit a CTA
+  if ((size_t)roi * 8 + (size_t)ntests * 9 + 5200 > 227 * 1024) return false;
   VixArgs a{};
   a.dem = dem.data;
   a.pitch = dem.pitch;
@@ -419,17 +470,13 @@ bool vix_args(const DemView &dem, int roi, int oht, int tht, int ntests, uint8_t
   a.rtab = reinterpret_cast<const float *>(a.jump + 2 * ntests);
   a.vtab = reinterpret_cast<const uint8_t *>(a.rtab + roi + 1);
   a.err = d_err;
-  memset(map, 0, sizeof(*map));
-  *smem = plan.use_smem && dem.tma_ok;
-  if (*smem) {
-    const HaloGeom g = halo_geom(plan.tile, roi);
-    a.halo_w = g.w;
-    a.box_rows = g.box_rows;
-    a.nboxes = g.nboxes;
-    if (!make_dem_tensor_map(map, dem, g.w, g.box_rows)) return false;
-  }
+  a.halo = plan_halo(plan, roi);
+  const HaloGeom g = halo_geom(plan, roi, ntests);
+  a.halo_w = g.w;
+  a.box_rows = g.box_rows;
+  a.nboxes = g.nboxes;
   *out = a;
-  return true;
+  return make_dem_tensor_map(map, dem, g.w, g.box_rows);
 }
 
 }  // namespace
@@ -438,30 +485,19 @@ cudaError_t launch_vix(const DemView &dem, int roi, int oht, int tht, int ntests
                        const void *d_tables, const VixPlan &plan, int *d_err, cudaStream_t st) {
   VixArgs a;
   CUtensorMap map;
-  bool smem;
-  if (!vix_args(dem, roi, oht, tht, ntests, vix, d_tables, plan, d_err, &a, &map, &smem))
+  if (!vix_args(dem, roi, oht, tht, ntests, vix, d_tables, plan, d_err, &a, &map))
     return cudaErrorInvalidValue;
-  VixPlan eff = plan;
-  eff.use_smem = smem;
-  const size_t shm = vix_smem_bytes(eff, roi, ntests);
+  const size_t shm = vix_smem_bytes(plan, roi, ntests);
   const int grid = a.tiles_per_row * a.tiles_per_row;
-  cudaError_t e;
-  if (smem) {
-    e = cudaFuncSetAttribute(vix_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)shm);
-    if (e != cudaSuccess) return e;
-    vix_kernel<true><<<grid, plan.threads, shm, st>>>(map, a);
-  } else {
-    e = cudaFuncSetAttribute(vix_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)shm);
-    if (e != cudaSuccess) return e;
-    vix_kernel<false><<<grid, plan.threads, shm, st>>>(map, a);
-  }
+  auto kern = plan.use_smem ? vix_kernel<false> : vix_kernel<true>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+  if (e != cudaSuccess) return e;
+  kern<<<grid, plan.threads, shm, st>>>(map, a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st) {
-  // jobs whose halo is staged, then those read through L1: one launch for
+  // jobs whose halo is staged, then the far form's: one launch for
   // each kind, at most kStageQueueMaxJobs jobs a launch
   static thread_local VixQTable tab;  // 20 KB: not on the host stack
   for (int kind = 0; kind < 2; kind++) {
@@ -474,20 +510,17 @@ cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st) {
         const StageJob &J = jobs[j];
         VixQJob &q = tab.jobs[tab.njobs];
         memset(&q, 0, sizeof(q));
-        bool smem;
+        if ((J.vplan.use_smem ? 0 : 1) != kind) continue;
         if (!vix_args(J.dem, J.roi, J.oht, J.tht, J.ntests, J.vix, J.vix_tables, J.vplan, J.err,
-                      &q.a, &q.map, &smem))
+                      &q.a, &q.map))
           return cudaErrorInvalidValue;
-        if ((smem ? 0 : 1) != kind) continue;
         q.first = total;
-        VixPlan eff = J.vplan;
-        eff.use_smem = smem;
-        shm = std::max(shm, vix_smem_bytes(eff, J.roi, J.ntests));
+        shm = std::max(shm, vix_smem_bytes(J.vplan, J.roi, J.ntests));
         total += (unsigned)(q.a.tiles_per_row * q.a.tiles_per_row);
         tab.njobs++;
       }
       if (!tab.njobs) continue;
-      auto kern = kind == 0 ? vixq_kernel<true> : vixq_kernel<false>;
+      auto kern = kind == 0 ? vixq_kernel<false> : vixq_kernel<true>;
       cudaError_t e =
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
       if (e != cudaSuccess) return e;
