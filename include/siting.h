@@ -68,10 +68,10 @@ typedef struct siting_plan {
   int vix_tile;     /* VIX cell tile side: 16, 32 or 64 (0 = default) */
   int vix_smem;     /* 1: stage the whole halo by TMA, 0: stage the cells within 64 of
                        the tile and read the rest through L1, -1: default */
-  int shed_smem;    /* VIEWSHED window: 1 two half windows staged by TMA, one
-                       CTA each (up to roi 151, else as 2), 2 the whole window
-                       in one CTA, staged up to roi 100, 0 the whole window
-                       through L1, -1 default (1 for roi 60..151, else 2) */
+  int shed_smem;    /* VIEWSHED window staged by TMA: 1 in halves or quarters, a
+                       CTA each, 2 whole in one CTA (as 1 above roi 111), 0 the
+                       window read through L1, -1 default (2 below roi 75, else
+                       1; both read through L1 where a quarter does not fit) */
   int site_ctas;    /* CTAs of the job's SITE group (0 = default) */
 } siting_plan;
 
@@ -260,8 +260,8 @@ int siting_selftest_wait(siting_ctx *ctx, int which, long long max_cycles);
 
 /* ---- autotuner -----------------------------------------------------------
  * No counterpart in the reference.  Times the launch plans of each stage
- * (VIX tile 16/32/64 with the whole halo or its near part staged; VIEWSHED half
- * windows, the whole window staged, or read through L1; SITE group size when the sample is the whole DEM) on the
+ * (VIX tile 16/32/64 with the whole halo or its near part staged; VIEWSHED
+ * windows staged in parts, whole, or read through L1; SITE group size when the sample is the whole DEM) on the
  * top-left sample_rows x sample_rows corner of the host DEM elevs (0 = 1024)
  * with p's parameters, and keeps the fastest for (roi, ntests) in the
  * context: later calls given no plan (siting_run*, siting_run_batch* with

@@ -37,7 +37,8 @@ __device__ __forceinline__ int round_i(float v) {
 
 // Packed FP32 pairs (low half, high half) for the f32x2 instructions of
 // sm_100 and later: each half is an IEEE round-to-nearest operation of its
-// own, so a packed add or multiply equals two scalar ones bit for bit.
+// own, so a packed add or multiply equals two scalar ones bit for bit.  (Not a
+// multiply that feeds an add.rn: ptxas 13.0 contracts the two, .rn or not.)
 __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
   unsigned long long v;
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
@@ -67,6 +68,13 @@ __device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsig
 __device__ __forceinline__ unsigned long long f2_add_rz(unsigned long long a, unsigned long long b) {
   unsigned long long d;
   asm("add.rz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// a*b + c, each half rounded once.
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
+                                                     unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
 // copysign(pred(0.5), v): the addend of round_i for v's sign
@@ -130,6 +138,22 @@ __device__ __forceinline__ void tma_load_window(void *dst, const CUtensorMap *ma
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y0 >> 3), "r"(x0), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// ---- thread-block clusters ---------------------------------------------------
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Stores to the shared memory of the cluster's CTA `rank`, at this CTA's address `addr`.
+__device__ __forceinline__ void cluster_store_u64(uint32_t addr, uint32_t rank, uint64_t v) {
+  asm volatile(
+      "{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\t"
+      "st.shared::cluster.b64 [r], %2;\n\t}" ::"r"(addr),
+      "r"(rank), "l"(v)
       : "memory");
 }
 

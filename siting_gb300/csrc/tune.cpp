@@ -112,7 +112,8 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
     const ShedPlan sp = shed_plan_for(p->roi, sm);
     bool seen = false;  // the same plan under another setting
     for (const ShedPlan &q : tried)
-      seen |= q.threads == sp.threads && q.use_smem == sp.use_smem && q.half == sp.half;
+      seen |= q.threads == sp.threads && q.use_smem == sp.use_smem && q.half == sp.half &&
+              q.quad == sp.quad;
     if (seen) continue;
     tried.push_back(sp);
     float t;

@@ -8,27 +8,32 @@
 // s = (elev - oalt)/|i| and marks the cell when elev + tht >= oalt + hs*|i|.
 // Bit (row, col) of a shed is word row*nwpr + col/64, bit 63 - col%64.
 //
-// GB300 mapping: one CTA per observer.  The observer's window (2roi+1 rows,
-// 2roi+8 columns from an 8-aligned start) is loaded into shared memory by one
-// TMA bulk-tensor copy; each thread sweeps rays (adjacent threads take
-// adjacent perimeter cells, so a warp's lanes touch neighbouring cells each
-// step and have nearly equal ray lengths).  Visible cells are OR-ed into a
-// shared-memory image of the shed (32-bit halves of the reference's 64-bit
-// words), which is then written to HBM with coalesced stores.  For windows
-// too large for two CTAs per SM the DEM is read through the read-only L1 path.
+// GB300 mapping: a thread sweeps a pair of rays that mirror each other about the
+// observer's column (or a quadrant's diagonal): the rounded minor offset, the step
+// table and the mark's line are the same for both, and the FP32 operations of the
+// two are packed pairs.  The observer's window is loaded into shared memory by TMA
+// bulk-tensor copies, whole, as the halves above and below the observer, or as
+// quarters, one CTA each (shed_staged_plan); windows that do not fit even so are
+// read through L1 by the same code.  Visible cells are marked in a shared-memory
+// image of the shed, which is then written to HBM with coalesced stores.
+//
+// Bound by instruction issue and shared-memory wavefronts alike (75% and 78% of
+// their peaks at roi 100).  2048^2, ms before (one ray a thread) and after: 65536
+// observers of roi 20 0.330, 0.318; roi 30 0.632, 0.454; roi 50 1.523, 1.144;
+// 45511 of roi 60 1.490, 1.016; 16384 of roi 100 1.240, 0.981; 7281 of roi 150
+// 1.314, 1.008; 4096 of roi 200 1.604, 1.138 (1.02-1.2 T ray steps/s).
 //
 // Half windows: every ray to a target row tx <= ox stays in rows ox-roi..ox,
-// every other ray in rows ox..ox+roi, so an observer can also be swept by two
-// CTAs that each stage roi+1 rows (half the bytes: twice the resident CTAs,
-// and windows up to roi ~150 staged).  The upper CTA writes shed rows 0..roi,
-// the lower one rows roi+1..2roi.  Row ox is the upper CTA's: the lower CTA's
-// rays meet it only in a prefix of steps k with round(k*slope) = 0, and such a
-// prefix samples the cells (ox, oy+-k) in the order and at the steps of the
-// straight ray to (ox, oy+-roi) of the upper CTA, with the same horizons, so
-// its marks there are a subset of that ray's.
+// every other ray in rows ox..ox+roi, so the sides can be swept apart.  The
+// observer's row is the upper side's: the lower side's rays meet it only in a
+// prefix of steps k with round(k*slope) = 0, and such a prefix samples the cells
+// (ox, oy+-k) in the order and at the steps of the straight ray to (ox, oy+-roi)
+// of the upper side, with the same horizons, so its marks there are a subset of
+// that ray's.  The same holds for the observer's column, which rows take from the
+// straight rays along it.
 //
 // Bit-exactness: separately rounded FP32 operations, IEEE division for the
-// slopes, round-half-away-from-zero for the minor coordinate.  The horizon
+// slopes (of which the sign goes with the strides, as rounding is symmetric), round-half-away-from-zero for the minor coordinate.  The horizon
 // slope s = RN(a/k) (a an integer elevation difference, k the step) is
 // q0 = RN(a*y), s = RN(q0 + RN(a - k*q0)*y) with y = RN(1/k) from a per-CTA
 // table: one fused correction of a quotient within an ulp, given a correctly
@@ -44,434 +49,635 @@
 namespace siting {
 namespace {
 
-// Word strides of the two shed images (odd, so consecutive rows/columns fall in
-// distinct banks); the column image has 32-column padding for the transpose.
-__host__ __device__ __forceinline__ int shed_row_stride(int nr) {
-  const int w = 2 * ((nr + 63) / 64);  // reference words per row, in halves
-  return w | 1;
+// 32x32 bit transpose: lane j's bit i becomes lane i's bit j.
+__device__ __forceinline__ unsigned warp_transpose(unsigned x, int lane) {
+  // halves and bytes are exchanged by byte permutations, the rest by masks
+  unsigned o = __shfl_xor_sync(0xffffffffu, x, 16);
+  x = __byte_perm(x, o, (lane & 16) ? 0x3276 : 0x5410);
+  o = __shfl_xor_sync(0xffffffffu, x, 8);
+  x = __byte_perm(x, o, (lane & 8) ? 0x3715 : 0x6240);
+#pragma unroll
+  for (int sh = 4; sh >= 1; sh >>= 1) {
+    const unsigned m = sh == 4 ? 0x0F0F0F0Fu : sh == 2 ? 0x33333333u : 0x55555555u;
+    o = __shfl_xor_sync(0xffffffffu, x, sh);
+    x = (lane & sh) ? (x & ~m) | ((o >> sh) & m) : (x & m) | ((o << sh) & ~m);
+  }
+  return x;
 }
-__host__ __device__ __forceinline__ int shed_col_stride(int nr) { return ((nr + 31) / 32) | 1; }
-__host__ __device__ __forceinline__ int shed_col_count(int nr) { return (nr + 31) / 32 * 32; }
 
 struct ShedArgs {
   const uint16_t *dem;
-  int pitch, n, roi, oht, tht, nsheds;
+  int pitch, n, roi, oht, tht;
   const int32_t *obs;
   uint64_t *sheds;
-  int win_w, box_rows, nboxes;
   int *err;
 };
 
-// DEM accessors by linear offset: `base` is the observer cell's offset, a cell
-// (dx, dy) away is at base + dx*stride + dy.
-struct SmemDem {
-  static constexpr bool kShared = true;
-  uint32_t s;  // shared-memory address of the window
-  int w, x0, y0;
-  __device__ __forceinline__ int base(int x, int y) const { return (x - x0) * w + (y - y0); }
-  __device__ __forceinline__ int stride() const { return w; }
-  __device__ __forceinline__ int at(int o) const {
-    unsigned short v;
-    asm("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(s + 2u * (uint32_t)o));
+// One CTA's share of an observer: rows on one side of it (kHalves = 1, block
+// 2o the upper side of observer o, 2o+1 the lower) or all (kHalves = 2).
+//
+// Shared memory: the window, the step table {RN(1/k), RN(1/k), -k, -k} and a pair
+// of bit images for each side.
+// An image has a line per minor offset 0..roi (`ls` words, odd, so that lines
+// start in distinct banks) with a bit per step k-1, the right and the left ray's
+// words interleaved: image X holds the x-major rays (line = column distance, bit
+// = row distance - 1), image Y the y-major ones (line = row distance, bit =
+// column distance - 1).
+__host__ __device__ __forceinline__ int pair_words(int roi) { return (roi + 31) / 32; }
+__host__ __device__ __forceinline__ int pair_line(int roi) { return 2 * pair_words(roi) + 1; }
+// The window's boxes.  A row pitch of an odd multiple of 4 words (the finest that
+// a tensor copy gives) starts 8 successive rows in distinct banks.
+struct WinGeom {
+  int w, box_rows, nboxes;
+  __host__ __device__ size_t bytes() const { return (size_t)nboxes * box_rows * w * 2; }
+};
+
+__host__ __device__ __forceinline__ WinGeom win_geom(int roi, int halves, bool staged) {
+  if (!staged) return WinGeom{0, 0, 0};
+  const int rows = halves == 2 ? 2 * roi + 1 : roi + 1;
+  WinGeom g;
+  g.w = ((2 * roi + 8 + 7) & ~7) | 8;
+  g.nboxes = (rows + 255) / 256;
+  g.box_rows = ((rows + g.nboxes - 1) / g.nboxes + 7) & ~7;  // boxes start on 128 bytes
+  return g;
+}
+
+// The first kNearSteps steps of the rays mark bytes instead of image bits: near
+// the observer many lanes of a warp meet in one cell, whose stores then merge,
+// where atomic ORs would queue up (at step k about roi/k lanes to a cell).  Line =
+// minor offset, byte = step - 1, an odd number of words a line; one such map
+// for each image and side.
+constexpr int kNearSteps = 16;
+constexpr int kNearLine = kNearSteps + 4;  // bytes
+constexpr int kNearMap = (kNearSteps + 1) * kNearLine;
+
+// Words of the images and near maps.
+__host__ __device__ __forceinline__ int pair_mark_words(int roi, int halves) {
+  return halves * (2 * (roi + 1) * pair_line(roi) + kNearMap);  // 4 maps of kNearMap bytes a side
+}
+
+size_t pair_smem_bytes(int roi, int halves, bool staged) {
+  return win_geom(roi, halves, staged).bytes() + (size_t)(roi + 1) * 16 + 16 +
+         (((size_t)pair_mark_words(roi, halves) * 4 + 15) & ~(size_t)15);
+}
+
+// Elevation at `at`: a shared-memory address in the staged window, or an element
+// offset of the DEM read through L1.
+template <bool kStaged>
+__device__ __forceinline__ int elevation(const uint16_t *dem, int at) {
+  if constexpr (kStaged) {
+    int v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(at));
     return v;
+  } else {
+    return __ldg(dem + at);
   }
-};
-
-struct GlobalDem {
-  static constexpr bool kShared = false;
-  const uint16_t *g;
-  int pitch;
-  __device__ __forceinline__ int base(int x, int y) const { return x * pitch + y; }
-  __device__ __forceinline__ int stride() const { return pitch; }
-  __device__ __forceinline__ int at(int o) const { return __ldg(g + o); }
-};
-
-// The shed is assembled in two shared-memory bit images.  Rays that step
-// along y put a warp's lanes on different rows at each step; they mark cells in
-// the row-major image R (word = row*rs + col/32, bit 31 - col%32, i.e. the
-// reference's words split into 32-bit halves, bit col%32 LSB-first; the
-// halves are bit-reversed into the reference's MSB-first order on the way
-// out).  Rays that step along x put the lanes on one row; they mark the
-// column-major image C (word = col*cs + row/32, bit row%32), where their words
-// differ.  rs and cs are odd, so distinct words also fall in distinct banks.
-// C is transposed into R at the end, 32x32 bits per warp.
-struct ShedImage {
-  unsigned *R, *C;
-  int rs, cs;
-};
-
-__device__ __forceinline__ void mark_row_major(const ShedImage &im, int row, int col) {
-  atomicOr(&im.R[row * im.rs + (col >> 5)], 1u << (col & 31));
 }
 
-// Perimeter index of ray t of a half window, in perimeter order: the upper
-// half (0) takes the 4roi+1 targets with tx <= ox, the lower half (1) the
-// other 4roi-1.
-__device__ __forceinline__ int half_ray(int t, int roi, int half) {
-  if (!half) return t + (t <= roi ? 0 : t <= 2 * roi ? roi - 1 : 2 * roi - 1);
-  return t + (t < roi - 1 ? roi + 1 : t < 2 * roi - 1 ? 2 * roi + 1 : 4 * roi + 1);
-}
+constexpr float kNoHorizon = -99999.f;
 
-// Rays of this CTA; the images hold shed rows r0.. (r0 = roi for a lower half).
-template <bool kRcp, bool kHalf, class Dem>
-__device__ __forceinline__ void sweep_rays(const Dem &dem, const ShedArgs &a, int ox, int oy,
-                                           const ShedImage &im, uint32_t rcp, int half) {
-  const int roi = a.roi, n = a.n, side = 2 * roi;
-  const int roi2 = roi * roi;
-  const int xmin = ox - roi, ymin = oy - roi, xmax = ox + roi, ymax = oy + roi;
-  const int W = dem.stride();
-  const int obase = dem.base(ox, oy);
-  const int oalt = dem.at(obase) + a.oht;
-  const float foalt = i2f(oalt), ftht = i2f(a.tht);
-  const int r0 = kHalf && half ? roi : 0;
-  const int nrays = !kHalf ? 4 * side : half ? 4 * roi - 1 : 4 * roi + 1;
-  for (int t = threadIdx.x; t < nrays; t += blockDim.x) {
-    const int ip = kHalf ? half_ray(t, roi, half) : t;
-    int tx, ty;
-    if (ip < side) {
-      tx = xmin + ip;
-      ty = ymin;
-    } else if (ip < 2 * side) {
-      tx = 1 + xmin - side + ip;
-      ty = ymax;
-    } else if (ip < 3 * side) {
-      tx = xmin;
-      ty = 1 + ymin - 2 * side + ip;
+// The steps k..k1 of a pair of rays: A and B are mirror images about the
+// observer's column, so the minor offset, the table entry and the image line
+// are shared and the FP32 operations are packed pairs.
+struct PairRays {
+  const uint16_t *dem;
+  int p0;      // the observer's cell (see elevation())
+  int pA, pB;  // cells of step k-1 at minor offset 0
+  int mA, mB;  // a step along the major axis
+  int sA, sB;  // a step along the minor axis
+  float sl;         // |slope|
+  unsigned long long hs;  // horizons
+  unsigned long long nalt, tht;  // -observer height, target height
+  unsigned long long one;  // 1, from memory
+  uint32_t img;     // image line 0
+  uint32_t near;    // near map line 0 of the right ray; the left one's follows
+  int ls4;          // bytes of an image line
+  const float4 *tab;  // step table
+};
+
+// Steps k..k+3 (k = 1 modulo 4: within one word of the image).  kClamp: a ray's
+// last group, whose steps beyond k1 repeat step k1, which changes nothing.
+template <bool kStaged, bool kRcp, bool kNear, bool kClamp>
+__device__ __forceinline__ void pair_group(PairRays &r, int k, int k1) {
+  float4 t[4];
+  int off[4], ea[4], eb[4], kk[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    kk[i] = kClamp ? min(k + i, k1) : k + i;
+    t[i] = r.tab[kk[i]];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    // round(k*|slope|), half away from zero
+    off[i] = f2i(__fsub_rn(0x1.fffffep-2f, fmul(t[i].z, r.sl)));
+    int cA, cB;  // the step's cells at minor offset 0
+    if constexpr (kClamp) {
+      cA = r.p0 + kk[i] * r.mA;
+      cB = r.p0 + kk[i] * r.mB;
     } else {
-      tx = xmax;
-      ty = ymin - 3 * side + ip;
+      cA = r.pA += r.mA;
+      cB = r.pB += r.mB;
     }
-    if (tx == ox && ty == oy) continue;
-    const int dx = tx - ox, dy = ty - oy;
-    const bool my = abs(dx) < abs(dy);
-    const int dmaj = my ? dy : dx, dmin = my ? dx : dy;
-    const float slope = fdiv(i2f(dmin), i2f(dmaj));
-    const int dir = dmaj > 0 ? 1 : -1;
-    // i*slope = |i| * (dir*slope) exactly (negation is exact), so the minor
-    // offset of step k is round(k * sl).
-    const float sl = dir > 0 ? slope : -slope;
-    const int omaj = my ? oy : ox, omin = my ? ox : oy;
-    // The ray stops at the DEM edge along the major axis (kedge steps), when
-    // the minor coordinate leaves the DEM, or outside the roi circle
-    // (siting.cpp:333-334).  |round(k*sl)| never decreases with k, so the last
-    // two hold from some step on and a binary search finds the last step.
-    int lo = 0, hi = min(dmaj * dir, dir > 0 ? n - 1 - omaj : omaj);
+    ea[i] = elevation<kStaged>(r.dem, cA + off[i] * r.sA);
+    eb[i] = elevation<kStaged>(r.dem, cB + off[i] * r.sB);
+  }
+  const uint32_t mk = r.img + 8u * (uint32_t)((k - 1) >> 5);
+  const unsigned bit0 = 1u << ((k - 1) & 31);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const unsigned long long y = f2_pack(t[i].x, t[i].y), nk = f2_pack(t[i].z, t[i].w);
+    const unsigned long long e = f2_pack(i2f(ea[i]), i2f(eb[i]));
+    // elevations and offsets are integers below 2^24: differences are exact
+    const unsigned long long a = f2_add(e, r.nalt);
+    unsigned long long s;  // RN(a/k)
+    if constexpr (kRcp) {
+      const unsigned long long q = f2_mul(a, y);
+      s = f2_fma(f2_fma(q, nk, a), y, q);
+    } else {
+      s = f2_pack(fdiv(f2_lo(a), -t[i].z), fdiv(f2_hi(a), -t[i].z));
+    }
+    r.hs = f2_pack(fmaxf(f2_lo(r.hs), f2_lo(s)), fmaxf(f2_hi(r.hs), f2_hi(s)));
+    // elev + tht >= oalt + hs*k, the right side carried negated
+    const unsigned long long nv = f2_fma(f2_mul(r.hs, nk), r.one, r.nalt);
+    const unsigned long long v = f2_add(e, r.tht);
+    if constexpr (kNear) {
+      const uint32_t m = r.near + (uint32_t)(off[i] * kNearLine + kk[i] - 1);
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\t@p st.shared.u8 [%0], %3;\n\t}" ::"r"(m),
+                   "f"(f2_lo(v)), "f"(-f2_lo(nv)), "r"(1)
+                   : "memory");
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\t@p st.shared.u8 [%0+%4], %3;\n\t}" ::"r"(m),
+                   "f"(f2_hi(v)), "f"(-f2_hi(nv)), "r"(1), "n"(kNearMap)
+                   : "memory");
+    } else {
+      // an invisible cell ORs nothing: a predicated OR would be a branch, with no
+      // overlap of the steps on either side
+      const uint32_t m = mk + (uint32_t)(off[i] * r.ls4);
+      const unsigned bit = bit0 << (kk[i] - k);
+      asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(m), "r"(f2_lo(v) >= -f2_lo(nv) ? bit : 0u)
+                   : "memory");
+      asm volatile("red.shared.or.b32 [%0+4], %1;" ::"r"(m), "r"(f2_hi(v) >= -f2_hi(nv) ? bit : 0u)
+                   : "memory");
+    }
+  }
+}
+
+// Steps of the two rays of slope sl.  A ray stops outside the roi circle, at
+// the DEM edge along the major axis (maj cells away), or when the minor
+// coordinate leaves the DEM (min cells away) (siting.cpp:333-334); the offset
+// never decreases with k, so each holds from some step on.
+__device__ __forceinline__ void pair_last(float sl, int roi, int majA, int minA, int majB, int minB,
+                                          int &kA, int &kB) {
+  const int roi2 = roi * roi;
+  auto off = [&](int k) { return f2i(fadd(fmul(i2f(k), sl), 0x1.fffffep-2f)); };
+  // the rounded offset moves the circle's crossing by less than a step from the
+  // straight line's, so the search starts just beyond that
+  int kc = min(roi, (int)(i2f(roi) * rsqrtf(1.f + sl * sl)) + 2);
+  for (int o = off(kc); kc * kc + o * o > roi2; o = off(kc)) kc--;
+  auto last = [&](int hi, int lim) {  // the last step <= hi with offset <= lim
+    int lo = 0;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      const int off = round_i(fmul(i2f(mid), sl));
-      if ((unsigned)(omin + off) < (unsigned)n && mid * mid + off * off <= roi2)
+      if (off(mid) <= lim)
         lo = mid;
       else
         hi = mid - 1;
     }
-    const int kend = lo;
-    const int smaj = my ? dir : dir * W, smin = my ? W : 1;
-    // y-major rays mark the row-major image (line = row), x-major rays the
-    // column-major one (line = column); pos is the cell's coordinate along
-    // the ray's axis, bit pos%32 of word line*stride + pos/32
-    const uint32_t img = smem_u32(my ? im.R : im.C);  // shared-memory address
-    const int stride = my ? im.rs : im.cs;
-    // the image line of minor offset 0 and the start's position along the
-    // line, rows counted from r0
-    const int lroi = my ? roi - r0 : roi;
-    int pb = obase, pos = my ? roi : roi - r0;
-    const float fend = i2f(kend);
-    // elevations and offsets are integers below 2^24: their differences and
-    // sums are exact in FP32, so (float)(pelev - oalt) = pelev_f - foalt
-    float hs = -99999.f;
-    if constexpr (kRcp && Dem::kShared) {
-      // the sign of |i|*slope is the slope's: round's addend is fixed per ray
-      const float hsl = round_addend(sl);
-      // The table division costs a few instructions: every step divides and
-      // takes the larger slope (s > hs ? s : hs, the reference's update),
-      // with no branch for the lanes of a warp to diverge on (window in
-      // shared memory; through L1 the extra table read per step costs more).
-      uint32_t rp = rcp + 4u;  // &rcp[|i|]
-      // the cell's shared-memory byte address, advanced by byte strides (no
-      // scaling of an element offset at every step)
-      uint32_t pbb = dem.s + 2u * (uint32_t)obase;
-      const int smajb = 2 * smaj, sminb = 2 * smin;
-#pragma unroll 2  // two steps a trip: half the loop tests and branches
-      for (float fai = 1.f; fai <= fend; fai = fadd(fai, 1.f)) {  // fai = (float)|i|, exact
-        pbb += smajb;
-        pos += dir;
-        const int off = f2i(fadd(fmul(fai, sl), hsl));  // round(|i|*slope), half away from zero
-        unsigned short ev;
-        asm("ld.shared.u16 %0, [%1];" : "=h"(ev) : "r"(pbb + off * sminb));
-        const float fe = i2f(ev);
-        const float fa = __fsub_rn(fe, foalt);
-        float y;
-        asm("ld.shared.f32 %0, [%1];" : "=f"(y) : "r"(rp));
-        rp += 4u;
-        const float q0 = __fmul_rn(fa, y);
-        const float sn = __fmaf_rn(__fmaf_rn(-q0, fai, fa), y, q0);
-        hs = hs < sn ? sn : hs;
-        const float t = fmul(hs, fai);
-        // pelev + tht against oalt + hs*|i|: both sums in one packed add
-        const unsigned long long V = f2_add(f2_pack(fe, foalt), f2_pack(ftht, t));
-        if (f2_lo(V) >= f2_hi(V))
-          asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(img + 4u * (uint32_t)((off + lroi) * stride + (pos >> 5))),
-                       "r"(__funnelshift_l(0u, 1u, pos)) : "memory");  // 1 << (pos & 31)
-      }
-    } else {
-      for (float fai = 1.f; fai <= fend; fai = fadd(fai, 1.f)) {  // fai = (float)|i|, exact
-        pb += smaj;
-        pos += dir;
-        const int off = round_i(fmul(fai, sl));
-        const float fe = i2f(dem.at(pb + off * smin));
-        const float fa = __fsub_rn(fe, foalt);
-        // s = RN(a/|i|) can exceed hs only if a > hs*|i|, and then t = RN(hs*|i|)
-        // <= a (rounding is monotone and a is a float): the division runs only
-        // when the horizon may rise, and t serves the visibility test as well
-        float t = fmul(hs, fai);
-        if (t <= fa) {
-          float sn;
-          if (kRcp) {
-            float y;
-            asm("ld.shared.f32 %0, [%1];" : "=f"(y) : "r"(rcp + 4u * (uint32_t)__float2int_rz(fai)));
-            const float q0 = __fmul_rn(fa, y);
-            sn = __fmaf_rn(__fmaf_rn(-q0, fai, fa), y, q0);
-          } else {
-            sn = fdiv(fa, fai);
-          }
-          if (hs < sn) {
-            hs = sn;
-            t = fmul(hs, fai);
-          }
-        }
-        const unsigned long long V = f2_add(f2_pack(fe, foalt), f2_pack(ftht, t));
-        if (f2_lo(V) >= f2_hi(V))
-          asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(img + 4u * (uint32_t)((off + lroi) * stride + (pos >> 5))),
-                       "r"(1u << (pos & 31)) : "memory");
-      }
-    }
+    return lo;
+  };
+  kA = min(kc, majA);
+  kB = min(kc, majB);
+  if (off(kA) > minA) kA = last(kA, minA);
+  if (off(kB) > minB) kB = last(kB, minB);
+}
+
+// Steps k..k1 (k = 1 modulo 4).
+template <bool kStaged, bool kRcp>
+__device__ __forceinline__ void pair_steps(PairRays &r, int k, int k1) {
+  r.pA = r.p0 + (k - 1) * r.mA;
+  r.pB = r.p0 + (k - 1) * r.mB;
+  for (; k <= kNearSteps && k + 3 <= k1; k += 4) pair_group<kStaged, kRcp, true, false>(r, k, k1);
+  for (; k + 3 <= k1; k += 4) pair_group<kStaged, kRcp, false, false>(r, k, k1);
+  if (k > k1) return;
+  if (k <= kNearSteps)
+    pair_group<kStaged, kRcp, true, true>(r, k, k1);
+  else
+    pair_group<kStaged, kRcp, false, true>(r, k, k1);
+}
+
+// Sweeps A to step kA and B to step kB: first both rays to the nearer end, then,
+// where the ends differ, the longer one alone; the other stays at the observer
+// with its targets out of sight.
+template <bool kStaged, bool kRcp>
+__device__ __forceinline__ void pair_sweep(PairRays &r, int kA, int kB) {
+  const int kmin = min(kA, kB);
+  pair_steps<kStaged, kRcp>(r, 1, kmin);
+  if (kA != kB) {
+    const bool a_on = kA > kB;
+    r.tht = a_on ? f2_pack(f2_lo(r.tht), -3e38f) : f2_pack(-3e38f, f2_hi(r.tht));
+    if (!a_on) r.mA = r.sA = 0;
+    if (a_on) r.mB = r.sB = 0;
+    // from the last group on again: a step done twice changes nothing
+    pair_steps<kStaged, kRcp>(r, (kmin & ~3) + 1, max(kA, kB));
   }
 }
 
-// One observer (whole window) or one half of one (kHalf: block 2o is the
-// upper half of observer o, block 2o+1 the lower).
-template <bool kSmem, bool kRcp, bool kHalf>
-__device__ __forceinline__ void shed_body(const CUtensorMap &map, const ShedArgs &a) {
+// Packs line `line` of a near map to the 16 bits of its steps.
+__device__ __forceinline__ unsigned near_bits(const unsigned char *map, int line) {
+  const unsigned *src = reinterpret_cast<const unsigned *>(map + line * kNearLine);
+  unsigned bits = 0;
+#pragma unroll
+  for (int j = 0; j < kNearSteps / 4; j++)  // four bytes of 0 or 1 to a nibble
+    bits |= (src[j] * 0x01020408u) >> 24 << (4 * j);
+  return bits;
+}
+
+template <int kHalves, bool kStaged, bool kRcp>
+__global__ void __launch_bounds__(448, 2)
+    shed_kernel(const __grid_constant__ CUtensorMap map, const ShedArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
-  const int nr = 2 * a.roi + 1, nwpr = (nr + 63) / 64, nwords = nr * nwpr;
-  const int half = kHalf ? (int)(blockIdx.x & 1u) : 0;
-  const int obi = kHalf ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const int r0 = half * a.roi;          // first shed row of this CTA's images
-  const int nri = kHalf ? a.roi + 1 : nr;  // rows of its images and window
-  // the shed rows this CTA writes: the upper half owns row roi
-  const int wr0 = kHalf && half ? a.roi + 1 : 0, wr1 = kHalf && !half ? a.roi + 1 : nr;
+  const int roi = a.roi, n = a.n, nr = 2 * roi + 1, nwpr = (nr + 63) / 64, nwords = nr * nwpr;
+  const int half0 = kHalves == 1 ? (int)(blockIdx.x & 1u) : 0;
+  const int obi = kHalves == 1 ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+  uint64_t *dst = a.sheds + (size_t)obi * nwords;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  // shed rows this CTA writes: the upper side owns the observer's row
+  const int wr0 = kHalves == 1 && half0 ? roi + 1 : 0, wr1 = kHalves == 1 && !half0 ? roi + 1 : nr;
   const int ob = a.obs[obi];
-  if (ob < 0 || ob >= a.n * a.n) {  // invalid observer: empty shed, flagged
-    uint64_t *dst = a.sheds + (size_t)obi * nwords;
-    for (int i = wr0 * nwpr + threadIdx.x; i < wr1 * nwpr; i += blockDim.x) dst[i] = 0ull;
-    if (threadIdx.x == 0) atomicOr(a.err, kErrBadInput);
+  if (ob < 0 || ob >= n * n) {  // invalid observer: empty shed, flagged
+    for (int i = wr0 * nwpr + tid; i < wr1 * nwpr; i += blockDim.x) dst[i] = 0ull;
+    if (tid == 0) atomicOr(a.err, kErrBadInput);
     return;
   }
-  const int ox = ob / a.n, oy = ob - (ob / a.n) * a.n;
-  const int hx0 = ox - a.roi + r0, hy0 = (oy - a.roi) & ~7;  // window origin, 16-byte aligned
-  uint16_t *win = reinterpret_cast<uint16_t *>(sm);
-  const uint32_t win_bytes = kSmem ? (uint32_t)a.nboxes * a.box_rows * a.win_w * 2u : 0u;
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(sm + win_bytes);
-  ShedImage im;
-  im.rs = shed_row_stride(nr);
-  im.cs = shed_col_stride(nri);
-  im.R = reinterpret_cast<unsigned *>(sm + win_bytes + 16);
-  im.C = im.R + nri * im.rs;
-  const int img_words = nri * im.rs + shed_col_count(nr) * im.cs;
-  float *rcp = reinterpret_cast<float *>(im.R + img_words);  // rcp[k] = RN(1/k)
-  if (kRcp)
-    for (int i = threadIdx.x; i <= a.roi; i += blockDim.x) rcp[i] = i ? __frcp_rn((float)i) : 0.f;
-  if (kSmem && threadIdx.x == 0) {
+  const int ox = ob / n, oy = ob - (ob / n) * n;
+  const WinGeom g = win_geom(roi, kHalves, kStaged);
+  const int W2 = 2 * g.w, nw = pair_words(roi);  // W2: row pitch, bytes
+  const int ls = pair_line(roi), ximg = (roi + 1) * ls;  // words of an image
+  const int hx0 = kHalves == 1 && half0 ? ox : ox - roi;  // window origin
+  const int hy0 = (oy - roi) & ~7;  // TMA inner coordinate: 16-byte aligned
+  const uint32_t win = smem_u32(sm);
+  float4 *tab = reinterpret_cast<float4 *>(sm + g.bytes());
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(tab + roi + 1);
+  unsigned *img = reinterpret_cast<unsigned *>(mbar + 2);
+  unsigned char *near = reinterpret_cast<unsigned char *>(img + kHalves * 2 * ximg);
+  if (kStaged && tid == 0) {
     mbar_init(mbar, 1);
-    mbar_expect_tx(mbar, win_bytes);
-    for (int b = 0; b < a.nboxes; b++)
-      tma_load_window(win + (size_t)b * a.box_rows * a.win_w, &map, hy0, hx0 + b * a.box_rows,
-                      mbar);
+    mbar_expect_tx(mbar, (uint32_t)g.bytes());
+    for (int b = 0; b < g.nboxes; b++)
+      tma_load_window(sm + (size_t)b * g.box_rows * g.w * 2, &map, hy0, hx0 + b * g.box_rows, mbar);
   }
-  for (int i = threadIdx.x; i < img_words; i += blockDim.x) im.R[i] = 0u;
+  for (int i = tid; i <= roi; i += blockDim.x) {
+    const float y = i ? __frcp_rn((float)i) : 0.f;
+    tab[i] = make_float4(y, y, -(float)i, -(float)i);
+  }
+  for (int i = tid; i < (pair_mark_words(roi, kHalves) + 3) / 4; i += blockDim.x)
+    reinterpret_cast<uint4 *>(img)[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
-  if (threadIdx.x == 0 && !half) mark_row_major(im, a.roi, a.roi);  // siting.cpp:279
-  if (kSmem) {
-    if (!mbar_wait(mbar, 0)) {
-      if (threadIdx.x == 0) atomicOr(a.err, kErrTmaTimeout);
-      return;
-    }
-    sweep_rays<kRcp, kHalf>(SmemDem{smem_u32(win), a.win_w, hx0, hy0}, a, ox, oy, im,
-                            smem_u32(rcp), half);
-  } else {
-    sweep_rays<kRcp, kHalf>(GlobalDem{a.dem, a.pitch}, a, ox, oy, im, smem_u32(rcp), half);
+  if (kStaged && !__all_sync(0xffffffffu, mbar_wait(mbar, 0))) {
+    if (tid == 0) atomicOr(a.err, kErrTmaTimeout);
+    return;
+  }
+
+  // ---- rays: roi+1 x-major pairs and then the y-major ones of each side; the
+  // straight y-major ray (minor offset 0) belongs to the upper side
+  const int up = 2 * roi + 1, npairs = kHalves == 2 ? 4 * roi + 1 : half0 ? 2 * roi : up;
+  // (a staged CTA has a thread for every pair: as a loop over pairs, the compiler
+  // lets a warp's rays part at their ends, 15% more instructions)
+  for (int t0 = tid; t0 < npairs; t0 += blockDim.x) {
+    const int half = kHalves == 2 ? t0 >= up : half0;
+    const int t = kHalves == 2 && half ? t0 - up : t0;
+    const bool xm = t <= roi;
+    // adjacent lanes take every second ray of their group: half as many meet in
+    // one image word (2048^2, roi 100: 1.018 -> 0.980 ms; every third 0.992, as the
+    // lengths of a warp's rays then differ more)
+    const int mt = xm ? t : t - (roi + 1), evens = ((xm ? roi + 1 : roi - half) + 1) / 2;
+    const int m = (mt < evens ? 2 * mt : 2 * (mt - evens) + 1) + (xm ? 0 : half);
+    const int rowlim = half ? n - 1 - ox : ox;  // rows on this side of the observer
+    const int collimA = n - 1 - oy, collimB = oy;
+    const float sl = fdiv(i2f(m), i2f(roi));
+    int kA, kB;
+    pair_last(sl, roi, xm ? rowlim : collimA, xm ? collimA : rowlim, xm ? rowlim : collimB,
+              xm ? collimB : rowlim, kA, kB);
+    PairRays r;
+    // strides: bytes of the window, or elements of the DEM
+    const int cell = kStaged ? 2 : 1, rowstep = (half ? 1 : -1) * (kStaged ? W2 : a.pitch);
+    const int p0 = kStaged ? (int)win + (ox - hx0) * W2 + 2 * (oy - hy0) : ox * a.pitch + oy;
+    r.dem = a.dem;
+    r.p0 = p0;
+    r.mA = xm ? rowstep : cell;
+    r.mB = xm ? rowstep : -cell;
+    r.sA = xm ? cell : rowstep;
+    r.sB = xm ? -cell : rowstep;
+    r.sl = sl;
+    const float nalt = -i2f(elevation<kStaged>(a.dem, p0) + a.oht), tht = i2f(a.tht);
+    r.nalt = f2_pack(nalt, nalt);
+    // A product times 1 plus a sum keeps the product's own rounding: ptxas 13.0
+    // contracts mul.rn.f32x2 into an add.rn.f32x2 that it feeds.
+    float one;
+    asm("ld.shared.f32 %0, [%1];" : "=f"(one) : "r"(smem_u32(tab + 1)));  // RN(1/1)
+    r.one = f2_pack(one, one);
+    r.img = smem_u32(img + ((kHalves == 2 && half ? 2 : 0) + (xm ? 0 : 1)) * ximg);
+    r.near = smem_u32(near + ((kHalves == 2 && half ? 2 : 0) + (xm ? 0 : 1)) * 2 * kNearMap);
+    r.ls4 = 4 * ls;
+    r.tab = tab;
+    r.hs = f2_pack(kNoHorizon, kNoHorizon);
+    r.tht = f2_pack(tht, tht);
+    pair_sweep<kStaged, kRcp>(r, kA, kB);
+    if (kStaged) break;
   }
   __syncthreads();
-  // fold C into R: one warp per 32x32 block; lane j holds column cb*32+j's
-  // bits of rows rb*32..+31, a 5-stage butterfly transpose leaves row rb*32+i
-  // in lane i (bit j = column cb*32+j), R's own bit order
-  const int nbr = (nri + 31) / 32, nbc = (nr + 31) / 32;
-  const int lane = threadIdx.x & 31;
-  for (int blk = threadIdx.x >> 5; blk < nbr * nbc; blk += blockDim.x >> 5) {
-    const int rb = blk / nbc, cb = blk - rb * nbc;
-    unsigned x = im.C[(cb * 32 + lane) * im.cs + rb];
+
+  // ---- near maps into the images: a thread packs a line
+  const int nlines = min(roi, kNearSteps) + 1;
+  for (int i = tid; i < kHalves * 4 * nlines; i += blockDim.x) {
+    const int map = i / nlines, line = i - map * nlines;
+    img[(map >> 1) * ximg + line * ls + (map & 1)] |= near_bits(near + map * kNearMap, line);
+  }
+  __syncthreads();
+
+  // ---- X into Y: one warp per 32x32 block; lane j holds column distance
+  // lb*32+1+j's bits of row distances w*32+1.., a 5-stage butterfly transpose
+  // leaves row distance w*32+1+i in lane i (bit j), Y's own order
+  const int nblk = nw * nw * 2;
+  for (int b0 = warp; b0 < kHalves * nblk; b0 += nwarps) {
+    const int hb = kHalves == 2 && b0 >= nblk, b = b0 - hb * nblk;
+    const int side = b & 1, lb = (b >> 1) / nw, w = (b >> 1) - lb * nw;
+    unsigned *X = img + hb * 2 * ximg, *Y = X + ximg;
+    const int line = lb * 32 + 1 + lane;
+    unsigned x = line <= roi ? X[line * ls + 2 * w + side] : 0u;
     if (!__any_sync(0xffffffffu, x != 0u)) continue;
-#pragma unroll
-    for (int sh = 16; sh >= 1; sh >>= 1) {
-      const unsigned m = sh == 16 ? 0x0000FFFFu : sh == 8 ? 0x00FF00FFu : sh == 4 ? 0x0F0F0F0Fu
-                         : sh == 2 ? 0x33333333u : 0x55555555u;
-      const unsigned o = __shfl_xor_sync(0xffffffffu, x, sh);
-      x = (lane & sh) ? (x & ~m) | ((o >> sh) & m) : (x & m) | ((o << sh) & ~m);
-    }
-    const int row = rb * 32 + lane;
-    if (row < nri && x) im.R[row * im.rs + cb] |= x;
+    x = warp_transpose(x, lane);
+    const int d = w * 32 + 1 + lane;
+    if (d <= roi && x) Y[d * ls + 2 * lb + side] |= x;
   }
   __syncthreads();
-  uint64_t *dst = a.sheds + (size_t)obi * nwords;
-  for (int i = wr0 * nwpr + threadIdx.x; i < wr1 * nwpr; i += blockDim.x) {
-    const int r = i / nwpr, q = i - r * nwpr;
-    const unsigned *src = im.R + (r - r0) * im.rs + 2 * q;
-    dst[i] = ((uint64_t)__brev(src[0]) << 32) | __brev(src[1]);
+
+  // ---- rows out.  A row is one number of 64*nwpr bits, column 0 the highest;
+  // the observer's column is bit S, the left string (bit 0 = column distance
+  // 1) starts at S+1 and the right one runs downwards from S-1.
+  // A thread keeps one word column q, so that its string positions are fixed.
+  const int S = 64 * nwpr - 1 - roi;
+  const int per = blockDim.x / nwpr;  // rows a pass (blockDim >= 64 > nwpr)
+  const int q = tid % nwpr, z = 2 * (nwpr - 1 - q);  // bits 32z..32z+63
+  const int l0 = 32 * z - (S + 1), r0 = S - 1 - 32 * z - 31;
+  const int li = l0 >> 5, ri = r0 >> 5, lsh = l0 & 31, rsh = r0 & 31;
+  const bool centre = (S >> 6) == (z >> 1);
+  for (int row = wr0 + tid / nwpr; row < wr1; row += per) {
+    if (tid >= per * nwpr) break;
+    const int d = abs(row - roi), hb = kHalves == 2 && row > roi;
+    const unsigned *X = img + hb * 2 * ximg, *line = X + ximg + d * ls;
+    auto at = [&](const unsigned *w, int i) { return (unsigned)i < (unsigned)nw ? w[2 * i] : 0u; };
+    const unsigned L0 = at(line + 1, li), L1 = at(line + 1, li + 1), L2 = at(line + 1, li + 2);
+    const unsigned R0 = at(line, ri - 1), R1 = at(line, ri), R2 = at(line, ri + 1);
+    uint64_t v = ((uint64_t)(__funnelshift_r(L1, L2, lsh) | __brev(__funnelshift_r(R0, R1, rsh)))
+                  << 32) |
+                 (__funnelshift_r(L0, L1, lsh) | __brev(__funnelshift_r(R1, R2, rsh)));
+    if (centre) {
+      // the observer's column: image X's line 0, the observer itself (siting.cpp:279)
+      const unsigned c = d == 0 ? 1u : (X[2 * ((d - 1) >> 5)] >> ((d - 1) & 31)) & 1u;
+      v |= (uint64_t)c << (S & 63);
+    }
+    dst[row * nwpr + q] = v;
   }
 }
 
-// CTAs of at most 800 threads compiled for two resident CTAs per SM (two
-// observers' windows in flight; the per-partition register file then allows
-// 32 registers per thread).
-template <bool kSmem, bool kRcp>
-__global__ void __launch_bounds__(800, 2)
-    shed_kernel2(const __grid_constant__ CUtensorMap map, const ShedArgs a) {
-  shed_body<kSmem, kRcp, false>(map, a);
-}
+// ---- quadrant windows ------------------------------------------------------------
 
-// Half windows, staged, one ray a thread: kThreads = 32*ceil((4roi+1)/32),
-// compiled for kMinBlocks resident CTAs per SM (what the window allows).
-template <int kThreads, int kMinBlocks>
-__global__ void __launch_bounds__(kThreads, kMinBlocks)
-    shed_half_kernel(const __grid_constant__ CUtensorMap map, const ShedArgs a) {
-  shed_body<true, true, true>(map, a);
-}
-
-int round8(int v) { return (v + 7) & ~7; }
-
-struct WinGeom {
-  int w, box_rows, nboxes;
-};
-
-WinGeom win_geom(int roi, bool half) {
+// A quarter of an observer a CTA, for radii whose half windows leave one CTA an
+// SM.  The pairs mirror about the quadrant's diagonal: A is x-major, B y-major, so
+// one image holds both (A: line = column distance, bit = row distance - 1; B: line
+// = row distance, bit = column distance - 1).  Block 4o + 2*lower + left of observer
+// o; the two sides of a row share the word of the observer's column, so they form a
+// cluster and the left one hands its bits of that word to the right one.
+__host__ __device__ __forceinline__ WinGeom quad_geom(int roi) {
   WinGeom g;
-  const int nr = half ? roi + 1 : 2 * roi + 1;  // window rows
-  g.w = round8(2 * roi + 8);
-  g.nboxes = (nr + 255) / 256;
-  g.box_rows = round8((nr + g.nboxes - 1) / g.nboxes);
+  g.w = ((roi + 1 + 7 + 7) & ~7) | 8;
+  g.nboxes = (roi + 1 + 255) / 256;
+  g.box_rows = g.nboxes == 1 ? roi + 1 : ((roi + g.nboxes) / g.nboxes + 7) & ~7;
   return g;
 }
 
-// Half windows are launched for roi 60..151 (4roi+1 rays in at most 608
-// threads).  16384 observers on a 2048^2 DEM, half against whole windows:
-// roi 25 +8%, 50 +0.5%, 75 -1.5%, 100 -8% (staged whole window); 110-120
-// -23..25%, 125-150 -9..13% (whole window through L1).  Below roi 60 the
-// halves' CTAs are too small (a few warps) to gain.
-constexpr int kHalfMinRoi = 60, kHalfMaxRoi = 151;
+// Words of the image and the two near maps.
+__host__ __device__ __forceinline__ int quad_mark_words(int roi) {
+  return (roi + 1) * pair_line(roi) + kNearMap / 2;
+}
+
+size_t quad_smem_bytes(int roi) {
+  return quad_geom(roi).bytes() + (size_t)(roi + 1) * (16 + 8) + 16 +
+         (((size_t)quad_mark_words(roi) * 4 + 15) & ~(size_t)15) + 16;
+}
+
+constexpr int kQuadMaxThreads = 320;
+
+__global__ void __cluster_dims__(2) __launch_bounds__(kQuadMaxThreads, 2)
+    shed_quad_kernel(const __grid_constant__ CUtensorMap map, const ShedArgs a) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  const int roi = a.roi, n = a.n, nr = 2 * roi + 1, nwpr = (nr + 63) / 64, nwords = nr * nwpr;
+  const int obi = (int)(blockIdx.x >> 2), half = (int)(blockIdx.x >> 1) & 1;
+  const bool left = blockIdx.x & 1u;
+  uint64_t *dst = a.sheds + (size_t)obi * nwords;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int ob = a.obs[obi];
+  if (ob < 0 || ob >= n * n) {  // invalid observer: empty shed, flagged (by the whole cluster)
+    const int wr0 = half ? roi + 1 : 0, wr1 = half ? nr : roi + 1;
+    if (!left)
+      for (int i = wr0 * nwpr + tid; i < wr1 * nwpr; i += blockDim.x) dst[i] = 0ull;
+    if (tid == 0) atomicOr(a.err, kErrBadInput);
+    return;
+  }
+  const int ox = ob / n, oy = ob - (ob / n) * n;
+  const WinGeom g = quad_geom(roi);
+  const int W2 = 2 * g.w, nw = pair_words(roi), ls = pair_line(roi);
+  const int hx0 = half ? ox : ox - roi;                 // window origin
+  const int hy0 = (left ? oy - roi : oy) & ~7;          // TMA inner coordinate: 16-byte aligned
+  const uint32_t win = smem_u32(sm);
+  float4 *tab = reinterpret_cast<float4 *>(sm + g.bytes());
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(tab + roi + 1);
+  uint64_t *cbuf = mbar + 2;  // the left side's bits of the shared word, by row distance
+  unsigned *img = reinterpret_cast<unsigned *>(cbuf + ((roi + 2) & ~1));
+  unsigned char *near = reinterpret_cast<unsigned char *>(img + (roi + 1) * ls);
+  if (tid == 0) {
+    mbar_init(mbar, 1);
+    mbar_expect_tx(mbar, (uint32_t)g.bytes());
+    for (int b = 0; b < g.nboxes; b++)
+      tma_load_window(sm + (size_t)b * g.box_rows * W2, &map, hy0, hx0 + b * g.box_rows, mbar);
+  }
+  for (int i = tid; i <= roi; i += blockDim.x) {
+    const float y = i ? __frcp_rn((float)i) : 0.f;
+    tab[i] = make_float4(y, y, -(float)i, -(float)i);
+  }
+  for (int i = tid; i < (quad_mark_words(roi) + 3) / 4; i += blockDim.x)
+    reinterpret_cast<uint4 *>(img)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  cluster_arrive();  // the peer may write to cbuf once this CTA runs
+  if (__all_sync(0xffffffffu, mbar_wait(mbar, 0))) {
+    if (const int t = tid; t <= roi) {
+      // every second ray, as in the half windows
+      const int evens = (roi + 2) / 2, m = t < evens ? 2 * t : 2 * (t - evens) + 1;
+      const float sl = fdiv(i2f(m), i2f(roi));
+      const int rowlim = half ? n - 1 - ox : ox, collim = left ? oy : n - 1 - oy;
+      int kA, kB;
+      pair_last(sl, roi, rowlim, collim, collim, rowlim, kA, kB);
+      const int rowstep = half ? W2 : -W2, cell = left ? -2 : 2;
+      const int p0 = (int)win + (ox - hx0) * W2 + 2 * (oy - hy0);
+      PairRays r;
+      r.dem = a.dem;
+      r.p0 = p0;
+      r.mA = r.sB = rowstep;
+      r.mB = r.sA = cell;
+      r.sl = sl;
+        const float nalt = -i2f(elevation<true>(a.dem, p0) + a.oht), tht = i2f(a.tht);
+      r.nalt = f2_pack(nalt, nalt);
+        float one;
+      asm("ld.shared.f32 %0, [%1];" : "=f"(one) : "r"(smem_u32(tab + 1)));  // RN(1/1)
+      r.one = f2_pack(one, one);
+      r.img = smem_u32(img);
+      r.near = smem_u32(near);
+      r.ls4 = 4 * ls;
+      r.tab = tab;
+      r.hs = f2_pack(kNoHorizon, kNoHorizon);
+      r.tht = f2_pack(tht, tht);
+      pair_sweep<true, true>(r, kA, kB);
+    }
+  } else if (tid == 0) {
+    atomicOr(a.err, kErrTmaTimeout);
+  }
+  __syncthreads();
+  const int nlines = min(roi, kNearSteps) + 1;
+  for (int i = tid; i < 2 * nlines; i += blockDim.x) {
+    const int map = i >= nlines, line = i - map * nlines;
+    img[line * ls + map] |= near_bits(near + map * kNearMap, line);
+  }
+  __syncthreads();
+  // A into B, as X into Y above
+  for (int b = warp; b < nw * nw; b += nwarps) {
+    const int lb = b / nw, w = b - lb * nw, line = lb * 32 + 1 + lane;
+    unsigned x = line <= roi ? img[line * ls + 2 * w] : 0u;
+    if (!__any_sync(0xffffffffu, x != 0u)) continue;
+    x = warp_transpose(x, lane);
+    const int d = w * 32 + 1 + lane;
+    if (d <= roi && x) img[d * ls + 2 * lb + 1] |= x;
+  }
+  __syncthreads();
+  // rows out (see shed_kernel): this side's words, the shared word by the right one
+  const int S = 64 * nwpr - 1 - roi, qc = nwpr - 1 - (S >> 6);
+  const int q0 = left ? 0 : qc, nq = left ? qc + 1 : nwpr - qc;
+  const int per = blockDim.x / nq, q = q0 + tid % nq, z = 2 * (nwpr - 1 - q);
+  const int s0 = left ? 32 * z - (S + 1) : S - 1 - 32 * z - 63, si = s0 >> 5, sh = s0 & 31;
+  auto word = [&](int d) {  // the string's 64 bits of word q, row distance d
+    const unsigned *line = img + d * ls + 1;
+    auto at = [&](int i) { return (unsigned)i < (unsigned)nw ? line[2 * i] : 0u; };
+    const unsigned w0 = at(si), w1 = at(si + 1), w2 = at(si + 2);
+    const unsigned lo = __funnelshift_r(w0, w1, sh), hi = __funnelshift_r(w1, w2, sh);
+    return left ? ((uint64_t)hi << 32) | lo : ((uint64_t)__brev(lo) << 32) | __brev(hi);
+  };
+  const int r0 = tid / nq + half;  // row distances half..roi
+  const bool mine = tid < per * nq;
+  __syncwarp();
+  cluster_wait();
+  if (left && mine) {
+    for (int d = r0; d <= roi; d += per) {
+      const uint64_t v = word(d);
+      if (q == qc)
+        cluster_store_u64(smem_u32(cbuf + d), 0, v);
+      else
+        dst[(half ? roi + d : roi - d) * nwpr + q] = v;
+    }
+  }
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  if (!left && mine) {
+    for (int d = r0; d <= roi; d += per) {
+      uint64_t v = word(d);
+      if (q == qc) {
+        const unsigned c = d == 0 ? 1u : (img[2 * ((d - 1) >> 5)] >> ((d - 1) & 31)) & 1u;
+        v |= cbuf[d] | (uint64_t)c << (S & 63);
+      }
+      dst[(half ? roi + d : roi - d) * nwpr + q] = v;
+    }
+  }
+}
+
+constexpr size_t kMaxSmem = 220 * 1024;
+constexpr size_t kTwoCtaSmem = 113 * 1024;  // two CTAs of an SM's 228 KB, 1 KB reserved for each
+
+constexpr int kPairMaxThreads = 448;  // the register budget of two CTAs an SM
+
+// Threads of a CTA: a pair of rays each, in even rounds where they are more than
+// kPairMaxThreads (the form read through L1 alone).
+int pair_threads(int pairs) {
+  const int rounds = (pairs + kPairMaxThreads - 1) / kPairMaxThreads;
+  return ((pairs + rounds - 1) / rounds + 31) / 32 * 32;
+}
+
+ShedPlan shed_l1_plan(int roi) { return ShedPlan{pair_threads(2 * roi + 1), false, true, false}; }
+
+ShedPlan shed_quad_plan(int roi) {
+  return ShedPlan{(roi + 1 + 31) / 32 * 32, true, false, true};
+}
+
+// The staged form of a radius.  The SM holds few CTAs of a large window, so the
+// window shrinks with the radius (ms at 2048^2, 1.6 G cells of rays; whole, half,
+// quarter): roi 30 0.454, 0.484; 60 1.016, 1.021, 1.233; 70 1.018, 1.056, 1.240;
+// 90 1.018, 0.987, 0.945; 100 1.032, 0.981, 1.067; 118 -, 0.956, 0.957; 125 -,
+// 1.039, 0.904; 140 -, 1.056, 0.962; 200 -, 1.390, 1.138.  From roi 209 quarters
+// are one CTA an SM and halves are faster while they fit (212: 1.344, 1.744).
+constexpr int kHalfMinRoi = 75, kQuadMinRoi = 119;
+
+ShedPlan shed_staged_plan(int roi, bool half) {
+  if (roi < 1) return shed_l1_plan(roi);
+  if (!half && 4 * roi + 1 <= kPairMaxThreads && pair_smem_bytes(roi, 2, true) <= kMaxSmem)
+    return ShedPlan{pair_threads(4 * roi + 1), true, false, false};
+  const bool quad_fits = (roi + 1 + 31) / 32 * 32 <= kQuadMaxThreads && quad_smem_bytes(roi) <= kMaxSmem;
+  if (roi >= kQuadMinRoi && quad_smem_bytes(roi) <= kTwoCtaSmem) return shed_quad_plan(roi);
+  if (pair_smem_bytes(roi, 1, true) <= kMaxSmem)
+    return ShedPlan{pair_threads(2 * roi + 1), true, true, false};
+  return quad_fits ? shed_quad_plan(roi) : shed_l1_plan(roi);
+}
 
 }  // namespace
 
 size_t shed_smem_bytes(const ShedPlan &p, int roi) {
-  const int nr = 2 * roi + 1, nri = p.half ? roi + 1 : nr;  // image rows
-  size_t b = 16 + 4 * ((size_t)nri * shed_row_stride(nr) + (size_t)shed_col_count(nr) * shed_col_stride(nri));
-  b += 4 * ((size_t)roi + 1);  // reciprocal table
-  if (p.use_smem) {
-    const WinGeom g = win_geom(roi, p.half);
-    b += (size_t)g.nboxes * g.box_rows * g.w * 2;
-  }
-  return b;
+  return p.quad ? quad_smem_bytes(roi) : pair_smem_bytes(roi, p.half ? 1 : 2, p.use_smem);
 }
 
-namespace {
+ShedPlan shed_default_plan(int roi) { return shed_staged_plan(roi, roi >= kHalfMinRoi); }
 
-// One CTA an observer: one ray per thread up to 800 rays (two resident CTAs
-// per SM at 32 registers a thread), else an even split into rounds of at most
-// 800 (a single 1024-thread CTA per SM ran 1.5x slower per ray step, roi
-// 104-128).  The window is staged only while two CTAs of a full round of rays
-// still share an SM: a ray's steps form one dependent chain, so fewer
-// resident warps cannot hide the shared-memory latency and the L1 path, with
-// more resident CTAs, is faster.
-ShedPlan shed_whole_plan(int roi) {
-  const int rays = 8 * roi;
-  const int rounds = (rays + 799) / 800;
-  const int threads = std::min(800, ((rays + rounds - 1) / rounds + 31) / 32 * 32);
-  ShedPlan p{std::max(threads, 64), true, false};
-  if (rounds > 1 || shed_smem_bytes(p, roi) > 112 * 1024) p.use_smem = false;
-  return p;
-}
-
-// Two CTAs an observer, each staging its half window, one ray a thread.
-ShedPlan shed_half_plan(int roi) { return ShedPlan{(4 * roi + 1 + 31) / 32 * 32, true, true}; }
-
-}  // namespace
-
-ShedPlan shed_default_plan(int roi) {
-  return roi >= kHalfMinRoi && roi <= kHalfMaxRoi ? shed_half_plan(roi) : shed_whole_plan(roi);
-}
-
-// smem: 1 half windows (up to roi 151, else as 2), 2 the whole window,
-// staged where it fits, 0 the whole window through L1, -1 the default.
+// smem: 1 half windows staged, 2 the whole window staged (as 1 where it does
+// not fit), 0 the window read through L1 (as 1 and 2 are where half a window
+// does not fit), -1 the default.
 ShedPlan shed_plan_for(int roi, int smem) {
-  if (smem == 1 && roi >= 1 && roi <= kHalfMaxRoi) return shed_half_plan(roi);
-  if (smem == 1 || smem == 2) return shed_whole_plan(roi);
-  if (smem == 0) {
-    ShedPlan p = shed_whole_plan(roi);
-    p.use_smem = false;
-    return p;
-  }
-  return shed_default_plan(roi);
+  if (smem == 1 || smem == 2) return shed_staged_plan(roi, smem == 1);
+  return smem == 0 ? shed_l1_plan(roi) : shed_default_plan(roi);
 }
 
 cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nsheds,
                          const int32_t *obs, uint64_t *sheds, const ShedPlan &plan, int *d_err,
                          cudaStream_t st) {
   if (nsheds <= 0) return cudaSuccess;
-  ShedArgs a{};
-  a.dem = dem.data;
-  a.pitch = dem.pitch;
-  a.n = dem.nrows;
-  a.roi = roi;
-  a.oht = oht;
-  a.tht = tht;
-  a.nsheds = nsheds;
-  a.obs = obs;
-  a.sheds = sheds;
-  a.err = d_err;
+  // radii up to 475: two bit images of a whole shed and a reciprocal a step fit a CTA
+  const size_t nr = 2 * (size_t)roi + 1, w32 = (nr + 31) / 32, w64 = (nr + 63) / 64;
+  if (4 * (nr * (2 * w64 | 1) + 32 * w32 * (w32 | 1) + roi + 1) + 16 > 227 * 1024)
+    return cudaErrorInvalidValue;
+  const ShedArgs a{dem.data, dem.pitch, dem.nrows, roi, oht, tht, obs, sheds, d_err};
   // the reciprocal-table division is exhaustively checked for |a| <= 2^21
   // (heights up to 10^6 over 16-bit elevations) and steps up to 2048
-  const bool rcp = roi <= 2048 && oht >= 0 && oht <= 1000000;
-  // half windows need the staged window and the table division
-  ShedPlan eff = plan;
-  if (eff.half && (!rcp || !dem.tma_ok || roi < 1 || roi > kHalfMaxRoi)) eff = shed_whole_plan(roi);
-  eff.use_smem = eff.use_smem && dem.tma_ok;
+  const bool rcp = oht >= 0 && oht <= 1000000;
+  const ShedPlan eff = plan.use_smem && !(rcp && dem.tma_ok) ? shed_l1_plan(roi) : plan;
+  const size_t shm = shed_smem_bytes(eff, roi);
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   if (eff.use_smem) {
-    const WinGeom g = win_geom(roi, eff.half);
-    a.win_w = g.w;
-    a.box_rows = g.box_rows;
-    a.nboxes = g.nboxes;
+    const WinGeom g = eff.quad ? quad_geom(roi) : win_geom(roi, eff.half ? 1 : 2, true);
     if (!make_dem_tensor_map(&map, dem, g.w, g.box_rows)) return cudaErrorInvalidValue;
   }
-  const size_t shm = shed_smem_bytes(eff, roi);
-  auto launch = [&](auto kern, int ctas) -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    if (e != cudaSuccess) return e;
-    kern<<<ctas, eff.threads, shm, st>>>(map, a);
-    return cudaSuccess;
-  };
-  cudaError_t e;
-  if (eff.half) {
-    // the variant compiled for as many resident CTAs as the window allows
-    e = eff.threads <= 416   ? launch(shed_half_kernel<416, 4>, 2 * nsheds)
-        : eff.threads <= 512 ? launch(shed_half_kernel<512, 3>, 2 * nsheds)
-                             : launch(shed_half_kernel<608, 2>, 2 * nsheds);
-  } else if (eff.use_smem) {
-    e = rcp ? launch(shed_kernel2<true, true>, nsheds) : launch(shed_kernel2<true, false>, nsheds);
-  } else {
-    e = rcp ? launch(shed_kernel2<false, true>, nsheds) : launch(shed_kernel2<false, false>, nsheds);
-  }
+  auto kern = !eff.use_smem ? (rcp ? shed_kernel<1, false, true> : shed_kernel<1, false, false>)
+              : eff.quad    ? shed_quad_kernel
+              : eff.half    ? shed_kernel<1, true, true>
+                            : shed_kernel<2, true, true>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
   if (e != cudaSuccess) return e;
+  kern<<<nsheds * (eff.quad ? 4 : eff.half ? 2 : 1), eff.threads, shm, st>>>(map, a);
   return cudaGetLastError();
 }
 
