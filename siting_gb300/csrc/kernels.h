@@ -94,6 +94,21 @@ cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st);
 cudaError_t launch_findmax_queue(const StageJob *jobs, int njobs, cudaStream_t st);
 
 // ---- SITE -----------------------------------------------------------------------
+// Device scratch of a SITE job without intervis (site_local.cuh).
+struct LocalScratch {
+  unsigned *count;             // [bins+1]: candidates of each bin, then their ranges' starts; zeroed
+  unsigned *fill;              // [bins]; zeroed
+  unsigned long long *gmax;    // [2]; zeroed
+  unsigned *npick;             // [2]; zeroed
+  int *ncount;                 // [2][cap]; zeroed
+  unsigned long long *binkey;  // [bins]: the bin's largest key
+  int2 *binat;                 // [bins]: its place in the sorted arrays, its cell
+  int *cand, *pos, *gain;      // sorted candidates: index, cell (row << 16 | column), gain
+  int4 *pick;                  // [cap]: the round's picks: place in the sorted arrays, index, cell, area
+  unsigned long long *plist;   // [nsheds]: keys of all picks taken
+  unsigned *rank;              // [nsheds]; zeroed
+};
+
 // Scratch layout of one SITE job (device, carved from one allocation).
 struct SiteScratch {
   uint64_t *cum;             // nrows * ceil(nrows/64) words, zeroed before launch
@@ -107,6 +122,7 @@ struct SiteScratch {
   int32_t *order;            // nsheds: picks in order
   int32_t *gains;            // nsheds: round-1 gains (site_score_kernel)
   void *table;               // job table of a one-job launch (site_job_table_bytes)
+  LocalScratch local;        // without intervis
 };
 
 // Phases of the SITE tracing clocks (siting_last_site_phase_cycles).
@@ -133,8 +149,9 @@ size_t site_job_table_bytes(int njobs, int total_ctas);
 // kept unchanged until the copy has run; NULL stages through pageable memory.
 cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void *h_stage,
                              cudaStream_t st);
-size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi);
-void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, SiteScratch *s);
+size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis);
+void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,
+                        SiteScratch *s);
 int site_default_ctas(int nsheds, int sm_count);
 // The CTA count near G0 that spreads a pick's neighbourhood most evenly over
 // the CTAs for the job's block geometry (nb blocks a row, npb candidates each).

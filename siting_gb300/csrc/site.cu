@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -88,7 +89,17 @@ struct SiteArgs {
   int nslots, pick_items, pick_cap, pair_cap;
   long long stop_area;  // smallest cumarea with 100.0*cumarea/n^2 > 95 (host-computed)
   int block0;           // first CTA of this job's group in the launch
+  LocalScratch local;   // without intervis
+  int local_words;      // shared-memory words for the picks' new bits
 };
+
+}  // namespace
+}  // namespace siting
+
+#include "site_local.cuh"
+
+namespace siting {
+namespace {
 
 __device__ __forceinline__ void shed_align(int c0, int &fw, int &fb) {
   fw = c0 >> 6;  // floor division by 64 (siting.cpp:400-405)
@@ -169,6 +180,17 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (threadIdx.x == 0) s_args = jobs[block_job[blockIdx.x]];
   __syncthreads();
   const SiteArgs &a = s_args;
+  // tracing: device cycles per phase, accumulated by CTA 0's thread 0 in
+  // shared memory (a register array would take registers in every thread)
+  __shared__ long long s_ph[kSitePhases], s_tmark;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kSitePhases; i++) s_ph[i] = 0;
+    s_tmark = clock64();
+  }
+  if (!a.intervis) {
+    site_local(a, *reinterpret_cast<LocalShared *>(sm), (int)blockIdx.x - a.block0, s_ph, &s_tmark);
+    return;
+  }
   __shared__ int s_m, s_mcut, s_stop_at, s_done, s_flagv, s_roundcut, s_npair, s_nvalid;
   __shared__ long long s_cum;
   __shared__ int s_poff[kMaxPicks + 1];
@@ -233,13 +255,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char *s_nmask = take(kMaskCap);
 
   GroupBarrier gb{a.bar, (unsigned)G, 0u};
-  // tracing: device cycles per phase, accumulated by CTA 0's thread 0 in
-  // shared memory (a register array would take registers in every thread)
-  __shared__ long long s_ph[kSitePhases], s_tmark;
-  if (tid == 0) {
-    for (int i = 0; i < kSitePhases; i++) s_ph[i] = 0;
-    s_tmark = clock64();
-  }
   auto mark = [&](int i) {
     if (k == 0 && tid == 0) {
       const long long now = clock64();
@@ -1057,41 +1072,55 @@ long long site_stop_area(int nrows) {
 
 namespace {
 
-size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, unsigned char *base,
+size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, unsigned char *base,
                       SiteScratch *s) {
   const size_t cw = (size_t)(nrows + 63) / 64;
+  const size_t nr = 2 * (size_t)roi + 1, row = ((nr + 63) / 64 + 1) * 8;
   size_t off = 0;
   auto take = [&](size_t bytes) {
     unsigned char *q = base ? base + off : nullptr;
     off += (bytes + 255) & ~(size_t)255;
     return q;
   };
+  SiteScratch t{};
+  auto carve = [&](auto *&p, size_t bytes) {
+    p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(take(bytes));
+  };
   // zeroed before a launch: everything up to `order`
-  unsigned char *c0 = take((size_t)nrows * cw * 8);
-  unsigned char *tk = take((size_t)2 * nctas * kTopK * 2 * 8);
-  unsigned char *cu = take((size_t)2 * nctas * 4);
-  unsigned char *nc = take((size_t)2 * kMaxPicks * 4);
-  unsigned char *br = take(64);
-  unsigned char *ou = take(128);
-  unsigned char *od = take((size_t)nsheds * 4);
-  unsigned char *gn = take((size_t)nsheds * 4);
-  const size_t nr = 2 * (size_t)roi + 1;  // every row is written before it is read
-  unsigned char *nb = take((size_t)kMaxPicks * nr * ((nr + 63) / 64 + 1) * 8);
-  unsigned char *nm = take((size_t)kMaxPicks * nr + 16);  // + the 16-byte loads' tail
-  unsigned char *tb = take(site_job_table_bytes(1, nctas));
-  if (s) {
-    s->cum = reinterpret_cast<uint64_t *>(c0);
-    s->nbits = reinterpret_cast<uint64_t *>(nb);
-    s->nmask = nm;
-    s->topk = reinterpret_cast<unsigned long long *>(tk);
-    s->cuts = reinterpret_cast<int *>(cu);
-    s->ncount = reinterpret_cast<int *>(nc);
-    s->bar = reinterpret_cast<unsigned *>(br);
-    s->out = reinterpret_cast<long long *>(ou);
-    s->order = reinterpret_cast<int32_t *>(od);
-    s->gains = reinterpret_cast<int32_t *>(gn);
-    s->table = tb;
+  carve(t.cum, (size_t)nrows * cw * 8);
+  carve(t.bar, 64);
+  carve(t.out, 128);
+  LocalScratch &l = t.local;
+  const size_t bins = intervis ? 0 : (size_t)local_bins(nrows, roi) * local_bins(nrows, roi);
+  const int cap = intervis ? kMaxPicks : local_cap(nsheds, roi);
+  if (intervis) {
+    carve(t.topk, (size_t)2 * nctas * kTopK * 2 * 8);
+    carve(t.cuts, (size_t)2 * nctas * 4);
+    carve(t.ncount, (size_t)2 * kMaxPicks * 4);
+  } else {
+    carve(l.count, (bins + 1) * 4);
+    carve(l.fill, bins * 4);
+    carve(l.gmax, 16);
+    carve(l.npick, 8);
+    carve(l.ncount, (size_t)2 * cap * 4);
+    carve(l.rank, (size_t)nsheds * 4);
   }
+  carve(t.order, (size_t)nsheds * 4);
+  carve(t.gains, (size_t)nsheds * 4);
+  carve(t.nbits, cap * nr * row);  // every row is written before it is read
+  if (intervis) {
+    carve(t.nmask, (size_t)kMaxPicks * nr + 16);  // + the 16-byte loads' tail
+  } else {
+    carve(l.binkey, bins * 8);
+    carve(l.binat, bins * 8);
+    carve(l.cand, (size_t)nsheds * 4);
+    carve(l.pos, (size_t)nsheds * 4);
+    carve(l.gain, (size_t)nsheds * 4);
+    carve(l.pick, (size_t)cap * 16);
+    carve(l.plist, (size_t)nsheds * 8);
+  }
+  t.table = take(site_job_table_bytes(1, nctas));
+  if (s) *s = t;
   return off;
 }
 
@@ -1099,12 +1128,13 @@ size_t round16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 }  // namespace
 
-size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi) {
-  return scratch_layout(nrows, nsheds, nctas, roi, nullptr, nullptr);
+size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis) {
+  return scratch_layout(nrows, nsheds, nctas, roi, intervis, nullptr, nullptr);
 }
 
-void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, SiteScratch *s) {
-  scratch_layout(nrows, nsheds, nctas, roi, static_cast<unsigned char *>(base), s);
+void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,
+                        SiteScratch *s) {
+  scratch_layout(nrows, nsheds, nctas, roi, intervis, static_cast<unsigned char *>(base), s);
 }
 
 // Up to one CTA per SM, about 100 candidates per CTA but at least 32 CTAs:
@@ -1192,6 +1222,8 @@ size_t site_smem_base(int roi, int nsheds, int nctas, int nblocks, int npb, floa
 constexpr size_t kSiteSmemPlan = 220 * 1024;
 constexpr int kMaxNWords = 4096;
 
+constexpr size_t kLocalSmem = 216 * 1024;  // of a job without intervis
+
 int site_ncap_words(size_t base) {
   if (base >= kSiteSmemPlan) return 0;
   return (int)std::min<size_t>(kMaxNWords, (kSiteSmemPlan - base) / 8 / 2 * 2);
@@ -1242,6 +1274,8 @@ SiteArgs make_site_args(const SiteJob &j, int block0) {
   a.pair_cap = site_pair_cap(pb);
   a.stop_area = site_stop_area(j.nrows);
   a.block0 = block0;
+  a.local = j.scratch.local;
+  a.local_words = (int)((kLocalSmem - sizeof(LocalShared)) / 8);
   return a;
 }
 
@@ -1261,8 +1295,10 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
     args[i] = make_site_args(jobs[i], total);
     for (int b = 0; b < jobs[i].nctas; b++) block_job.push_back(i);
     total += jobs[i].nctas;
-    shm = std::max(shm, site_smem_bytes(jobs[i].roi, jobs[i].nsheds, jobs[i].nctas,
-                                        jobs[i].nblocks, jobs[i].npb, jobs[i].blocksize));
+    shm = std::max(shm, jobs[i].intervis
+                            ? site_smem_bytes(jobs[i].roi, jobs[i].nsheds, jobs[i].nctas,
+                                              jobs[i].nblocks, jobs[i].npb, jobs[i].blocksize)
+                            : kLocalSmem);
   }
   if (total == 0) return cudaSuccess;
   // job table: arguments, then the CTA -> job map
@@ -1361,7 +1397,10 @@ cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int3
 // it and must be serialised by the caller.
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;  // 16 MiB per device
+// Jobs are admitted by the scratch that a selection with intervis takes (16 MiB at
+// most); one without takes up to 24 bytes a candidate and 8 MiB of new bits more.
+constexpr size_t kNoAllocLimit = size_t(16) << 20;
+constexpr size_t kNoAllocScratchBytes = size_t(40) << 20;  // per device
 
 }  // namespace
 
@@ -1409,14 +1448,15 @@ extern "C" int siting_site_it_noalloc(int nrows, int roi, int intervis, int nshe
   // candidates are taken in any order: one block row holding them all
   const float bs = (float)nrows;
   if (site_smem_bytes(roi, nsheds, G, 1, nsheds, bs) > 220 * 1024) return SITING_EINVAL;
-  const size_t need = site_scratch_bytes(nrows, nsheds, G, roi) + 256;  // + error flag
-  if (need > kNoAllocScratchBytes) return SITING_ENOMEM;  // beyond the 16 MiB array
+  if (site_scratch_bytes(nrows, nsheds, G, roi, 1) + 256 > kNoAllocLimit) return SITING_ENOMEM;
+  const size_t need = site_scratch_bytes(nrows, nsheds, G, roi, intervis) + 256;  // + error flag
+  if (need > kNoAllocScratchBytes) return SITING_ENOMEM;
   void *base = nullptr;
   int rc = noalloc_scratch(&base);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   SiteScratch s;
-  site_carve_scratch(base, nrows, nsheds, G, roi, &s);
+  site_carve_scratch(base, nrows, nsheds, G, roi, intervis, &s);
   int *d_err = reinterpret_cast<int *>(static_cast<unsigned char *>(base) + need - 256);
   // zero coverage, key lists, cuts, self-check counters, barrier and outputs
   if (cudaMemsetAsync(base, 0, (unsigned char *)s.order - (unsigned char *)base, st) != cudaSuccess ||
