@@ -94,19 +94,24 @@ cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st);
 cudaError_t launch_findmax_queue(const StageJob *jobs, int njobs, cudaStream_t st);
 
 // ---- SITE -----------------------------------------------------------------------
-// Device scratch of a SITE job without intervis (site_local.cuh).
+// Device scratch of a selection (site_local.cuh).
 struct LocalScratch {
   unsigned *count;             // [bins+1]: candidates of each bin, then their ranges' starts; zeroed
   unsigned *fill;              // [bins]; zeroed
-  unsigned long long *gmax;    // [2]; zeroed
-  unsigned *npick;             // [2]; zeroed
-  int *ncount;                 // [2][cap]; zeroed
+  unsigned long long *gmax;    // [2]: the round's largest key; zeroed
+  unsigned *ndom, *npick;      // [2]: the round's dominant candidates and picks; zeroed
+  int *ncount;                 // [2][cap]: popcount of each pick's new bits (self-check); zeroed
+  int *bad;                    // [2][cells], with intervis: dominant ones that may be overtaken; zeroed
   unsigned long long *binkey;  // [bins]: the bin's largest key
+  unsigned long long *bincap;  // [bins]: and of those that a pick may make eligible (intervis)
+  unsigned *search;            // [G]: the searches of B2 (intervis)
   int2 *binat;                 // [bins]: its place in the sorted arrays, its cell
-  int *cand, *pos, *gain;      // sorted candidates: index, cell (row << 16 | column), gain
-  int4 *pick;                  // [cap]: the round's picks: place in the sorted arrays, index, cell, area
+  int4 *rec;                   // sorted candidates: cell (row << 16 | column), gain, index, flags
+  int4 *dom, *pick;            // [cells], [cap]: place in the sorted arrays, index, cell, area
   unsigned long long *plist;   // [nsheds]: keys of all picks taken
-  unsigned *rank;              // [nsheds]; zeroed
+  // with intervis, of each pick: its level, the pick that covered its cell (or -1)
+  unsigned long long *preach;
+  int *pparent;
 };
 
 // Scratch layout of one SITE job (device, carved from one allocation).

@@ -12,7 +12,9 @@
 //     100.0*cumarea/n^2 > 95 (after adding the pick).
 //
 // GB300 mapping: one persistent kernel of G co-resident CTAs (one per SM)
-// with a bounded group barrier.  Candidate c is owned by CTA c % G, which
+// with a bounded group barrier.  A job is selected by local dominance
+// (site_local.cuh) or, with intervis and few candidates or dense ones
+// (site_is_local), in the global order below.  Candidate c is owned by CTA c % G, which
 // keeps its true gain, area, cell and flags in shared memory and a top-K key
 // list per 32 slots (key = area << 32 | ~c, K = kTopK).  A round:
 //   A. every CTA publishes its own top-K keys; one barrier;
@@ -28,7 +30,7 @@
 //      bits are disjoint.  Small rounds compute N in every CTA's shared
 //      memory; larger ones spread its rows over the CTAs (a global buffer
 //      read after one more barrier);
-//   E. with intervis, a candidate of area 0 whose cell a pick covers can
+//   E. a candidate of area 0 whose cell a pick covers can
 //      become eligible: each CTA finds the first prefix position it would
 //      overtake, and a second barrier takes the minimum (the round's cut);
 //   F. the picks before the cut are applied: gains fall by the summed
@@ -59,8 +61,7 @@ int site_threads_for(int nslots, int roi) { return (nslots > 1024 || roi > 127) 
 constexpr int kMaxSlots = 4096;  // candidates owned by one CTA
 // Keys each CTA publishes per round.  Rounds end at distance conflicts and
 // intervis cuts long before the threshold of K keys binds (4096^2: 343
-// rounds with 3, 4, 6 or 8), and fewer keys make each merge cheaper; with 2
-// the threshold binds (16384^2: 725 -> 1015 rounds).
+// rounds with 3, 4, 6 or 8), and fewer keys make each merge cheaper.
 constexpr int kTopK = 3;
 constexpr int kMaxPicks = 64;    // picks accepted in one round at most
 constexpr int kSmallRecip = 128; // reciprocals tabled in shared memory (>= kMaxPicks)
@@ -89,7 +90,8 @@ struct SiteArgs {
   int nslots, pick_items, pick_cap, pair_cap;
   long long stop_area;  // smallest cumarea with 100.0*cumarea/n^2 > 95 (host-computed)
   int block0;           // first CTA of this job's group in the launch
-  LocalScratch local;   // without intervis
+  LocalScratch local;   // of site_local
+  int use_local;        // the selection by local dominance
   int local_words;      // shared-memory words for the picks' new bits
 };
 
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < kSitePhases; i++) s_ph[i] = 0;
     s_tmark = clock64();
   }
-  if (!a.intervis) {
+  if (a.use_local) {
     site_local(a, *reinterpret_cast<LocalShared *>(sm), (int)blockIdx.x - a.block0, s_ph, &s_tmark);
     return;
   }
@@ -566,11 +568,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           s_pairslot[pr] = s;
           s_pairdelta[pr] = 0;
-          unsigned char cv = 0;
-          if (a.intervis)  // own cell already covered?
-            cv = (unsigned char)(((__ldcg(cum + (size_t)cx * cw + (cy >> 6)) >> (63 - (cy & 63))) & 1ull)
-                                 << 1);
-          s_paircov[pr] = cv;
+          // own cell already covered?
+          s_paircov[pr] = (unsigned char)(
+              ((__ldcg(cum + (size_t)cx * cw + (cy >> 6)) >> (63 - (cy & 63))) & 1ull) << 1);
         } else {
           atomicOr(a.err, kErrCapacity);
         }
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(cy - roi, fwc, fbc);
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = s_N + (size_t)(pi * nr + prow) * nb2;
-        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
+        if (r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((nrow[j] >> (63 - (cy & 63))) & 1ull))
             atomicOr(reinterpret_cast<unsigned *>(s_paircov + (pr & ~3)), 1u << (8 * (pr & 3)));
@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
         const unsigned rowm = masked ? s_nmask[pi * nr + prow] : 0xffu;
-        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
+        if (r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((rowm >> j) & 1u) &&
               ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
         const unsigned rowm = masked ? s_nmask[pi * nr + prow] : 0xffu;
-        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
+        if (r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((rowm >> j) & 1u) &&
               ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(cy - roi, fwc, fbc);
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
-        if (a.intervis && r == roi && ch == 0) {  // own cell: newly covered by the pick?
+        if (r == roi && ch == 0) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
             atomicOr(reinterpret_cast<unsigned *>(s_paircov + (pr & ~3)), 1u << (8 * (pr & 3)));
@@ -864,72 +864,66 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     mark(6);
 
-    // ---- E. intervis: where would a newly covered candidate overtake? --------
+    // ---- E. where would a newly covered candidate overtake? --------
     if (tid == 0) s_roundcut = m;
     __syncthreads();
-    if (a.intervis) {
-      for (int u = tid; u < npair; u += blockDim.x) {
-        const int i = s_plist[u];
-        const int j = div_by(i, s_rpcap);
-        const int s = s_pairslot[i];
-        if (!(s_flag[s] & kInel) || !(s_paircov[i] & 1)) continue;
-        const int c = s * G + k;
-        // this candidate's deltas by pick: it is within 2roi of few picks, which
-        // are > 2roi apart; more than 8 falls back to cutting at the first
-        // position it could matter, which is always safe
-        int dpick0 = -1, dpick1 = -1, dpick2 = -1, dpick3 = -1, dpick4 = -1, dpick5 = -1;
-        int dval0 = 0, dval1 = 0, dval2 = 0, dval3 = 0, dval4 = 0, dval5 = 0, nd = 0;
-        bool many = false;
-        for (int j2 = 0; j2 < m; j2++) {
-          const int cnt2 = min(s_pcnt[j2], pcap);
-          for (int q2 = 0; q2 < cnt2; q2++)
-            if (s_pairslot[j2 * pcap + q2] == s) {
-              const int dv = s_pairdelta[j2 * pcap + q2];
-              switch (nd) {
-                case 0: dpick0 = j2; dval0 = dv; break;
-                case 1: dpick1 = j2; dval1 = dv; break;
-                case 2: dpick2 = j2; dval2 = dv; break;
-                case 3: dpick3 = j2; dval3 = dv; break;
-                case 4: dpick4 = j2; dval4 = dv; break;
-                case 5: dpick5 = j2; dval5 = dv; break;
-                default: many = true;
-              }
-              nd++;
+    for (int u = tid; u < npair; u += blockDim.x) {
+      const int i = s_plist[u];
+      const int j = div_by(i, s_rpcap);
+      const int s = s_pairslot[i];
+      if (!(s_flag[s] & kInel) || !(s_paircov[i] & 1)) continue;
+      const int c = s * G + k;
+      // this candidate's deltas by pick: it is within 2roi of few picks, which
+      // are > 2roi apart; more than 8 falls back to cutting at the first
+      // position it could matter, which is always safe
+      int dpick0 = -1, dpick1 = -1, dpick2 = -1, dpick3 = -1, dpick4 = -1, dpick5 = -1;
+      int dval0 = 0, dval1 = 0, dval2 = 0, dval3 = 0, dval4 = 0, dval5 = 0, nd = 0;
+      bool many = false;
+      for (int j2 = 0; j2 < m; j2++) {
+        const int cnt2 = min(s_pcnt[j2], pcap);
+        for (int q2 = 0; q2 < cnt2; q2++)
+          if (s_pairslot[j2 * pcap + q2] == s) {
+            const int dv = s_pairdelta[j2 * pcap + q2];
+            switch (nd) {
+              case 0: dpick0 = j2; dval0 = dv; break;
+              case 1: dpick1 = j2; dval1 = dv; break;
+              case 2: dpick2 = j2; dval2 = dv; break;
+              case 3: dpick3 = j2; dval3 = dv; break;
+              case 4: dpick4 = j2; dval4 = dv; break;
+              case 5: dpick5 = j2; dval5 = dv; break;
+              default: many = true;
             }
-        }
-        int cut = m;
-        if (many) {
-          cut = j + 1;
-        } else {
-          for (int qq = j + 1; qq < m; qq++) {  // gain after picks 0..qq-1
-            int g = s_gain[s];
-            g -= (dpick0 >= 0 && dpick0 < qq) ? dval0 : 0;
-            g -= (dpick1 >= 0 && dpick1 < qq) ? dval1 : 0;
-            g -= (dpick2 >= 0 && dpick2 < qq) ? dval2 : 0;
-            g -= (dpick3 >= 0 && dpick3 < qq) ? dval3 : 0;
-            g -= (dpick4 >= 0 && dpick4 < qq) ? dval4 : 0;
-            g -= (dpick5 >= 0 && dpick5 < qq) ? dval5 : 0;
-            if (make_key(g, c) > s_pkey[qq]) {
-              cut = qq;
-              break;
-            }
+            nd++;
+          }
+      }
+      int cut = m;
+      if (many) {
+        cut = j + 1;
+      } else {
+        for (int qq = j + 1; qq < m; qq++) {  // gain after picks 0..qq-1
+          int g = s_gain[s];
+          g -= (dpick0 >= 0 && dpick0 < qq) ? dval0 : 0;
+          g -= (dpick1 >= 0 && dpick1 < qq) ? dval1 : 0;
+          g -= (dpick2 >= 0 && dpick2 < qq) ? dval2 : 0;
+          g -= (dpick3 >= 0 && dpick3 < qq) ? dval3 : 0;
+          g -= (dpick4 >= 0 && dpick4 < qq) ? dval4 : 0;
+          g -= (dpick5 >= 0 && dpick5 < qq) ? dval5 : 0;
+          if (make_key(g, c) > s_pkey[qq]) {
+            cut = qq;
+            break;
           }
         }
-        if (cut < m) atomicMin(&s_roundcut, cut);
       }
-      __syncthreads();
-      if (tid == 0) __stcg(a.cuts + par * G + k, s_roundcut);
+      if (cut < m) atomicMin(&s_roundcut, cut);
     }
+    __syncthreads();
+    if (tid == 0) __stcg(a.cuts + par * G + k, s_roundcut);
     mark(12);
-    // every read of the coverage this round is done once all CTAs pass here.
-    // Without intervis there is no cut to agree on, and in a spread round the
-    // coverage is read only before the spread barrier: the coverage update
-    // may start at once.  (The buffers reused by the next round are written
-    // only after its first barrier, which every CTA reaches after this one.)
-    if ((a.intervis || !dist) && !group_sync(gb, a.err, &s_flagv)) return;
+    // every read of the coverage this round is done once all CTAs pass here
+    if (!group_sync(gb, a.err, &s_flagv)) return;
     if (tid == 0) s_mcut = m;
     __syncthreads();
-    if (a.intervis) {  // the smallest cut of any CTA: one load per thread
+    {  // the smallest cut of any CTA: one load per thread
       int c = tid < G ? __ldcg(a.cuts + par * G + tid) : m;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) c = min(c, __shfl_xor_sync(0xffffffffu, c, o));
@@ -999,7 +993,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int g = s_gain[s] - s_dacc[s];
         s_gain[s] = g;
         s_dacc[s] = 0;
-        const bool inel = a.intervis && !(tag & 6);
+        const bool inel = !(tag & 6);
         s_area[s] = inel ? 0 : g;
         s_flag[s] = (unsigned char)((s_flag[s] & ~kInel) | (inel ? kInel : 0));
         s_dirty[s >> 5] = 1;
@@ -1072,8 +1066,26 @@ long long site_stop_area(int nrows) {
 
 namespace {
 
-size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, unsigned char *base,
-                      SiteScratch *s) {
+// Whether a job is selected by local dominance (site_local): any without intervis
+// (1537^2, 18 456 candidates: 0.93 ms against 1.93 ms in the global order; 287^2, 648
+// candidates: 0.24 against 0.19).  With intervis a round also searches for the
+// candidates that its picks would uncover (B2).  That pays where many regions are
+// independent and a search meets few candidates: from 16 384 candidates on, with at
+// most 512 in a pick's circle, and at most 64 where more than a twentieth of all cells
+// are candidates.  Measured on 98 jobs of 15 000 to 180 000 candidates, radius 7 to 200:
+// the 61 within these lines took 0.54 of the global order's time in the mean
+// (4055^2, radius 14, 54 675 candidates: 36 ms against 143; the slowest 1.1 times), the
+// other 37 1.01 of it (915^2, radius 16, 93 025: 6.2 ms against 4.0; 1152^2, radius 61,
+// 147 456: 5.3 against 3.2; with fewer candidates 992^2, radius 58, 15 376: 1.7
+// against 1.3).
+bool site_is_local(int nrows, int nsheds, int roi, int intervis) {
+  const double n2 = (double)nrows * nrows, circle = 3.14159 * roi * roi / n2 * nsheds;
+  return !intervis ||
+         (nsheds >= 16384 && circle <= 512 && (circle <= 64 || 20.0 * nsheds <= n2));
+}
+
+size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, bool local,
+                      unsigned char *base, SiteScratch *s) {
   const size_t cw = (size_t)(nrows + 63) / 64;
   const size_t nr = 2 * (size_t)roi + 1, row = ((nr + 63) / 64 + 1) * 8;
   size_t off = 0;
@@ -1091,33 +1103,40 @@ size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, u
   carve(t.bar, 64);
   carve(t.out, 128);
   LocalScratch &l = t.local;
-  const size_t bins = intervis ? 0 : (size_t)local_bins(nrows, roi) * local_bins(nrows, roi);
-  const int cap = intervis ? kMaxPicks : local_cap(nsheds, roi);
-  if (intervis) {
-    carve(t.topk, (size_t)2 * nctas * kTopK * 2 * 8);
-    carve(t.cuts, (size_t)2 * nctas * 4);
-    carve(t.ncount, (size_t)2 * kMaxPicks * 4);
-  } else {
+  const size_t bins = local ? (size_t)local_bins(nrows, roi) * local_bins(nrows, roi) : 0;
+  const size_t cells = local ? (size_t)local_cells(nrows, roi) * local_cells(nrows, roi) : 0;
+  const int cap = local ? local_cap(roi) : kMaxPicks;
+  if (local) {
     carve(l.count, (bins + 1) * 4);
     carve(l.fill, bins * 4);
     carve(l.gmax, 16);
+    carve(l.ndom, 8);
     carve(l.npick, 8);
     carve(l.ncount, (size_t)2 * cap * 4);
-    carve(l.rank, (size_t)nsheds * 4);
+    if (intervis) carve(l.bad, 2 * cells * 4);
+  } else {
+    carve(t.topk, (size_t)2 * nctas * kTopK * 2 * 8);
+    carve(t.cuts, (size_t)2 * nctas * 4);
+    carve(t.ncount, (size_t)2 * kMaxPicks * 4);
   }
   carve(t.order, (size_t)nsheds * 4);
   carve(t.gains, (size_t)nsheds * 4);
   carve(t.nbits, cap * nr * row);  // every row is written before it is read
-  if (intervis) {
-    carve(t.nmask, (size_t)kMaxPicks * nr + 16);  // + the 16-byte loads' tail
-  } else {
+  if (local) {
     carve(l.binkey, bins * 8);
     carve(l.binat, bins * 8);
-    carve(l.cand, (size_t)nsheds * 4);
-    carve(l.pos, (size_t)nsheds * 4);
-    carve(l.gain, (size_t)nsheds * 4);
+    carve(l.rec, (size_t)nsheds * 16);
     carve(l.pick, (size_t)cap * 16);
     carve(l.plist, (size_t)nsheds * 8);
+    if (intervis) {
+      carve(l.bincap, bins * 8);
+      carve(l.search, (size_t)nctas * kLocalSearch * 4);
+      carve(l.dom, cells * 16);
+      carve(l.preach, (size_t)nsheds * 8);
+      carve(l.pparent, (size_t)nsheds * 4);
+    }
+  } else {
+    carve(t.nmask, (size_t)kMaxPicks * nr + 16);  // + the 16-byte loads' tail
   }
   t.table = take(site_job_table_bytes(1, nctas));
   if (s) *s = t;
@@ -1129,12 +1148,14 @@ size_t round16(size_t b) { return (b + 15) & ~(size_t)15; }
 }  // namespace
 
 size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis) {
-  return scratch_layout(nrows, nsheds, nctas, roi, intervis, nullptr, nullptr);
+  return scratch_layout(nrows, nsheds, nctas, roi, intervis,
+                        site_is_local(nrows, nsheds, roi, intervis), nullptr, nullptr);
 }
 
 void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,
                         SiteScratch *s) {
-  scratch_layout(nrows, nsheds, nctas, roi, intervis, static_cast<unsigned char *>(base), s);
+  scratch_layout(nrows, nsheds, nctas, roi, intervis, site_is_local(nrows, nsheds, roi, intervis),
+                 static_cast<unsigned char *>(base), s);
 }
 
 // Up to one CTA per SM, about 100 candidates per CTA but at least 32 CTAs:
@@ -1222,7 +1243,7 @@ size_t site_smem_base(int roi, int nsheds, int nctas, int nblocks, int npb, floa
 constexpr size_t kSiteSmemPlan = 220 * 1024;
 constexpr int kMaxNWords = 4096;
 
-constexpr size_t kLocalSmem = 216 * 1024;  // of a job without intervis
+constexpr size_t kLocalSmem = 216 * 1024;  // of a job of site_local
 
 int site_ncap_words(size_t base) {
   if (base >= kSiteSmemPlan) return 0;
@@ -1275,6 +1296,7 @@ SiteArgs make_site_args(const SiteJob &j, int block0) {
   a.stop_area = site_stop_area(j.nrows);
   a.block0 = block0;
   a.local = j.scratch.local;
+  a.use_local = site_is_local(j.nrows, j.nsheds, j.roi, j.intervis);
   a.local_words = (int)((kLocalSmem - sizeof(LocalShared)) / 8);
   return a;
 }
@@ -1295,10 +1317,10 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
     args[i] = make_site_args(jobs[i], total);
     for (int b = 0; b < jobs[i].nctas; b++) block_job.push_back(i);
     total += jobs[i].nctas;
-    shm = std::max(shm, jobs[i].intervis
-                            ? site_smem_bytes(jobs[i].roi, jobs[i].nsheds, jobs[i].nctas,
-                                              jobs[i].nblocks, jobs[i].npb, jobs[i].blocksize)
-                            : kLocalSmem);
+    shm = std::max(shm, args[i].use_local
+                            ? kLocalSmem
+                            : site_smem_bytes(jobs[i].roi, jobs[i].nsheds, jobs[i].nctas,
+                                              jobs[i].nblocks, jobs[i].npb, jobs[i].blocksize));
   }
   if (total == 0) return cudaSuccess;
   // job table: arguments, then the CTA -> job map
@@ -1397,10 +1419,10 @@ cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int3
 // it and must be serialised by the caller.
 namespace {
 
-// Jobs are admitted by the scratch that a selection with intervis takes (16 MiB at
-// most); one without takes up to 24 bytes a candidate and 8 MiB of new bits more.
+// Jobs are admitted by the scratch that a selection in the global order takes (16 MiB at
+// most); site_local takes up to 36 bytes a candidate and 12 MiB more.
 constexpr size_t kNoAllocLimit = size_t(16) << 20;
-constexpr size_t kNoAllocScratchBytes = size_t(40) << 20;  // per device
+constexpr size_t kNoAllocScratchBytes = size_t(48) << 20;  // per device
 
 }  // namespace
 
@@ -1448,7 +1470,8 @@ extern "C" int siting_site_it_noalloc(int nrows, int roi, int intervis, int nshe
   // candidates are taken in any order: one block row holding them all
   const float bs = (float)nrows;
   if (site_smem_bytes(roi, nsheds, G, 1, nsheds, bs) > 220 * 1024) return SITING_EINVAL;
-  if (site_scratch_bytes(nrows, nsheds, G, roi, 1) + 256 > kNoAllocLimit) return SITING_ENOMEM;
+  if (scratch_layout(nrows, nsheds, G, roi, 1, false, nullptr, nullptr) + 256 > kNoAllocLimit)
+    return SITING_ENOMEM;
   const size_t need = site_scratch_bytes(nrows, nsheds, G, roi, intervis) + 256;  // + error flag
   if (need > kNoAllocScratchBytes) return SITING_ENOMEM;
   void *base = nullptr;
