@@ -154,9 +154,9 @@ size_t site_job_table_bytes(int njobs, int total_ctas);
 // kept unchanged until the copy has run; NULL stages through pageable memory.
 cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void *h_stage,
                              cudaStream_t st);
-size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis);
+size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis, int nblocks);
 void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,
-                        SiteScratch *s);
+                        int nblocks, SiteScratch *s);
 int site_default_ctas(int nsheds, int sm_count);
 // The CTA count near G0 that spreads a pick's neighbourhood most evenly over
 // the CTAs for the job's block geometry (nb blocks a row, npb candidates each).

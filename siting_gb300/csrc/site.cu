@@ -1078,9 +1078,13 @@ namespace {
 // other 37 1.01 of it (915^2, radius 16, 93 025: 6.2 ms against 4.0; 1152^2, radius 61,
 // 147 456: 5.3 against 3.2; with fewer candidates 992^2, radius 58, 15 376: 1.7
 // against 1.3).
-bool site_is_local(int nrows, int nsheds, int roi, int intervis) {
+// Observers in no block order (one block) cost the global order more, since every
+// candidate is a possible neighbour of a pick: there the line is 4096 candidates with 64 in a
+// circle (17 jobs up to 16 384: 0.62 of its time; 1500^2, radius 60, 8836: 3.1 ms against
+// 4.6; below it 1.2).
+bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks) {
   const double n2 = (double)nrows * nrows, circle = 3.14159 * roi * roi / n2 * nsheds;
-  return !intervis ||
+  return !intervis || (nblocks <= 1 && nsheds >= 4096 && circle <= 64) ||
          (nsheds >= 16384 && circle <= 512 && (circle <= 64 || 20.0 * nsheds <= n2));
 }
 
@@ -1147,14 +1151,14 @@ size_t round16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 }  // namespace
 
-size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis) {
+size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis, int nblocks) {
   return scratch_layout(nrows, nsheds, nctas, roi, intervis,
-                        site_is_local(nrows, nsheds, roi, intervis), nullptr, nullptr);
+                        site_is_local(nrows, nsheds, roi, intervis, nblocks), nullptr, nullptr);
 }
 
 void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,
-                        SiteScratch *s) {
-  scratch_layout(nrows, nsheds, nctas, roi, intervis, site_is_local(nrows, nsheds, roi, intervis),
+                        int nblocks, SiteScratch *s) {
+  scratch_layout(nrows, nsheds, nctas, roi, intervis, site_is_local(nrows, nsheds, roi, intervis, nblocks),
                  static_cast<unsigned char *>(base), s);
 }
 
@@ -1296,7 +1300,7 @@ SiteArgs make_site_args(const SiteJob &j, int block0) {
   a.stop_area = site_stop_area(j.nrows);
   a.block0 = block0;
   a.local = j.scratch.local;
-  a.use_local = site_is_local(j.nrows, j.nsheds, j.roi, j.intervis);
+  a.use_local = site_is_local(j.nrows, j.nsheds, j.roi, j.intervis, j.nblocks);
   a.local_words = (int)((kLocalSmem - sizeof(LocalShared)) / 8);
   return a;
 }
@@ -1472,14 +1476,14 @@ extern "C" int siting_site_it_noalloc(int nrows, int roi, int intervis, int nshe
   if (site_smem_bytes(roi, nsheds, G, 1, nsheds, bs) > 220 * 1024) return SITING_EINVAL;
   if (scratch_layout(nrows, nsheds, G, roi, 1, false, nullptr, nullptr) + 256 > kNoAllocLimit)
     return SITING_ENOMEM;
-  const size_t need = site_scratch_bytes(nrows, nsheds, G, roi, intervis) + 256;  // + error flag
+  const size_t need = site_scratch_bytes(nrows, nsheds, G, roi, intervis, 1) + 256;  // + error flag
   if (need > kNoAllocScratchBytes) return SITING_ENOMEM;
   void *base = nullptr;
   int rc = noalloc_scratch(&base);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   SiteScratch s;
-  site_carve_scratch(base, nrows, nsheds, G, roi, intervis, &s);
+  site_carve_scratch(base, nrows, nsheds, G, roi, intervis, 1, &s);
   int *d_err = reinterpret_cast<int *>(static_cast<unsigned char *>(base) + need - 256);
   // zero coverage, key lists, cuts, self-check counters, barrier and outputs
   if (cudaMemsetAsync(base, 0, (unsigned char *)s.order - (unsigned char *)base, st) != cudaSuccess ||

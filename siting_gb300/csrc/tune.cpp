@@ -142,10 +142,10 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
               220 * 1024)
         continue;
       void *sp;
-      const size_t sb = site_scratch_bytes(n, g.nwanted, G, p->roi, p->intervis);
+      const size_t sb = site_scratch_bytes(n, g.nwanted, G, p->roi, p->intervis, g.nblocks);
       if ((rc = ws_get(ctx, kSite, sb, &sp))) return rc;
       SiteScratch s;
-      site_carve_scratch(sp, n, g.nwanted, G, p->roi, p->intervis, &s);
+      site_carve_scratch(sp, n, g.nwanted, G, p->roi, p->intervis, g.nblocks, &s);
       float t;
       rc = time_ms(ctx, [&] {
         cudaError_t e = cudaMemsetAsync(sp, 0, (unsigned char *)s.order - (unsigned char *)sp, st);

@@ -1,7 +1,7 @@
 """SITE by local dominance, pick by pick against the sequential greedy.
 
-With intervis it takes over at 16 384 candidates, unless they are dense: both sides of
-that line; window widths of one word and two; candidates in any order
+With intervis it takes over at 16 384 candidates (4096 in no block order, as here),
+unless they are dense: both sides of these lines; window widths of one word and two; candidates in any order
 and on the same cell; one CTA, a few, and the default.  Every result is a whole
 number, so all are compared exactly.
 """
@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n, roi, count, intervis, height", [
     (256, 5, 16384, 1, 10), (256, 5, 16383, 1, 10), (256, 1, 20000, 1, 0), (257, 12, 16641, 1, 60),
     (600, 12, 17000, 1, 60),
+    (200, 4, 4096, 1, 10), (200, 4, 4095, 1, 10), (200, 12, 4096, 1, 10),
     (700, 31, 16400, 1, 150), (700, 32, 16400, 1, 40), (331, 2, 17000, 1, 5),
     (64, 3, 300, 0, 10), (97, 40, 60, 0, 100), (33, 16, 500, 0, 50), (50, 1, 2500, 0, 0),
     (40, 5, 1, 0, 10), (300, 63, 700, 0, 200), (300, 64, 700, 0, 200), (256, 5, 16384, 0, 10),
