@@ -71,6 +71,7 @@ struct ShedArgs {
   const int32_t *obs;
   uint64_t *sheds;
   int *err;
+  int items, chunk;  // quarters: halves of observers in all and to a cluster
 };
 
 // One CTA's share of an observer: rows on one side of it (kHalves = 1, block
@@ -106,14 +107,16 @@ __host__ __device__ __forceinline__ WinGeom win_geom(int roi, int halves, bool s
 // the observer many lanes of a warp meet in one cell, whose stores then merge,
 // where atomic ORs would queue up (at step k about roi/k lanes to a cell).  Line =
 // minor offset, byte = step - 1, an odd number of words a line; one such map
-// for each image and side.
-constexpr int kNearSteps = 16;
-constexpr int kNearLine = kNearSteps + 4;  // bytes
-constexpr int kNearMap = (kNearSteps + 1) * kNearLine;
+// for each image and side.  Large quarters map more steps (quad_near): at radius 200 the
+// ORs' conflicts are a quarter of all shared wavefronts, three in four of them between
+// steps 17 and 48.
+constexpr int kNearSteps = 16, kFarNearSteps = 48;
+__host__ __device__ constexpr int near_line(int steps) { return steps + 4; }  // bytes
+__host__ __device__ constexpr int near_map(int steps) { return (steps + 1) * near_line(steps); }
 
 // Words of the images and near maps.
 __host__ __device__ __forceinline__ int pair_mark_words(int roi, int halves) {
-  return halves * (2 * (roi + 1) * pair_line(roi) + kNearMap);  // 4 maps of kNearMap bytes a side
+  return halves * (2 * (roi + 1) * pair_line(roi) + near_map(kNearSteps));  // 4 maps of bytes a side
 }
 
 size_t pair_smem_bytes(int roi, int halves, bool staged) {
@@ -157,7 +160,8 @@ struct PairRays {
 
 // Steps k..k+3 (k = 1 modulo 4: within one word of the image).  kClamp: a ray's
 // last group, whose steps beyond k1 repeat step k1, which changes nothing.
-template <bool kStaged, bool kRcp, bool kNear, bool kClamp>
+// kNear: the near maps' steps, which mark bytes there; 0: bits of the image.
+template <bool kStaged, bool kRcp, int kNear, bool kClamp>
 __device__ __forceinline__ void pair_group(PairRays &r, int k, int k1) {
   float4 t[4];
   int off[4], ea[4], eb[4], kk[4];
@@ -200,13 +204,13 @@ __device__ __forceinline__ void pair_group(PairRays &r, int k, int k1) {
     // elev + tht >= oalt + hs*k, the right side carried negated
     const unsigned long long nv = f2_fma(f2_mul(r.hs, nk), r.one, r.nalt);
     const unsigned long long v = f2_add(e, r.tht);
-    if constexpr (kNear) {
-      const uint32_t m = r.near + (uint32_t)(off[i] * kNearLine + kk[i] - 1);
+    if constexpr (kNear > 0) {
+      const uint32_t m = r.near + (uint32_t)(off[i] * near_line(kNear) + kk[i] - 1);
       asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\t@p st.shared.u8 [%0], %3;\n\t}" ::"r"(m),
                    "f"(f2_lo(v)), "f"(-f2_lo(nv)), "r"(1)
                    : "memory");
       asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\t@p st.shared.u8 [%0+%4], %3;\n\t}" ::"r"(m),
-                   "f"(f2_hi(v)), "f"(-f2_hi(nv)), "r"(1), "n"(kNearMap)
+                   "f"(f2_hi(v)), "f"(-f2_hi(nv)), "r"(1), "n"(near_map(kNear))
                    : "memory");
     } else {
       // an invisible cell ORs nothing: a predicated OR would be a branch, with no
@@ -251,44 +255,48 @@ __device__ __forceinline__ void pair_last(float sl, int roi, int majA, int minA,
 }
 
 // Steps k..k1 (k = 1 modulo 4).
-template <bool kStaged, bool kRcp>
+template <bool kStaged, bool kRcp, int kNear>
 __device__ __forceinline__ void pair_steps(PairRays &r, int k, int k1) {
   r.pA = r.p0 + (k - 1) * r.mA;
   r.pB = r.p0 + (k - 1) * r.mB;
-  for (; k <= kNearSteps && k + 3 <= k1; k += 4) pair_group<kStaged, kRcp, true, false>(r, k, k1);
-  for (; k + 3 <= k1; k += 4) pair_group<kStaged, kRcp, false, false>(r, k, k1);
+  for (; k <= kNear && k + 3 <= k1; k += 4) pair_group<kStaged, kRcp, kNear, false>(r, k, k1);
+  for (; k + 3 <= k1; k += 4) pair_group<kStaged, kRcp, 0, false>(r, k, k1);
   if (k > k1) return;
-  if (k <= kNearSteps)
-    pair_group<kStaged, kRcp, true, true>(r, k, k1);
+  if (k <= kNear)
+    pair_group<kStaged, kRcp, kNear, true>(r, k, k1);
   else
-    pair_group<kStaged, kRcp, false, true>(r, k, k1);
+    pair_group<kStaged, kRcp, 0, true>(r, k, k1);
 }
 
 // Sweeps A to step kA and B to step kB: first both rays to the nearer end, then,
 // where the ends differ, the longer one alone; the other stays at the observer
 // with its targets out of sight.
-template <bool kStaged, bool kRcp>
+template <bool kStaged, bool kRcp, int kNear>
 __device__ __forceinline__ void pair_sweep(PairRays &r, int kA, int kB) {
   const int kmin = min(kA, kB);
-  pair_steps<kStaged, kRcp>(r, 1, kmin);
+  pair_steps<kStaged, kRcp, kNear>(r, 1, kmin);
   if (kA != kB) {
     const bool a_on = kA > kB;
     r.tht = a_on ? f2_pack(f2_lo(r.tht), -3e38f) : f2_pack(-3e38f, f2_hi(r.tht));
     if (!a_on) r.mA = r.sA = 0;
     if (a_on) r.mB = r.sB = 0;
     // from the last group on again: a step done twice changes nothing
-    pair_steps<kStaged, kRcp>(r, (kmin & ~3) + 1, max(kA, kB));
+    pair_steps<kStaged, kRcp, kNear>(r, (kmin & ~3) + 1, max(kA, kB));
   }
 }
 
-// Packs line `line` of a near map to the 16 bits of its steps.
-__device__ __forceinline__ unsigned near_bits(const unsigned char *map, int line) {
-  const unsigned *src = reinterpret_cast<const unsigned *>(map + line * kNearLine);
-  unsigned bits = 0;
+// ORs line `line` of a near map into the words of an image line, two apart.
+template <int kNear>
+__device__ __forceinline__ void near_bits(const unsigned char *map, int line, unsigned *dst) {
+  const unsigned *src = reinterpret_cast<const unsigned *>(map + line * near_line(kNear));
 #pragma unroll
-  for (int j = 0; j < kNearSteps / 4; j++)  // four bytes of 0 or 1 to a nibble
-    bits |= (src[j] * 0x01020408u) >> 24 << (4 * j);
-  return bits;
+  for (int w = 0; w < (kNear + 31) / 32; w++) {
+    unsigned bits = 0;
+#pragma unroll
+    for (int j = 0; j < 8 && w * 8 + j < kNear / 4; j++)  // four bytes of 0 or 1 to a nibble
+      bits |= (src[w * 8 + j] * 0x01020408u) >> 24 << (4 * j);
+    if (bits) dst[2 * w] |= bits;
+  }
 }
 
 template <int kHalves, bool kStaged, bool kRcp>
@@ -376,12 +384,12 @@ __global__ void __launch_bounds__(448, 2)
     asm("ld.shared.f32 %0, [%1];" : "=f"(one) : "r"(smem_u32(tab + 1)));  // RN(1/1)
     r.one = f2_pack(one, one);
     r.img = smem_u32(img + ((kHalves == 2 && half ? 2 : 0) + (xm ? 0 : 1)) * ximg);
-    r.near = smem_u32(near + ((kHalves == 2 && half ? 2 : 0) + (xm ? 0 : 1)) * 2 * kNearMap);
+    r.near = smem_u32(near + ((kHalves == 2 && half ? 2 : 0) + (xm ? 0 : 1)) * 2 * near_map(kNearSteps));
     r.ls4 = 4 * ls;
     r.tab = tab;
     r.hs = f2_pack(kNoHorizon, kNoHorizon);
     r.tht = f2_pack(tht, tht);
-    pair_sweep<kStaged, kRcp>(r, kA, kB);
+    pair_sweep<kStaged, kRcp, kNearSteps>(r, kA, kB);
     if (kStaged) break;
   }
   __syncthreads();
@@ -390,7 +398,8 @@ __global__ void __launch_bounds__(448, 2)
   const int nlines = min(roi, kNearSteps) + 1;
   for (int i = tid; i < kHalves * 4 * nlines; i += blockDim.x) {
     const int map = i / nlines, line = i - map * nlines;
-    img[(map >> 1) * ximg + line * ls + (map & 1)] |= near_bits(near + map * kNearMap, line);
+    near_bits<kNearSteps>(near + map * near_map(kNearSteps), line,
+                          img + (map >> 1) * ximg + line * ls + (map & 1));
   }
   __syncthreads();
 
@@ -445,9 +454,15 @@ __global__ void __launch_bounds__(448, 2)
 // A quarter of an observer a CTA, for radii whose half windows leave one CTA an
 // SM.  The pairs mirror about the quadrant's diagonal: A is x-major, B y-major, so
 // one image holds both (A: line = column distance, bit = row distance - 1; B: line
-// = row distance, bit = column distance - 1).  Block 4o + 2*lower + left of observer
-// o; the two sides of a row share the word of the observer's column, so they form a
-// cluster and the left one hands its bits of that word to the right one.
+// = row distance, bit = column distance - 1).  The two sides of a row share the word
+// of the observer's column, so they form a cluster and the left one hands its bits of
+// that word to the right one.  A cluster takes `chunk` halves (2o + lower of observer o)
+// in turn.
+//
+// At radius 200 two CTAs (14 warps) fill an SM: 58% of issue slots, shared-memory
+// pipe 68%, a quarter of the warps' time at the barriers between the sweep and the rows
+// out.  Reading a group's elevations ahead of the marks before them does not help (1.14
+// -> 1.17 ms).
 __host__ __device__ __forceinline__ WinGeom quad_geom(int roi) {
   WinGeom g;
   g.w = ((roi + 1 + 7 + 7) & ~7) | 8;
@@ -457,144 +472,164 @@ __host__ __device__ __forceinline__ WinGeom quad_geom(int roi) {
 }
 
 // Words of the image and the two near maps.
-__host__ __device__ __forceinline__ int quad_mark_words(int roi) {
-  return (roi + 1) * pair_line(roi) + kNearMap / 2;
+__host__ __device__ __forceinline__ int quad_mark_words(int roi, int near) {
+  return (roi + 1) * pair_line(roi) + near_map(near) / 2;
 }
 
-size_t quad_smem_bytes(int roi) {
+size_t quad_smem_bytes(int roi, int near) {
   return quad_geom(roi).bytes() + (size_t)(roi + 1) * (16 + 8) + 16 +
-         (((size_t)quad_mark_words(roi) * 4 + 15) & ~(size_t)15) + 16;
+         (((size_t)quad_mark_words(roi, near) * 4 + 15) & ~(size_t)15) + 16;
 }
 
 constexpr int kQuadMaxThreads = 320;
 
+template <int kNear>
 __global__ void __cluster_dims__(2) __launch_bounds__(kQuadMaxThreads, 2)
     shed_quad_kernel(const __grid_constant__ CUtensorMap map, const ShedArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
   const int roi = a.roi, n = a.n, nr = 2 * roi + 1, nwpr = (nr + 63) / 64, nwords = nr * nwpr;
-  const int obi = (int)(blockIdx.x >> 2), half = (int)(blockIdx.x >> 1) & 1;
   const bool left = blockIdx.x & 1u;
-  uint64_t *dst = a.sheds + (size_t)obi * nwords;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  const int ob = a.obs[obi];
-  if (ob < 0 || ob >= n * n) {  // invalid observer: empty shed, flagged (by the whole cluster)
-    const int wr0 = half ? roi + 1 : 0, wr1 = half ? nr : roi + 1;
-    if (!left)
-      for (int i = wr0 * nwpr + tid; i < wr1 * nwpr; i += blockDim.x) dst[i] = 0ull;
-    if (tid == 0) atomicOr(a.err, kErrBadInput);
-    return;
-  }
-  const int ox = ob / n, oy = ob - (ob / n) * n;
   const WinGeom g = quad_geom(roi);
   const int W2 = 2 * g.w, nw = pair_words(roi), ls = pair_line(roi);
-  const int hx0 = half ? ox : ox - roi;                 // window origin
-  const int hy0 = (left ? oy - roi : oy) & ~7;          // TMA inner coordinate: 16-byte aligned
   const uint32_t win = smem_u32(sm);
   float4 *tab = reinterpret_cast<float4 *>(sm + g.bytes());
   uint64_t *mbar = reinterpret_cast<uint64_t *>(tab + roi + 1);
   uint64_t *cbuf = mbar + 2;  // the left side's bits of the shared word, by row distance
   unsigned *img = reinterpret_cast<unsigned *>(cbuf + ((roi + 2) & ~1));
   unsigned char *near = reinterpret_cast<unsigned char *>(img + (roi + 1) * ls);
-  if (tid == 0) {
-    mbar_init(mbar, 1);
+  auto valid = [&](int ob) { return ob >= 0 && ob < n * n; };
+  auto load = [&](int item, int ob) {  // the item's window, by one thread
+    const int ox = ob / n, oy = ob - ox * n;
+    const int hx0 = item & 1 ? ox : ox - roi, hy0 = (left ? oy - roi : oy) & ~7;
     mbar_expect_tx(mbar, (uint32_t)g.bytes());
     for (int b = 0; b < g.nboxes; b++)
       tma_load_window(sm + (size_t)b * g.box_rows * W2, &map, hy0, hx0 + b * g.box_rows, mbar);
+  };
+  int item = (int)(blockIdx.x >> 1) * a.chunk;
+  const int end = min(a.items, item + a.chunk);
+  int ob = __ldg(a.obs + (item >> 1));
+  if (tid == 0) {
+    mbar_init(mbar, 1);
+    if (valid(ob)) load(item, ob);
   }
   for (int i = tid; i <= roi; i += blockDim.x) {
     const float y = i ? __frcp_rn((float)i) : 0.f;
     tab[i] = make_float4(y, y, -(float)i, -(float)i);
   }
-  for (int i = tid; i < (quad_mark_words(roi) + 3) / 4; i += blockDim.x)
-    reinterpret_cast<uint4 *>(img)[i] = make_uint4(0u, 0u, 0u, 0u);
-  __syncthreads();
-  cluster_arrive();  // the peer may write to cbuf once this CTA runs
-  if (__all_sync(0xffffffffu, mbar_wait(mbar, 0))) {
-    if (const int t = tid; t <= roi) {
-      // every second ray, as in the half windows
-      const int evens = (roi + 2) / 2, m = t < evens ? 2 * t : 2 * (t - evens) + 1;
-      const float sl = fdiv(i2f(m), i2f(roi));
-      const int rowlim = half ? n - 1 - ox : ox, collim = left ? oy : n - 1 - oy;
-      int kA, kB;
-      pair_last(sl, roi, rowlim, collim, collim, rowlim, kA, kB);
-      const int rowstep = half ? W2 : -W2, cell = left ? -2 : 2;
-      const int p0 = (int)win + (ox - hx0) * W2 + 2 * (oy - hy0);
-      PairRays r;
-      r.dem = a.dem;
-      r.p0 = p0;
-      r.mA = r.sB = rowstep;
-      r.mB = r.sA = cell;
-      r.sl = sl;
-        const float nalt = -i2f(elevation<true>(a.dem, p0) + a.oht), tht = i2f(a.tht);
-      r.nalt = f2_pack(nalt, nalt);
-        float one;
-      asm("ld.shared.f32 %0, [%1];" : "=f"(one) : "r"(smem_u32(tab + 1)));  // RN(1/1)
-      r.one = f2_pack(one, one);
-      r.img = smem_u32(img);
-      r.near = smem_u32(near);
-      r.ls4 = 4 * ls;
-      r.tab = tab;
-      r.hs = f2_pack(kNoHorizon, kNoHorizon);
-      r.tht = f2_pack(tht, tht);
-      pair_sweep<true, true>(r, kA, kB);
-    }
-  } else if (tid == 0) {
-    atomicOr(a.err, kErrTmaTimeout);
-  }
-  __syncthreads();
-  const int nlines = min(roi, kNearSteps) + 1;
-  for (int i = tid; i < 2 * nlines; i += blockDim.x) {
-    const int map = i >= nlines, line = i - map * nlines;
-    img[line * ls + map] |= near_bits(near + map * kNearMap, line);
-  }
-  __syncthreads();
-  // A into B, as X into Y above
-  for (int b = warp; b < nw * nw; b += nwarps) {
-    const int lb = b / nw, w = b - lb * nw, line = lb * 32 + 1 + lane;
-    unsigned x = line <= roi ? img[line * ls + 2 * w] : 0u;
-    if (!__any_sync(0xffffffffu, x != 0u)) continue;
-    x = warp_transpose(x, lane);
-    const int d = w * 32 + 1 + lane;
-    if (d <= roi && x) img[d * ls + 2 * lb + 1] |= x;
-  }
-  __syncthreads();
-  // rows out (see shed_kernel): this side's words, the shared word by the right one
-  const int S = 64 * nwpr - 1 - roi, qc = nwpr - 1 - (S >> 6);
-  const int q0 = left ? 0 : qc, nq = left ? qc + 1 : nwpr - qc;
-  const int per = blockDim.x / nq, q = q0 + tid % nq, z = 2 * (nwpr - 1 - q);
-  const int s0 = left ? 32 * z - (S + 1) : S - 1 - 32 * z - 63, si = s0 >> 5, sh = s0 & 31;
-  auto word = [&](int d) {  // the string's 64 bits of word q, row distance d
-    const unsigned *line = img + d * ls + 1;
-    auto at = [&](int i) { return (unsigned)i < (unsigned)nw ? line[2 * i] : 0u; };
-    const unsigned w0 = at(si), w1 = at(si + 1), w2 = at(si + 2);
-    const unsigned lo = __funnelshift_r(w0, w1, sh), hi = __funnelshift_r(w1, w2, sh);
-    return left ? ((uint64_t)hi << 32) | lo : ((uint64_t)__brev(lo) << 32) | __brev(hi);
-  };
-  const int r0 = tid / nq + half;  // row distances half..roi
-  const bool mine = tid < per * nq;
-  __syncwarp();
-  cluster_wait();
-  if (left && mine) {
-    for (int d = r0; d <= roi; d += per) {
-      const uint64_t v = word(d);
-      if (q == qc)
-        cluster_store_u64(smem_u32(cbuf + d), 0, v);
-      else
-        dst[(half ? roi + d : roi - d) * nwpr + q] = v;
-    }
-  }
-  __syncwarp();
-  cluster_arrive();
-  cluster_wait();
-  if (!left && mine) {
-    for (int d = r0; d <= roi; d += per) {
-      uint64_t v = word(d);
-      if (q == qc) {
-        const unsigned c = d == 0 ? 1u : (img[2 * ((d - 1) >> 5)] >> ((d - 1) & 31)) & 1u;
-        v |= cbuf[d] | (uint64_t)c << (S & 63);
+  unsigned parity = 0;
+  for (; item < end; item++) {
+    const int half = item & 1, next = item + 1 < end ? __ldg(a.obs + ((item + 1) >> 1)) : -1;
+    uint64_t *dst = a.sheds + (size_t)(item >> 1) * nwords;
+    if (!valid(ob)) {  // invalid observer: empty shed, flagged (by the whole cluster)
+      const int wr0 = half ? roi + 1 : 0, wr1 = half ? nr : roi + 1;
+      if (!left)
+        for (int i = wr0 * nwpr + tid; i < wr1 * nwpr; i += blockDim.x) dst[i] = 0ull;
+      if (tid == 0) {
+        atomicOr(a.err, kErrBadInput);
+        if (valid(next)) load(item + 1, next);
       }
-      dst[(half ? roi + d : roi - d) * nwpr + q] = v;
+      ob = next;
+      continue;
     }
+    const int ox = ob / n, oy = ob - (ob / n) * n;
+    const int hx0 = half ? ox : ox - roi;                 // window origin
+    const int hy0 = (left ? oy - roi : oy) & ~7;          // TMA inner coordinate: 16-byte aligned
+    for (int i = tid; i < (quad_mark_words(roi, kNear) + 3) / 4; i += blockDim.x)
+      reinterpret_cast<uint4 *>(img)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    cluster_arrive();  // the peer may write to cbuf once this CTA runs
+    if (__all_sync(0xffffffffu, mbar_wait(mbar, parity))) {
+      if (const int t = tid; t <= roi) {
+        // every second ray, as in the half windows
+        const int evens = (roi + 2) / 2, m = t < evens ? 2 * t : 2 * (t - evens) + 1;
+        const float sl = fdiv(i2f(m), i2f(roi));
+        const int rowlim = half ? n - 1 - ox : ox, collim = left ? oy : n - 1 - oy;
+        int kA, kB;
+        pair_last(sl, roi, rowlim, collim, collim, rowlim, kA, kB);
+        const int rowstep = half ? W2 : -W2, cell = left ? -2 : 2;
+        const int p0 = (int)win + (ox - hx0) * W2 + 2 * (oy - hy0);
+        PairRays r;
+        r.dem = a.dem;
+        r.p0 = p0;
+        r.mA = r.sB = rowstep;
+        r.mB = r.sA = cell;
+        r.sl = sl;
+        const float nalt = -i2f(elevation<true>(a.dem, p0) + a.oht), tht = i2f(a.tht);
+        r.nalt = f2_pack(nalt, nalt);
+        float one;
+        asm("ld.shared.f32 %0, [%1];" : "=f"(one) : "r"(smem_u32(tab + 1)));  // RN(1/1)
+        r.one = f2_pack(one, one);
+        r.img = smem_u32(img);
+        r.near = smem_u32(near);
+        r.ls4 = 4 * ls;
+        r.tab = tab;
+        r.hs = f2_pack(kNoHorizon, kNoHorizon);
+        r.tht = f2_pack(tht, tht);
+        pair_sweep<true, true, kNear>(r, kA, kB);
+      }
+    } else if (tid == 0) {
+      atomicOr(a.err, kErrTmaTimeout);
+    }
+    parity ^= 1u;
+    __syncthreads();
+    if (tid == 0 && valid(next)) load(item + 1, next);  // the window is free
+    const int nlines = min(roi, kNear) + 1;
+    for (int i = tid; i < 2 * nlines; i += blockDim.x) {
+      const int map = i >= nlines, line = i - map * nlines;
+      near_bits<kNear>(near + map * near_map(kNear), line, img + line * ls + map);
+    }
+    __syncthreads();
+    // A into B, as X into Y above
+    for (int b = warp; b < nw * nw; b += nwarps) {
+      const int lb = b / nw, w = b - lb * nw, line = lb * 32 + 1 + lane;
+      unsigned x = line <= roi ? img[line * ls + 2 * w] : 0u;
+      if (!__any_sync(0xffffffffu, x != 0u)) continue;
+      x = warp_transpose(x, lane);
+      const int d = w * 32 + 1 + lane;
+      if (d <= roi && x) img[d * ls + 2 * lb + 1] |= x;
+    }
+    __syncthreads();
+    // rows out (see shed_kernel): this side's words, the shared word by the right one
+    const int S = 64 * nwpr - 1 - roi, qc = nwpr - 1 - (S >> 6);
+    const int q0 = left ? 0 : qc, nq = left ? qc + 1 : nwpr - qc;
+    const int per = blockDim.x / nq, q = q0 + tid % nq, z = 2 * (nwpr - 1 - q);
+    const int s0 = left ? 32 * z - (S + 1) : S - 1 - 32 * z - 63, si = s0 >> 5, sh = s0 & 31;
+    auto word = [&](int d) {  // the string's 64 bits of word q, row distance d
+      const unsigned *line = img + d * ls + 1;
+      auto at = [&](int i) { return (unsigned)i < (unsigned)nw ? line[2 * i] : 0u; };
+      const unsigned w0 = at(si), w1 = at(si + 1), w2 = at(si + 2);
+      const unsigned lo = __funnelshift_r(w0, w1, sh), hi = __funnelshift_r(w1, w2, sh);
+      return left ? ((uint64_t)hi << 32) | lo : ((uint64_t)__brev(lo) << 32) | __brev(hi);
+    };
+    const int r0 = tid / nq + half;  // row distances half..roi
+    const bool mine = tid < per * nq;
+    __syncwarp();
+    cluster_wait();
+    if (left && mine) {
+      for (int d = r0; d <= roi; d += per) {
+        const uint64_t v = word(d);
+        if (q == qc)
+          cluster_store_u64(smem_u32(cbuf + d), 0, v);
+        else
+          dst[(half ? roi + d : roi - d) * nwpr + q] = v;
+      }
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (!left && mine) {
+      for (int d = r0; d <= roi; d += per) {
+        uint64_t v = word(d);
+        if (q == qc) {
+          const unsigned c = d == 0 ? 1u : (img[2 * ((d - 1) >> 5)] >> ((d - 1) & 31)) & 1u;
+          v |= cbuf[d] | (uint64_t)c << (S & 63);
+        }
+        dst[(half ? roi + d : roi - d) * nwpr + q] = v;
+      }
+    }
+    __syncthreads();  // the images are free
+    ob = next;
   }
 }
 
@@ -628,8 +663,10 @@ ShedPlan shed_staged_plan(int roi, bool half) {
   if (roi < 1) return shed_l1_plan(roi);
   if (!half && 4 * roi + 1 <= kPairMaxThreads && pair_smem_bytes(roi, 2, true) <= kMaxSmem)
     return ShedPlan{pair_threads(4 * roi + 1), true, false, false};
-  const bool quad_fits = (roi + 1 + 31) / 32 * 32 <= kQuadMaxThreads && quad_smem_bytes(roi) <= kMaxSmem;
-  if (roi >= kQuadMinRoi && quad_smem_bytes(roi) <= kTwoCtaSmem) return shed_quad_plan(roi);
+  const bool quad_fits =
+      (roi + 1 + 31) / 32 * 32 <= kQuadMaxThreads && quad_smem_bytes(roi, kNearSteps) <= kMaxSmem;
+  if (roi >= kQuadMinRoi && quad_smem_bytes(roi, kNearSteps) <= kTwoCtaSmem)
+    return shed_quad_plan(roi);
   if (pair_smem_bytes(roi, 1, true) <= kMaxSmem)
     return ShedPlan{pair_threads(2 * roi + 1), true, true, false};
   return quad_fits ? shed_quad_plan(roi) : shed_l1_plan(roi);
@@ -637,8 +674,22 @@ ShedPlan shed_staged_plan(int roi, bool half) {
 
 }  // namespace
 
+namespace {
+
+// Steps of a quarter's near maps: 48 where they leave as many CTAs an SM as 16 (ms at
+// 2048^2 with 16 and 48: roi 137 0.986, 0.972; 200 1.130, 1.080; 208 1.061, 1.031; at 170
+// 48 would cost the third CTA: 0.989, 1.248).
+int quad_near(int roi) {
+  auto ctas = [&](int steps) { return 228 * 1024 / (quad_smem_bytes(roi, steps) + 1024); };
+  return quad_smem_bytes(roi, kFarNearSteps) <= kMaxSmem && ctas(kFarNearSteps) == ctas(kNearSteps)
+             ? kFarNearSteps
+             : kNearSteps;
+}
+
+}  // namespace
+
 size_t shed_smem_bytes(const ShedPlan &p, int roi) {
-  return p.quad ? quad_smem_bytes(roi) : pair_smem_bytes(roi, p.half ? 1 : 2, p.use_smem);
+  return p.quad ? quad_smem_bytes(roi, quad_near(roi)) : pair_smem_bytes(roi, p.half ? 1 : 2, p.use_smem);
 }
 
 ShedPlan shed_default_plan(int roi) { return shed_staged_plan(roi, roi >= kHalfMinRoi); }
@@ -659,7 +710,7 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
   const size_t nr = 2 * (size_t)roi + 1, w32 = (nr + 31) / 32, w64 = (nr + 63) / 64;
   if (4 * (nr * (2 * w64 | 1) + 32 * w32 * (w32 | 1) + roi + 1) + 16 > 227 * 1024)
     return cudaErrorInvalidValue;
-  const ShedArgs a{dem.data, dem.pitch, dem.nrows, roi, oht, tht, obs, sheds, d_err};
+  ShedArgs a{dem.data, dem.pitch, dem.nrows, roi, oht, tht, obs, sheds, d_err, 2 * nsheds, 1};
   // the reciprocal-table division is exhaustively checked for |a| <= 2^21
   // (heights up to 10^6 over 16-bit elevations) and steps up to 2048
   const bool rcp = oht >= 0 && oht <= 1000000;
@@ -672,12 +723,25 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
     if (!make_dem_tensor_map(&map, dem, g.w, g.box_rows)) return cudaErrorInvalidValue;
   }
   auto kern = !eff.use_smem ? (rcp ? shed_kernel<1, false, true> : shed_kernel<1, false, false>)
-              : eff.quad    ? shed_quad_kernel
+              : eff.quad    ? (quad_near(roi) == kNearSteps ? shed_quad_kernel<kNearSteps>
+                                                            : shed_quad_kernel<kFarNearSteps>)
               : eff.half    ? shed_kernel<1, true, true>
                             : shed_kernel<2, true, true>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
   if (e != cudaSuccess) return e;
-  kern<<<nsheds * (eff.quad ? 4 : eff.half ? 2 : 1), eff.threads, shm, st>>>(map, a);
+  int grid = nsheds * (eff.half ? 2 : 1);
+  if (eff.quad) {
+    // One CTA an SM has nothing to run while a window arrives: there a cluster takes up
+    // to 4 halves in turn and asks for the next window when the rays of one are done (roi
+    // 216 1.69 -> 1.63 ms, 240 1.56 -> 1.46, 300 1.46 -> 1.37), in 8 or more rounds of
+    // clusters.  With two CTAs an SM their ends overlap anyhow (200: 1.08, 1.15).
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (shm > kTwoCtaSmem) a.chunk = std::max(1, std::min(4, a.items / (8 * std::max(1, sms / 2))));
+    grid = 2 * ceil_div(a.items, a.chunk);
+  }
+  kern<<<grid, eff.threads, shm, st>>>(map, a);
   return cudaGetLastError();
 }
 

@@ -60,3 +60,18 @@ def test_many_observers_random_sizes(native, oracle):
         with native.Context(0) as ctx:
             got = ctx.calc_sheds(n, dem, roi, 7, 3, obs)
         assert np.array_equal(got, oracle.sheds(dem, n, roi, 7, 3, obs))
+
+
+def test_a_cluster_takes_several_quarters(native, oracle):
+    # one CTA an SM from radius 216 on; 1300 observers give each cluster four halves
+    n, roi = 470, 216
+    dem = native.fbm_dem(n, seed=3, octaves=7, range_max=40000)
+    obs = _observers(n, roi, 1300, 3)
+    want = oracle.sheds(dem, n, roi, 60, 5, obs)
+    with native.Context(0) as ctx:
+        assert np.array_equal(ctx.calc_sheds(n, dem, roi, 60, 5, obs), want)
+        bad = obs.copy()
+        bad[[0, 5, 6, 641]] = n * n, -1, n * n + 7, -5  # first, inside and last of a cluster's
+        with pytest.raises(native.SitingError):
+            ctx.calc_sheds(n, dem, roi, 60, 5, bad)
+        assert np.array_equal(ctx.calc_sheds(n, dem, roi, 60, 5, obs), want)
