@@ -72,7 +72,14 @@ struct ShedArgs {
   uint64_t *sheds;
   int *err;
   int items, chunk;  // quarters: halves of observers in all and to a cluster
+  unsigned long long rn;  // ceil(2^64/n)
+  unsigned rw;            // ceil(2^16/nwpr): a thread's number by nwpr
 };
+
+// floor(v / n), 0 <= v < 2^31: v*rn exceeds 2^64*v/n by less than 2^64/n.
+__device__ __forceinline__ int div_n(int v, const ShedArgs &a) {
+  return a.n > 1 ? (int)__umul64hi((unsigned long long)(unsigned)v, a.rn) : v;
+}
 
 // One CTA's share of an observer: rows on one side of it (kHalves = 1, block
 // 2o the upper side of observer o, 2o+1 the lower) or all (kHalves = 2).
@@ -225,6 +232,16 @@ __device__ __forceinline__ void pair_group(PairRays &r, int k, int k1) {
   }
 }
 
+// RN(m/k) by the table entry of k, as in pair_group.  (Whole and half windows are half
+// ends at small radii: this, the search of pair_last from within a step of the end, and
+// the divisions by n and nwpr as products took roi 30 from 0.705 to 0.655 ms at 2048^2,
+// 1.6 G cells of rays, 74 1.039 to 0.997, 118 0.957 to 0.925; the long sweeps of the
+// quarters gain nothing by the first and the last.)
+__device__ __forceinline__ float step_slope(const float4 &t, int m) {
+  const float a = i2f(m), q = fmul(a, t.x);
+  return __fmaf_rn(__fmaf_rn(q, t.z, a), t.x, q);
+}
+
 // Steps of the two rays of slope sl.  A ray stops outside the roi circle, at
 // the DEM edge along the major axis (maj cells away), or when the minor
 // coordinate leaves the DEM (min cells away) (siting.cpp:333-334); the offset
@@ -233,9 +250,9 @@ __device__ __forceinline__ void pair_last(float sl, int roi, int majA, int minA,
                                           int &kA, int &kB) {
   const int roi2 = roi * roi;
   auto off = [&](int k) { return f2i(fadd(fmul(i2f(k), sl), 0x1.fffffep-2f)); };
-  // the rounded offset moves the circle's crossing by less than a step from the
-  // straight line's, so the search starts just beyond that
-  int kc = min(roi, (int)(i2f(roi) * rsqrtf(1.f + sl * sl)) + 2);
+  // an offset at most half below the line lets the ray stay inside the circle for at
+  // most sl/(2 + 2*sl^2) <= 1/4 step longer than the line, so the search starts there
+  int kc = min(roi, (int)(i2f(roi) * rsqrtf(1.f + sl * sl) + 0.2525f));
   for (int o = off(kc); kc * kc + o * o > roi2; o = off(kc)) kc--;
   auto last = [&](int hi, int lim) {  // the last step <= hi with offset <= lim
     int lo = 0;
@@ -316,7 +333,7 @@ __global__ void __launch_bounds__(448, 2)
     if (tid == 0) atomicOr(a.err, kErrBadInput);
     return;
   }
-  const int ox = ob / n, oy = ob - (ob / n) * n;
+  const int ox = div_n(ob, a), oy = ob - ox * n;
   const WinGeom g = win_geom(roi, kHalves, kStaged);
   const int W2 = 2 * g.w, nw = pair_words(roi);  // W2: row pitch, bytes
   const int ls = pair_line(roi), ximg = (roi + 1) * ls;  // words of an image
@@ -361,7 +378,7 @@ __global__ void __launch_bounds__(448, 2)
     const int m = (mt < evens ? 2 * mt : 2 * (mt - evens) + 1) + (xm ? 0 : half);
     const int rowlim = half ? n - 1 - ox : ox;  // rows on this side of the observer
     const int collimA = n - 1 - oy, collimB = oy;
-    const float sl = fdiv(i2f(m), i2f(roi));
+    const float sl = kRcp ? step_slope(tab[roi], m) : fdiv(i2f(m), i2f(roi));
     int kA, kB;
     pair_last(sl, roi, xm ? rowlim : collimA, xm ? collimA : rowlim, xm ? rowlim : collimB,
               xm ? collimB : rowlim, kA, kB);
@@ -395,9 +412,10 @@ __global__ void __launch_bounds__(448, 2)
   __syncthreads();
 
   // ---- near maps into the images: a thread packs a line
-  const int nlines = min(roi, kNearSteps) + 1;
-  for (int i = tid; i < kHalves * 4 * nlines; i += blockDim.x) {
-    const int map = i / nlines, line = i - map * nlines;
+  const int nlines = min(roi, kNearSteps) + 1, lsh2 = 32 - __clz(nlines - 1);  // lines, as 2^lsh2 slots
+  for (int i = tid; i < kHalves * 4 << lsh2; i += blockDim.x) {
+    const int map = i >> lsh2, line = i - (map << lsh2);
+    if (line >= nlines) continue;
     near_bits<kNearSteps>(near + map * near_map(kNearSteps), line,
                           img + (map >> 1) * ximg + line * ls + (map & 1));
   }
@@ -425,12 +443,13 @@ __global__ void __launch_bounds__(448, 2)
   // 1) starts at S+1 and the right one runs downwards from S-1.
   // A thread keeps one word column q, so that its string positions are fixed.
   const int S = 64 * nwpr - 1 - roi;
-  const int per = blockDim.x / nwpr;  // rows a pass (blockDim >= 64 > nwpr)
-  const int q = tid % nwpr, z = 2 * (nwpr - 1 - q);  // bits 32z..32z+63
+  auto by_nwpr = [&](int t) { return (int)((unsigned)t * a.rw >> 16); };
+  const int per = by_nwpr(blockDim.x);  // rows a pass (blockDim >= 64 > nwpr)
+  const int tr = by_nwpr(tid), q = tid - tr * nwpr, z = 2 * (nwpr - 1 - q);  // bits 32z..32z+63
   const int l0 = 32 * z - (S + 1), r0 = S - 1 - 32 * z - 31;
   const int li = l0 >> 5, ri = r0 >> 5, lsh = l0 & 31, rsh = r0 & 31;
   const bool centre = (S >> 6) == (z >> 1);
-  for (int row = wr0 + tid / nwpr; row < wr1; row += per) {
+  for (int row = wr0 + tr; row < wr1; row += per) {
     if (tid >= per * nwpr) break;
     const int d = abs(row - roi), hb = kHalves == 2 && row > roi;
     const unsigned *X = img + hb * 2 * ximg, *line = X + ximg + d * ls;
@@ -710,7 +729,8 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
   const size_t nr = 2 * (size_t)roi + 1, w32 = (nr + 31) / 32, w64 = (nr + 63) / 64;
   if (4 * (nr * (2 * w64 | 1) + 32 * w32 * (w32 | 1) + roi + 1) + 16 > 227 * 1024)
     return cudaErrorInvalidValue;
-  ShedArgs a{dem.data, dem.pitch, dem.nrows, roi, oht, tht, obs, sheds, d_err, 2 * nsheds, 1};
+  ShedArgs a{dem.data, dem.pitch, dem.nrows, roi, oht, tht, obs, sheds, d_err, 2 * nsheds, 1,
+             ~0ull / (unsigned)dem.nrows + 1ull, 65536u / (unsigned)w64 + 1u};
   // the reciprocal-table division is exhaustively checked for |a| <= 2^21
   // (heights up to 10^6 over 16-bit elevations) and steps up to 2048
   const bool rcp = oht >= 0 && oht <= 1000000;
