@@ -73,7 +73,7 @@ struct ShedArgs {
   int *err;
   int items, chunk;  // quarters: halves of observers in all and to a cluster
   unsigned long long rn;  // ceil(2^64/n)
-  unsigned rw;            // ceil(2^16/nwpr): a thread's number by nwpr
+  unsigned rw, rb;        // ceil(2^16/nwpr), ceil(2^16/nw): a thread's or block's number by these
 };
 
 // floor(v / n), 0 <= v < 2^31: v*rn exceeds 2^64*v/n by less than 2^64/n.
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(448, 2)
   const int nblk = nw * nw * 2;
   for (int b0 = warp; b0 < kHalves * nblk; b0 += nwarps) {
     const int hb = kHalves == 2 && b0 >= nblk, b = b0 - hb * nblk;
-    const int side = b & 1, lb = (b >> 1) / nw, w = (b >> 1) - lb * nw;
+    const int side = b & 1, lb = (int)((unsigned)(b >> 1) * a.rb >> 16), w = (b >> 1) - lb * nw;
     unsigned *X = img + hb * 2 * ximg, *Y = X + ximg;
     const int line = lb * 32 + 1 + lane;
     unsigned x = line <= roi ? X[line * ls + 2 * w + side] : 0u;
@@ -601,7 +601,7 @@ __global__ void __cluster_dims__(2) __launch_bounds__(kQuadMaxThreads, 2)
     __syncthreads();
     // A into B, as X into Y above
     for (int b = warp; b < nw * nw; b += nwarps) {
-      const int lb = b / nw, w = b - lb * nw, line = lb * 32 + 1 + lane;
+      const int lb = (int)((unsigned)b * a.rb >> 16), w = b - lb * nw, line = lb * 32 + 1 + lane;
       unsigned x = line <= roi ? img[line * ls + 2 * w] : 0u;
       if (!__any_sync(0xffffffffu, x != 0u)) continue;
       x = warp_transpose(x, lane);
@@ -730,7 +730,8 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
   if (4 * (nr * (2 * w64 | 1) + 32 * w32 * (w32 | 1) + roi + 1) + 16 > 227 * 1024)
     return cudaErrorInvalidValue;
   ShedArgs a{dem.data, dem.pitch, dem.nrows, roi, oht, tht, obs, sheds, d_err, 2 * nsheds, 1,
-             ~0ull / (unsigned)dem.nrows + 1ull, 65536u / (unsigned)w64 + 1u};
+             ~0ull / (unsigned)dem.nrows + 1ull, 65536u / (unsigned)w64 + 1u,
+             65536u / (unsigned)pair_words(roi) + 1u};
   // the reciprocal-table division is exhaustively checked for |a| <= 2^21
   // (heights up to 10^6 over 16-bit elevations) and steps up to 2048
   const bool rcp = oht >= 0 && oht <= 1000000;
