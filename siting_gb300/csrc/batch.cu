@@ -27,10 +27,15 @@ namespace {
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// CTAs of a job's SITE group in a batch: the fewest that keep each CTA's
-// candidates within the kernel's per-CTA capacity, so many jobs share the SMs.
+// CTAs of a job's SITE group in a batch: one for 2048 candidates, so many jobs share
+// the SMs and a launch still starts before the last jobs' stages (with one for 4096, the
+// fewest that the kernel takes, nearly all jobs fell into the first launch, which
+// nothing was left to overlap; ms at 4096, 2048 and 1024: 16 jobs of 512^2 to 2048^2
+// 48.8, 46.0, 45.4; 20 of 500^2 to 2000^2, dense 51.4, 47.7, 50.2; 24 of 512^2 to 2048^2
+// 43.7, 37.3, 37.3; 24 of 300^2 to 900^2 11.0, 11.0, 10.2; 12 of 256^2 to 2200^2 23.5,
+// 21.3, 22.5).
 int batch_site_ctas(int nsheds, int sm_count) {
-  const int g = std::max(1, (nsheds + 4095) / 4096);
+  const int g = std::max(1, (nsheds + 2047) / 2048);
   return std::min(std::min(g, std::max(1, nsheds)), sm_count);
 }
 
