@@ -310,20 +310,20 @@ def stage_bytes(w, nwanted, site_bytes):
 
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from
-# ncu: VIX, VIEWSHED (shed_half_kernel) and SITE captured at full size.
+# ncu: VIX, VIEWSHED (shed_kernel<1>) and SITE captured at full size.
 NCU_TRAFFIC = {
-    "c2_4096": {"vix": 33720064 + 1536, "viewshed": 33861632 + 361607680,
-                "site": 2494835712 + 10062080},
+    "c2_4096": {"vix": 33597184 + 428288, "viewshed": 33922560 + 358754816,
+                "site": 2581495040 + 41751552},
 }
 
 # Warp instructions per unit of work of the two issue-bound stages, from ncu
 # (smsp__inst_executed.sum of one launch / its units) on the 2048^2 captures
 # with roi 100 and 100 targets: per target for VIX (vix_kernel), per observer
-# for VIEWSHED (shed_half_kernel, both halves).  Keyed by the parameters they
+# for VIEWSHED (shed_kernel<1>, both halves).  Keyed by the parameters they
 # were measured with.
 ISSUE_WORK = {
-    ("vix", 100, 100): (2.058e9 / (2048 * 2048 * 100), "target"),
-    ("viewshed", 100, 100): (1.398323148e9 / 16384, "observer"),
+    ("vix", 100, 100): (1.739e9 / (2048 * 2048 * 100), "target"),
+    ("viewshed", 100, 100): (8.885e8 / 16384, "observer"),
 }
 ISSUE_SLOTS_PER_SM = 4  # one warp instruction per cycle from each SM sub-partition
 
@@ -331,7 +331,7 @@ ROOFLINE_NOTES = {
     "vix": "VIX is bound by SM instruction issue, not HBM: its compulsory traffic is 3 B/cell; "
            "achieved = warp instructions per target (ncu) x targets / stage time, peak = SMs x "
            "4 issue slots x the median SM clock of the timed region",
-    "viewshed": "VIEWSHED is bound by SM instruction issue (one dependent chain per ray); "
+    "viewshed": "VIEWSHED is bound by SM instruction issue and the shared-memory pipe; "
                 "achieved = warp instructions per observer (ncu) x observers / stage time",
     "site": "SITE's algorithmic bytes are the reference's rescoring traffic (every rescored "
             "candidate's shed and coverage window per pick); this kernel updates gains by "

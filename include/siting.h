@@ -187,16 +187,22 @@ int siting_last_pick_order(siting_ctx *ctx, int32_t *order, int cap, int *count)
  * candidates near the picks (and, in large rounds, this CTA's rows of the
  * picks' new bits), 11 the barrier after those rows (large rounds), 5
  * compacting the pairs, 6 gain deltas, 12 intervis cut, 7 second barrier and
- * the smallest cut, 8 applying the picks.  Writes min(n, 13) values. */
+ * the smallest cut, 8 applying the picks.  A selection by local dominance
+ * (all without intervis, large sparse ones with it): 0 sorting into bins, 1
+ * each bin's first candidate, 3 the dominant ones, 10 the search for
+ * candidates they would uncover (intervis), 5 the picks' new bits, 7 coverage
+ * and gains, 2, 4, 11, 6 and 8 the barriers after these, 9 the picks' order at
+ * the end.  Writes min(n, 13) values. */
 int siting_last_site_phase_cycles(siting_ctx *ctx, long long *cycles, int n);
 
 /* SITE on device buffers without allocating any memory.  No counterpart in
  * the reference: it is for callers that cannot allocate device memory on
  * their call path (a serving loop that reserves its HBM budget at start-up,
  * or an application whose memory pool already owns the device's memory).
- * Scratch comes from a 16 MiB array in the library's device image, held by
+ * Scratch comes from a 48 MiB array in the library's device image, held by
  * every GPU that loads the library until the process exits; a job whose
- * scratch would exceed it returns SITING_ENOMEM, and invalid arguments return
+ * coverage bitmap, new-bit rows and pick lists (as of a selection in the global
+ * key order) take more than 16 MiB returns SITING_ENOMEM, and invalid arguments return
  * SITING_EINVAL (an observer index outside the DEM is found before SITE
  * reads through it).  Runs on `stream` (a cudaStream_t, NULL = default
  * stream) of the current device, synchronises that stream twice and returns

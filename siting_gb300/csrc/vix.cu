@@ -17,7 +17,7 @@
 // become VIX bytes through a host-computed table.
 //
 // Bound by instruction issue (92-95% of the slots at roi 100).  2048^2, roi
-// 100, 100 targets: 157 -> 139 thread instructions a target and 1.894 -> 1.473
+// 100, 100 targets: 157 -> 133 thread instructions a target and 1.894 -> 1.473
 // ms (285 G targets/s) with offsets as magnitudes whose signs go with the
 // strides (one rounding addend, no sign handling a sample), the samples unrolled
 // with one FMA for each scaled sum, the draws doubled modulo 2^32, and 32x32
