@@ -120,7 +120,7 @@ struct SiteScratch {
   uint64_t *nbits;           // the round's new bits of each pick: [64][nr][nwpr+1] words
   unsigned char *nmask;      // [64][nr]: bit j set when word j of that new-bit row is nonzero
   unsigned long long *topk;  // [2][nctas][top-K] x {key, cell}: published top keys
-  int *cuts;                 // [2][nctas]: per-CTA prefix cut (intervis)
+  int *cuts;                 // [2] of [2][nctas]: the smallest cut of the round's prefix (intervis)
   int *ncount;               // [2][64]: popcount of each pick's new bits (self-check)
   unsigned *bar;             // group barrier counter, zeroed
   long long *out;            // [0] nused, [1] cumarea, [2] rounds, [3..15] phase cycles

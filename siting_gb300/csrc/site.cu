@@ -79,7 +79,7 @@ struct SiteArgs {
   unsigned char *nmask;  // [kMaxPicks][nr]: bit j set when word j of that row is nonzero
   int ncap_words;   // shared-memory words for a small round's new bits
   unsigned long long *topk;  // [2][G][kTopK] x {key, cell}
-  int *cuts;                 // [2][G]: per-CTA cut of the round's prefix (intervis)
+  int *cuts;                 // [2]: the smallest cut of the round's prefix, as kMaxPicks+1-cut (0: none)
   int *ncount;               // [2][kMaxPicks]: popcount of each pick's new bits
   unsigned *bar;
   long long *out;
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     site_local(a, *reinterpret_cast<LocalShared *>(sm), (int)blockIdx.x - a.block0, s_ph, &s_tmark);
     return;
   }
-  __shared__ int s_m, s_mcut, s_stop_at, s_done, s_flagv, s_roundcut, s_npair, s_nvalid;
+  __shared__ int s_m, s_stop_at, s_done, s_flagv, s_roundcut, s_npair, s_nvalid;
   __shared__ long long s_cum;
   __shared__ int s_poff[kMaxPicks + 1];
   // reciprocals (div_recip) of the kernel's divisors and of each pick's run
@@ -310,7 +310,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 0) {
       unsigned long long *out = a.topk + ((size_t)par * G + k) * kTopK * 2;
       int h0 = 0, h1 = 0, h2 = 0, h3 = 0;  // heads of groups lane, lane+32, lane+64, lane+96
-      for (int e = 0; e < kTopK; e++) {
+      unsigned long long pub = 0;  // lane e: the e-th key
+      if (ngroups == 1 && lane < kTopK) pub = s_gtop[lane];
+      for (int e = 0; e < (ngroups == 1 ? 0 : kTopK); e++) {
         unsigned long long key = 0;
         int gi = -1;
 #pragma unroll
@@ -335,11 +337,12 @@ __global__ void __launch_bounds__(kThreads, 1)
           h2 += q == 2;
           h3 += q == 3;
         }
-        if (lane == 0) {
-          const int pos = key ? s_pos[key_index(key) / G] : 0;
-          __stcg(out + 2 * e, key);
-          __stcg(out + 2 * e + 1, (unsigned long long)pos);
-        }
+        if (lane == e) pub = key;
+      }
+      if (lane < kTopK) {
+        const int pos = pub ? s_pos[div_by(key_index(pub), s_rG)] : 0;
+        __stcg(out + 2 * lane, pub);
+        __stcg(out + 2 * lane + 1, (unsigned long long)pos);
       }
     }
     mark(1);
@@ -917,20 +920,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (cut < m) atomicMin(&s_roundcut, cut);
     }
     __syncthreads();
-    if (tid == 0) __stcg(a.cuts + par * G + k, s_roundcut);
+    if (tid == 0) {
+      if (s_roundcut < m) atomicMax(a.cuts + par, kMaxPicks + 1 - s_roundcut);
+      if (k == 0) __stcg(a.cuts + (par ^ 1), 0);  // read by all before this round's first barrier
+    }
     mark(12);
     // every read of the coverage this round is done once all CTAs pass here
     if (!group_sync(gb, a.err, &s_flagv)) return;
-    if (tid == 0) s_mcut = m;
-    __syncthreads();
-    {  // the smallest cut of any CTA: one load per thread
-      int c = tid < G ? __ldcg(a.cuts + par * G + tid) : m;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) c = min(c, __shfl_xor_sync(0xffffffffu, c, o));
-      if (lane == 0 && c < m) atomicMin(&s_mcut, c);
-    }
-    __syncthreads();
-    const int mcut = s_mcut;
+    const int latest = __ldcg(a.cuts + par);  // of the smallest cut of any CTA
+    const int mcut = latest ? kMaxPicks + 1 - latest : m;
     mark(7);
 
     // ---- F. apply picks 0..mcut-1 -------------------------------------------
