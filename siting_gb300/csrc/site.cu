@@ -63,6 +63,7 @@ constexpr int kMaxSlots = 4096;  // candidates owned by one CTA
 // intervis cuts long before the threshold of K keys binds (4096^2: 343
 // rounds with 3, 4, 6 or 8), and fewer keys make each merge cheaper.
 constexpr int kTopK = 3;
+constexpr int kFewKeys = 256;     // published keys that one warp orders
 constexpr int kMaxPicks = 64;    // picks accepted in one round at most
 constexpr int kSmallRecip = 128; // reciprocals tabled in shared memory (>= kMaxPicks)
 constexpr int kMaxPairs = 8192;  // (candidate, pick) pairs one CTA updates per round
@@ -169,6 +170,88 @@ __global__ void __launch_bounds__(256) site_score_kernel(const uint64_t *sheds, 
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0) gains[c] = cnt;
   }
+}
+
+// B for few published keys, by one warp: it takes the largest again and again, a
+// handful a round, where the general form below ranks all of them (SITE ms ranked and so:
+// 256^2, 1024 candidates 0.74, 0.72; 370^2, 1152 0.66, 0.63; 743^2, 8649 0.69, 0.66;
+// 1741^2, 23 762 3.33, 3.16).  A function of its own: inside the round's loop its code
+// costs the larger jobs 2-4%.  Returns the number of picks and, from bit 8 on, that at
+// the 95% stop plus one.
+__device__ __noinline__ int few_picks(const SiteArgs &a, int par, int max_m, long long cumv,
+                                      int *s_pk, int *s_ppos, unsigned long long *s_pkey,
+                                      int4 *s_pbox, unsigned long long *s_rrun) {
+  const int lane = threadIdx.x & 31, GK = a.G * kTopK, roi = a.roi, lim2 = 4 * roi * roi;
+  unsigned long long key[kFewKeys / 32], T = 0;
+  int pos[kFewKeys / 32];
+#pragma unroll
+  for (int q = 0; q < kFewKeys / 32; q++) {
+    const int e = lane + 32 * q;
+    const unsigned long long *src = a.topk + ((size_t)par * GK + e) * 2;
+    key[q] = e < GK ? __ldcg(src) : 0ull;
+    pos[q] = e < GK ? (int)__ldcg(src + 1) : 0;
+    if (e % kTopK == kTopK - 1 && key[q] > T) T = key[q];
+  }
+  T = warp_max_key(T);  // exactness threshold: unpublished keys are below it
+#pragma unroll
+  for (int q = 0; q < kFewKeys / 32; q++)
+    if ((key[q] >> 32) == 0 || key[q] < T) key[q] = 0;
+  unsigned long long k0 = 0, k1 = 0;  // lane l holds picks l and l+32
+  int q0 = 0, q1 = 0, m = 0, stop_at = -1;
+  while (m < max_m) {
+    unsigned long long best = key[0];
+    int bpos = pos[0];
+#pragma unroll
+    for (int q = 1; q < kFewKeys / 32; q++)
+      if (key[q] > best) {
+        best = key[q];
+        bpos = pos[q];
+      }
+    const unsigned long long mx = warp_max_key(best);
+    if (mx == 0) break;
+    const int p1 = __shfl_sync(0xffffffffu, bpos, __ffs(__ballot_sync(0xffffffffu, best == mx)) - 1);
+    const int x1 = p1 >> 16, y1 = p1 & 0xffff;
+    const int dx0 = (q0 >> 16) - x1, dy0 = (q0 & 0xffff) - y1;
+    const int dx1 = (q1 >> 16) - x1, dy1 = (q1 & 0xffff) - y1;
+    const bool near = (lane < m && dx0 * dx0 + dy0 * dy0 <= lim2) ||
+                      (lane + 32 < m && dx1 * dx1 + dy1 * dy1 <= lim2);
+    if (__any_sync(0xffffffffu, near)) break;
+    if (lane == m) {
+      k0 = mx;
+      q0 = p1;
+    } else if (lane + 32 == m) {
+      k1 = mx;
+      q1 = p1;
+    }
+#pragma unroll
+    for (int q = 0; q < kFewKeys / 32; q++)
+      if (key[q] == mx) key[q] = 0;
+    m++;
+    cumv += (long long)(mx >> 32);
+    if (cumv >= a.stop_area) {
+      stop_at = m;
+      break;
+    }
+  }
+  const int nr = 2 * roi + 1, per = nr * ((nr + 63) / 64);
+  for (int j = lane; j < m; j += 32) {
+    const unsigned long long k = j < 32 ? k0 : k1;
+    const int ps = j < 32 ? q0 : q1, c = key_index(k), px = ps >> 16, py = ps & 0xffff;
+    s_pk[j] = c;
+    s_ppos[j] = ps;
+    s_pkey[j] = k;
+    prefetch_l2(a.sheds + (size_t)c * per, (size_t)per * 8);  // the pick's shed, for D1
+    // the block rectangle of the neighbour search (FINDMAX geometry, +-2 blocks)
+    const float r2f = (float)(2 * roi);
+    const int bxl = max(0, (int)floorf(((float)px - r2f) / a.bs) - 2);
+    const int bxh = min(a.nb - 1, (int)floorf(((float)px + r2f) / a.bs) + 2);
+    const int byl = max(0, (int)floorf(((float)py - r2f) / a.bs) - 2);
+    const int byh = min(a.nb - 1, (int)floorf(((float)py + r2f) / a.bs) + 2);
+    const int run = (byh - byl + 1) * a.npb, per_run = run / a.G + 2;
+    s_pbox[j] = make_int4((bxl * a.nb + byl) * a.npb, run, per_run, (bxh - bxl + 1) * per_run);
+    s_rrun[j] = div_recip(per_run);
+  }
+  return m | (stop_at + 1) << 8;
 }
 
 // One launch runs the greedy selection of one or more jobs (DEMs): CTA b
@@ -349,124 +432,138 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (!group_sync(gb, a.err, &s_flagv)) return;
     mark(2);
     // ---- B. merge the published lists; accept the exact prefix --------------
+    if (GK <= kFewKeys) {
+      if (warp == 0) {
+        const int got = few_picks(a, par, min(kMaxPicks, a.pair_cap / max(pcap, 1)), s_cum, s_pk,
+                                  s_ppos, s_pkey, s_pbox, s_rrun);
+        if (lane == 0) {
+          s_m = got & 255;
+          s_stop_at = (got >> 8) - 1;
+          s_rm = s_rsmall[max(got & 255, 1)];
+        }
+      } else if (tid >= 32 && tid < 32 + kMaxPicks) {
+        s_pcnt[tid - 32] = 0;
+      }
+    } else {
 #pragma unroll 2
-    for (int i = tid; i < GK; i += blockDim.x) {
-      const unsigned long long *src = a.topk + ((size_t)par * GK + i) * 2;
-      s_mkey[i] = __ldcg(src);
-      s_mpos[i] = (int)__ldcg(src + 1);
-    }
-    if (tid < kMaxPicks) s_pcnt[tid] = 0;
-    if (tid == 0) s_nvalid = 0;
-    __syncthreads();
-    {  // exactness threshold: unpublished keys are below each full list's last key
-      unsigned long long T = 0;
-      if (tid < G) T = s_mkey[tid * kTopK + kTopK - 1];
-      T = warp_max_key(T);
-      if (lane == 0 && warp * 32 < G) s_red[warp] = T;
-    }
-    __syncthreads();
-    {
-      unsigned long long T = 0;
-      for (int w = 0; w * 32 < G; w++) T = s_red[w] > T ? s_red[w] : T;
-      // exactly ordered entries: keys >= T with a positive area
-      auto valid_key = [&](unsigned long long key) {
-        return key != 0 && (key >> 32) != 0 && key >= T;
-      };
-      for (int e0 = warp * 32; e0 < GK; e0 += blockDim.x) {  // one shared atomic a warp
-        const int e = e0 + lane;
-        const unsigned long long key = e < GK ? s_mkey[e] : 0ull;
-        const bool ok = key != 0 && (key >> 32) != 0 && key >= T;
-        const unsigned bal = __ballot_sync(0xffffffffu, ok);
-        if (!bal) continue;
-        int v0 = 0;
-        if (lane == 0) v0 = atomicAdd(&s_nvalid, __popc(bal));
-        v0 = __shfl_sync(0xffffffffu, v0, 0);
-        if (ok) {
-          const int v = v0 + __popc(bal & ((1u << lane) - 1u));
-          s_valid[v] = e;  // GK entries fit
-          s_vkey[v] = key;
-          s_vrank[v] = 0;
+      for (int i = tid; i < GK; i += blockDim.x) {
+        const unsigned long long *src = a.topk + ((size_t)par * GK + i) * 2;
+        s_mkey[i] = __ldcg(src);
+        s_mpos[i] = (int)__ldcg(src + 1);
+      }
+      if (tid < kMaxPicks) s_pcnt[tid] = 0;
+      if (tid == 0) s_nvalid = 0;
+      __syncthreads();
+      {  // exactness threshold: unpublished keys are below each full list's last key
+        unsigned long long T = 0;
+        if (tid < G) T = s_mkey[tid * kTopK + kTopK - 1];
+        T = warp_max_key(T);
+        if (lane == 0 && warp * 32 < G) s_red[warp] = T;
+      }
+      __syncthreads();
+      {
+        unsigned long long T = 0;
+        for (int w = 0; w * 32 < G; w++) T = s_red[w] > T ? s_red[w] : T;
+        // exactly ordered entries: keys >= T with a positive area
+        auto valid_key = [&](unsigned long long key) {
+          return key != 0 && (key >> 32) != 0 && key >= T;
+        };
+        for (int e0 = warp * 32; e0 < GK; e0 += blockDim.x) {  // one shared atomic a warp
+          const int e = e0 + lane;
+          const unsigned long long key = e < GK ? s_mkey[e] : 0ull;
+          const bool ok = key != 0 && (key >> 32) != 0 && key >= T;
+          const unsigned bal = __ballot_sync(0xffffffffu, ok);
+          if (!bal) continue;
+          int v0 = 0;
+          if (lane == 0) v0 = atomicAdd(&s_nvalid, __popc(bal));
+          v0 = __shfl_sync(0xffffffffu, v0, 0);
+          if (ok) {
+            const int v = v0 + __popc(bal & ((1u << lane) - 1u));
+            s_valid[v] = e;  // GK entries fit
+            s_vkey[v] = key;
+            s_vrank[v] = 0;
+          }
         }
       }
-    }
-    __syncthreads();
-    mark(9);
-    const int nvalid = s_nvalid;
-    {  // rank of each valid key: count larger valid keys, 32 at a time
-      // lanes take consecutive keys against one chunk: the chunk's reads are
-      // broadcasts, free of bank conflicts
-      const int nch = (nvalid + 31) / 32;
-      for (int i = tid; i < nvalid * nch; i += blockDim.x) {
-        const int ch = i / nvalid, v = i - ch * nvalid, c0 = ch * 32;
-        const unsigned long long key = s_vkey[v];
-        const int c1 = min(c0 + 32, nvalid);
-        int cnt = 0;
+      __syncthreads();
+      mark(9);
+      const int nvalid = s_nvalid;
+      {  // rank of each valid key: count larger valid keys, 32 at a time
+        // lanes take consecutive keys against one chunk: the chunk's reads are
+        // broadcasts, free of bank conflicts
+        const int nch = (nvalid + 31) / 32;
+        for (int i = tid; i < nvalid * nch; i += blockDim.x) {
+          const int ch = i / nvalid, v = i - ch * nvalid, c0 = ch * 32;
+          const unsigned long long key = s_vkey[v];
+          const int c1 = min(c0 + 32, nvalid);
+          int cnt = 0;
 #pragma unroll 8
-        for (int j = c0; j < c1; j++) cnt += s_vkey[j] > key;
-        if (cnt) atomicAdd(&s_vrank[v], cnt);
-      }
-    }
-    __syncthreads();
-    for (int v = tid; v < nvalid; v += blockDim.x)
-      if (s_vrank[v] < kMaxPicks) {
-        s_rank[s_vrank[v]] = s_valid[v];
-        s_rpos[s_vrank[v]] = s_mpos[s_valid[v]];
-      }
-    __syncthreads();
-    mark(10);
-    const int nrank = min(nvalid, kMaxPicks);
-    if (warp == 0) {
-      // prefix: leading ranks that are each > 2roi from every better-ranked
-      // one, capped, up to the 95% stop.  Lane l holds ranks l and l+32.
-      const int max_m = min(kMaxPicks, a.pair_cap / max(pcap, 1));
-      const int lim = min(nrank, max_m);
-      const int q0 = lane < lim ? s_rpos[lane] : 0;
-      const int q1 = lane + 32 < lim ? s_rpos[lane + 32] : 0;
-      const int a0 = lane < lim ? (int)(s_mkey[s_rank[lane]] >> 32) : 0;
-      const int a1 = lane + 32 < lim ? (int)(s_mkey[s_rank[lane + 32]] >> 32) : 0;
-      long long cumv = s_cum;
-      int m = 0, stop_at = -1;
-      for (int r = 0; r < lim; r++) {
-        const int p1 = __shfl_sync(0xffffffffu, r < 32 ? q0 : q1, r & 31);
-        const int area = __shfl_sync(0xffffffffu, r < 32 ? a0 : a1, r & 31);
-        const int x1 = p1 >> 16, y1 = p1 & 0xffff;
-        const int dx0 = (q0 >> 16) - x1, dy0 = (q0 & 0xffff) - y1;
-        const int dx1 = (q1 >> 16) - x1, dy1 = (q1 & 0xffff) - y1;
-        const bool near = (lane < r && dx0 * dx0 + dy0 * dy0 <= lim2) ||
-                          (lane + 32 < r && dx1 * dx1 + dy1 * dy1 <= lim2);
-        if (__any_sync(0xffffffffu, near)) break;
-        cumv += area;
-        m = r + 1;
-        if (cumv >= a.stop_area) {
-          stop_at = m;
-          break;
+          for (int j = c0; j < c1; j++) cnt += s_vkey[j] > key;
+          if (cnt) atomicAdd(&s_vrank[v], cnt);
         }
       }
-      for (int j = lane; j < m; j += 32) {
-        const int e = s_rank[j];
-        const int c = key_index(s_mkey[e]);
-        s_pk[j] = c;
-        s_ppos[j] = s_mpos[e];
-        s_pkey[j] = s_mkey[e];
-        prefetch_l2(a.sheds + (size_t)c * per, per * 8);  // the pick's shed, for D1
-        {  // the block rectangle of the neighbour search (FINDMAX geometry, +-2 blocks)
-          const float r2f = (float)(2 * roi);
-          const int pos = s_mpos[e];
-          const int px = pos >> 16, py = pos & 0xffff;
-          const int bxl = max(0, (int)floorf(((float)px - r2f) / a.bs) - 2);
-          const int bxh = min(a.nb - 1, (int)floorf(((float)px + r2f) / a.bs) + 2);
-          const int byl = max(0, (int)floorf(((float)py - r2f) / a.bs) - 2);
-          const int byh = min(a.nb - 1, (int)floorf(((float)py + r2f) / a.bs) + 2);
-          const int run = (byh - byl + 1) * a.npb;
-          const int per_run = run / G + 2;
-          s_pbox[j] = make_int4((bxl * a.nb + byl) * a.npb, run, per_run, (bxh - bxl + 1) * per_run);
-          s_rrun[j] = per_run <= kSmallRecip ? s_rsmall[per_run] : div_recip(per_run);
+      __syncthreads();
+      for (int v = tid; v < nvalid; v += blockDim.x)
+        if (s_vrank[v] < kMaxPicks) {
+          s_rank[s_vrank[v]] = s_valid[v];
+          s_rpos[s_vrank[v]] = s_mpos[s_valid[v]];
         }
-      }
-      if (lane == 0) {
-        s_m = m;
-        s_stop_at = stop_at;
-        s_rm = s_rsmall[max(m, 1)];  // m <= kMaxPicks <= kSmallRecip
+      __syncthreads();
+      mark(10);
+      const int nrank = min(nvalid, kMaxPicks);
+      if (warp == 0) {
+        // prefix: leading ranks that are each > 2roi from every better-ranked
+        // one, capped, up to the 95% stop.  Lane l holds ranks l and l+32.
+        const int max_m = min(kMaxPicks, a.pair_cap / max(pcap, 1));
+        const int lim = min(nrank, max_m);
+        const int q0 = lane < lim ? s_rpos[lane] : 0;
+        const int q1 = lane + 32 < lim ? s_rpos[lane + 32] : 0;
+        const int a0 = lane < lim ? (int)(s_mkey[s_rank[lane]] >> 32) : 0;
+        const int a1 = lane + 32 < lim ? (int)(s_mkey[s_rank[lane + 32]] >> 32) : 0;
+        long long cumv = s_cum;
+        int m = 0, stop_at = -1;
+        for (int r = 0; r < lim; r++) {
+          const int p1 = __shfl_sync(0xffffffffu, r < 32 ? q0 : q1, r & 31);
+          const int area = __shfl_sync(0xffffffffu, r < 32 ? a0 : a1, r & 31);
+          const int x1 = p1 >> 16, y1 = p1 & 0xffff;
+          const int dx0 = (q0 >> 16) - x1, dy0 = (q0 & 0xffff) - y1;
+          const int dx1 = (q1 >> 16) - x1, dy1 = (q1 & 0xffff) - y1;
+          const bool near = (lane < r && dx0 * dx0 + dy0 * dy0 <= lim2) ||
+                            (lane + 32 < r && dx1 * dx1 + dy1 * dy1 <= lim2);
+          if (__any_sync(0xffffffffu, near)) break;
+          cumv += area;
+          m = r + 1;
+          if (cumv >= a.stop_area) {
+            stop_at = m;
+            break;
+          }
+        }
+        for (int j = lane; j < m; j += 32) {
+          const int e = s_rank[j];
+          const int c = key_index(s_mkey[e]);
+          s_pk[j] = c;
+          s_ppos[j] = s_mpos[e];
+          s_pkey[j] = s_mkey[e];
+          prefetch_l2(a.sheds + (size_t)c * per, per * 8);  // the pick's shed, for D1
+          {  // the block rectangle of the neighbour search (FINDMAX geometry, +-2 blocks)
+            const float r2f = (float)(2 * roi);
+            const int pos = s_mpos[e];
+            const int px = pos >> 16, py = pos & 0xffff;
+            const int bxl = max(0, (int)floorf(((float)px - r2f) / a.bs) - 2);
+            const int bxh = min(a.nb - 1, (int)floorf(((float)px + r2f) / a.bs) + 2);
+            const int byl = max(0, (int)floorf(((float)py - r2f) / a.bs) - 2);
+            const int byh = min(a.nb - 1, (int)floorf(((float)py + r2f) / a.bs) + 2);
+            const int run = (byh - byl + 1) * a.npb;
+            const int per_run = run / G + 2;
+            s_pbox[j] = make_int4((bxl * a.nb + byl) * a.npb, run, per_run, (bxh - bxl + 1) * per_run);
+            s_rrun[j] = per_run <= kSmallRecip ? s_rsmall[per_run] : div_recip(per_run);
+          }
+        }
+        if (lane == 0) {
+          s_m = m;
+          s_stop_at = stop_at;
+          s_rm = s_rsmall[max(m, 1)];  // m <= kMaxPicks <= kSmallRecip
+        }
       }
     }
     __syncthreads();
