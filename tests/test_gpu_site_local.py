@@ -58,3 +58,19 @@ def test_noalloc_scratch_holds_a_local_selection(native, oracle):
         assert rc == 0
         assert np.array_equal(sel.cpu().numpy(), want)
         assert (res.nusedsheds, res.cumarea) == (used, area)
+
+
+@pytest.mark.parametrize("ctas", [1, 42, 43, 85, 86, 152])
+def test_global_order_takes_picks_by_one_warp_or_by_ranking(native, oracle, ctas):
+    # 3 published keys a CTA: up to 256 are taken by one warp, more are ranked
+    n, roi, count = 180, 9, 1500
+    dem = native.fbm_dem(n, seed=4, octaves=7, range_max=6000)
+    obs = np.random.default_rng(4).integers(0, n * n, count).astype(np.int32)
+    sheds = oracle.sheds(dem, n, roi, 15, 15, obs)
+    want, used, area, order = oracle.site(n, roi, 1, obs, sheds, want_order=True)
+    with native.Context(0) as ctx:
+        ctx.set_site_ctas(ctas)
+        sel, res = ctx.site_it(n, roi, 1, obs, sheds)
+        assert np.array_equal(ctx.last_pick_order(count), order)
+    assert np.array_equal(sel, want)
+    assert (res.nusedsheds, res.cumarea) == (used, area)
