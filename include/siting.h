@@ -118,6 +118,12 @@ int siting_ctx_trim(siting_ctx *ctx);
 /* Tuning knob: CTAs of the SITE kernel (0 = automatic, capped at the SM
  * count).  Results do not depend on it. */
 int siting_ctx_set_site_ctas(siting_ctx *ctx, int nctas);
+/* Tuning knob: how SITE of single jobs takes its picks (batches and servers choose
+ * for each job).  1 = in the global key order, the longest prefix of it without a
+ * conflict a round, 2 = by local dominance, every candidate that nothing within 2*roi
+ * can precede a round, 0 = automatic, by the number and the spread of the candidates.
+ * Results do not depend on it. */
+int siting_ctx_set_site_order(siting_ctx *ctx, int order);
 /* Tuning knob of the batched form (no counterpart in the reference): how a
  * batch launches VIX and FINDMAX.  1 = for the jobs of each SITE launch, one
  * grid over their (job, tile) VIX items (two when some halos are staged and
@@ -187,8 +193,7 @@ int siting_last_pick_order(siting_ctx *ctx, int32_t *order, int cap, int *count)
  * candidates near the picks (and, in large rounds, this CTA's rows of the
  * picks' new bits), 11 the barrier after those rows (large rounds), 5
  * compacting the pairs, 6 gain deltas, 12 intervis cut, 7 second barrier and
- * the smallest cut, 8 applying the picks.  A selection by local dominance
- * (all without intervis, large sparse ones with it): 0 sorting into bins, 1
+ * the smallest cut, 8 applying the picks.  A selection by local dominance: 0 sorting into bins, 1
  * each bin's first candidate, 3 the dominant ones, 10 the search for
  * candidates they would uncover (intervis), 5 the picks' new bits, 7 coverage
  * and gains, 2, 4, 11, 6 and 8 the barriers after these, 9 the picks' order at

@@ -157,6 +157,7 @@ def load() -> C.CDLL:
         "siting_ctx_workspace_bytes": ([_P], sz),
         "siting_ctx_trim": ([_P], i),
         "siting_ctx_set_site_ctas": ([_P, i], i),
+        "siting_ctx_set_site_order": ([_P, i], i),
         "siting_ctx_set_batch_mode": ([_P, i], i),
         "siting_ctx_set_batch_graphs": ([_P, i], i),
         "siting_ctx_batch_graph_stats": ([_P, C.POINTER(ll), C.POINTER(ll)], i),
@@ -316,6 +317,11 @@ class Context:
 
     def set_site_ctas(self, n: int):
         self._check(self._lib.siting_ctx_set_site_ctas(self.h, n))
+
+    def set_site_order(self, order: int):
+        """How SITE takes its picks: 0 automatic, 1 in the global key order, 2 by local
+        dominance."""
+        self._check(self._lib.siting_ctx_set_site_order(self.h, order))
 
     def set_batch_mode(self, mode: int):
         """How batches run VIX and FINDMAX: 0 automatic, 1 one queued launch per

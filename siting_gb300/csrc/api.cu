@@ -246,16 +246,18 @@ int site_enqueue(siting_ctx *ctx, int nrows, int roi, int intervis, int nsheds,
   if (site_smem_bytes(roi, nsheds, G, nb, npb, bs) > 220 * 1024)
     return fail(ctx, SITING_EINVAL, "SITE: shared-memory plan exceeds 220 KB");
   void *p;
-  const size_t sb = site_scratch_bytes(nrows, nsheds, G, roi, intervis, nb);
+  const bool local = ctx->site_order == kOrderAuto ? site_is_local(nrows, nsheds, roi, intervis, nb)
+                                                   : ctx->site_order == kOrderLocal;
+  const size_t sb = site_scratch_bytes(nrows, nsheds, G, roi, intervis, local);
   int rc = ws_get(ctx, kSite, sb, &p);
   if (rc) return rc;
   SiteScratch s;
-  site_carve_scratch(p, nrows, nsheds, G, roi, intervis, nb, &s);
+  site_carve_scratch(p, nrows, nsheds, G, roi, intervis, local, &s);
   // zero coverage, slots, barrier and outputs (order is written before read)
   CK(cudaMemsetAsync(p, 0, (unsigned char *)s.order - (unsigned char *)p, ctx->stream));
   CK(cudaMemsetAsync(d_selected, 0, nsheds, ctx->stream));
   CK(launch_site(nrows, roi, intervis, nsheds, d_obs, d_sheds, bs, nb, npb, d_selected, s, G,
-                 d_err, ctx->stream));
+                 d_err, local, ctx->stream));
   CK(cudaMemcpyAsync(ctx->h_out, s.out, (3 + kSitePhases) * sizeof(long long), cudaMemcpyDeviceToHost,
                      ctx->stream));
   ctx->d_last_order = s.order;
@@ -417,6 +419,12 @@ size_t siting_ctx_workspace_bytes(const siting_ctx *ctx) { return ctx ? ctx->hel
 int siting_ctx_set_site_ctas(siting_ctx *ctx, int nctas) {
   if (!ctx || nctas < 0) return SITING_EINVAL;
   ctx->site_ctas = nctas;
+  return SITING_OK;
+}
+
+int siting_ctx_set_site_order(siting_ctx *ctx, int order) {
+  if (!ctx || order < siting::kOrderAuto || order > siting::kOrderLocal) return SITING_EINVAL;
+  ctx->site_order = order;
   return SITING_OK;
 }
 

@@ -22,6 +22,7 @@ struct Job {
   ShedPlan sp;
   // workspace offsets
   size_t o_dem, o_vix, o_obs, o_sel, o_sheds, o_tab, o_site, o_err;
+  bool local;        // SITE by local dominance
   size_t site_zero;  // bytes of the SITE scratch that start at zero
 };
 

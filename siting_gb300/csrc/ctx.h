@@ -21,6 +21,9 @@ enum Slot { kDem, kVix, kObs, kSheds, kTables, kSite, kSel, kErr, kBatch, kNumSl
 // How a batch launches VIX and FINDMAX (siting_ctx_set_batch_mode).
 enum BatchMode { kBatchAuto = 0, kBatchMerged = 1, kBatchPerJob = 2 };
 
+// How SITE takes its picks (siting_ctx_set_site_order).
+enum SiteOrder { kOrderAuto = 0, kOrderGlobal = 1, kOrderLocal = 2 };
+
 // Launch plan measured fastest by siting_autotune for (roi, ntests).
 struct TunedPlan {
   int roi, ntests;
@@ -39,6 +42,7 @@ struct siting_ctx {
   cudaEvent_t ev[8] = {};
   std::string err;
   int site_ctas = 0;                  // 0 = automatic
+  int site_order = 0;                 // siting::SiteOrder
   int batch_mode = 0;                 // siting::BatchMode
   int tab_roi = -1, tab_ntests = -1;  // VIX tables currently on the device
   std::vector<unsigned char> tab_host;

@@ -144,6 +144,7 @@ struct SiteJob {
   SiteScratch scratch;  // zeroed as site_dev does before the launch
   int nctas;
   int *err;
+  bool local;  // by local dominance (as its scratch was laid out)
 };
 // Device bytes of a job table for `njobs` jobs and `total_ctas` CTAs.
 size_t site_job_table_bytes(int njobs, int total_ctas);
@@ -154,9 +155,11 @@ size_t site_job_table_bytes(int njobs, int total_ctas);
 // kept unchanged until the copy has run; NULL stages through pageable memory.
 cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void *h_stage,
                              cudaStream_t st);
-size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis, int nblocks);
+// Whether a job is faster by local dominance than in the global key order.
+bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks);
+size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis, bool local);
 void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,
-                        int nblocks, SiteScratch *s);
+                        bool local, SiteScratch *s);
 int site_default_ctas(int nsheds, int sm_count);
 // The CTA count near G0 that spreads a pick's neighbourhood most evenly over
 // the CTAs for the job's block geometry (nb blocks a row, npb candidates each).
@@ -167,7 +170,7 @@ size_t site_smem_bytes(int roi, int nsheds, int nctas, int nblocks, int npb, flo
 bool site_supported(int roi, int nsheds, int nctas);
 cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int32_t *obs,
                         const uint64_t *sheds, float blocksize, int nblocks, int npb,
-                        uint8_t *selected, const SiteScratch &s, int nctas, int *d_err,
+                        uint8_t *selected, const SiteScratch &s, int nctas, int *d_err, bool local,
                         cudaStream_t st);
 
 }  // namespace siting

@@ -279,7 +279,7 @@ int siting_server::launch_stages(long long id, Request &r) {
   for (int x = 0; x < J.n; x++)
     std::memcpy(hdem + (size_t)x * J.n, r.elevs + (size_t)x * sp, (size_t)J.n * 2);
   SiteScratch s;
-  site_carve_scratch(base + J.o_site, J.n, J.g.nwanted, J.G, J.p.roi, J.p.intervis, J.g.nblocks, &s);
+  site_carve_scratch(base + J.o_site, J.n, J.g.nwanted, J.G, J.p.roi, J.p.intervis, J.local, &s);
   const size_t site_zero = (unsigned char *)s.order - (base + J.o_site);
   int *err = reinterpret_cast<int *>(base + J.o_err);
   CK(cudaMemsetAsync(base + J.o_site, 0, site_zero, s1));
@@ -312,7 +312,7 @@ int siting_server::launch_site(long long id, Request &r) {
   unsigned char *base = d_arena + r.d_off;
   unsigned char *pin = h_arena + r.h_off;
   SiteScratch s;
-  site_carve_scratch(base + J.o_site, J.n, J.g.nwanted, J.G, J.p.roi, J.p.intervis, J.g.nblocks, &s);
+  site_carve_scratch(base + J.o_site, J.n, J.g.nwanted, J.G, J.p.roi, J.p.intervis, J.local, &s);
   int *err = reinterpret_cast<int *>(base + J.o_err);
   int32_t *d_obs = reinterpret_cast<int32_t *>(base + J.o_obs);
   uint8_t *d_sel = reinterpret_cast<uint8_t *>(base + J.o_sel);
@@ -320,7 +320,7 @@ int siting_server::launch_site(long long id, Request &r) {
   CK(cudaStreamWaitEvent(site, r.staged, 0));
   CK(cudaMemsetAsync(d_sel, 0, J.g.nwanted, site));
   SiteJob sj{J.n, J.p.roi, J.p.intervis, J.g.nwanted, d_obs, d_sheds, J.g.blocksize,
-             J.g.nblocks, J.g.nwantedperblock, d_sel, s, J.G, err};
+             J.g.nblocks, J.g.nwantedperblock, d_sel, s, J.G, err, J.local};
   CK(launch_site_jobs(&sj, 1, base + bp.o_wtabs + bp.o_wtab[0], pin + L.wtab, site));
   long long *hout = reinterpret_cast<long long *>(pin + L.out);
   CK(cudaMemcpyAsync(hout, s.out, 3 * sizeof(long long), cudaMemcpyDeviceToHost, site));

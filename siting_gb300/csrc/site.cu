@@ -13,8 +13,8 @@
 //
 // GB300 mapping: one persistent kernel of G co-resident CTAs (one per SM)
 // with a bounded group barrier.  A job is selected by local dominance
-// (site_local.cuh) or, with intervis and few candidates or dense ones
-// (site_is_local), in the global order below.  Candidate c is owned by CTA c % G, which
+// (site_local.cuh) or, where candidates are few or dense (site_is_local), in the
+// global order below.  Candidate c is owned by CTA c % G, which
 // keeps its true gain, area, cell and flags in shared memory and a top-K key
 // list per 32 slots (key = area << 32 | ~c, K = kTopK).  A round:
 //   A. every CTA publishes its own top-K keys; one barrier;
@@ -30,7 +30,7 @@
 //      bits are disjoint.  Small rounds compute N in every CTA's shared
 //      memory; larger ones spread its rows over the CTAs (a global buffer
 //      read after one more barrier);
-//   E. a candidate of area 0 whose cell a pick covers can
+//   E. with intervis, a candidate of area 0 whose cell a pick covers can
 //      become eligible: each CTA finds the first prefix position it would
 //      overtake, and a second barrier takes the minimum (the round's cut);
 //   F. the picks before the cut are applied: gains fall by the summed
@@ -668,9 +668,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           s_pairslot[pr] = s;
           s_pairdelta[pr] = 0;
-          // own cell already covered?
-          s_paircov[pr] = (unsigned char)(
-              ((__ldcg(cum + (size_t)cx * cw + (cy >> 6)) >> (63 - (cy & 63))) & 1ull) << 1);
+          unsigned char cv = 0;
+          if (a.intervis)  // own cell already covered?
+            cv = (unsigned char)(((__ldcg(cum + (size_t)cx * cw + (cy >> 6)) >> (63 - (cy & 63))) & 1ull)
+                                 << 1);
+          s_paircov[pr] = cv;
         } else {
           atomicOr(a.err, kErrCapacity);
         }
@@ -759,7 +761,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(cy - roi, fwc, fbc);
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = s_N + (size_t)(pi * nr + prow) * nb2;
-        if (r == roi) {  // own cell: newly covered by the pick?
+        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((nrow[j] >> (63 - (cy & 63))) & 1ull))
             atomicOr(reinterpret_cast<unsigned *>(s_paircov + (pr & ~3)), 1u << (8 * (pr & 3)));
@@ -832,7 +834,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
         const unsigned rowm = masked ? s_nmask[pi * nr + prow] : 0xffu;
-        if (r == roi) {  // own cell: newly covered by the pick?
+        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((rowm >> j) & 1u) &&
               ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
@@ -888,7 +890,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
         const unsigned rowm = masked ? s_nmask[pi * nr + prow] : 0xffu;
-        if (r == roi) {  // own cell: newly covered by the pick?
+        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((rowm >> j) & 1u) &&
               ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
@@ -933,7 +935,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(cy - roi, fwc, fbc);
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
-        if (r == roi && ch == 0) {  // own cell: newly covered by the pick?
+        if (a.intervis && r == roi && ch == 0) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
             atomicOr(reinterpret_cast<unsigned *>(s_paircov + (pr & ~3)), 1u << (8 * (pr & 3)));
@@ -964,10 +966,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     mark(6);
 
-    // ---- E. where would a newly covered candidate overtake? --------
+    // ---- E. intervis: where would a newly covered candidate overtake? --------
     if (tid == 0) s_roundcut = m;
     __syncthreads();
-    for (int u = tid; u < npair; u += blockDim.x) {
+    for (int u = a.intervis ? tid : npair; u < npair; u += blockDim.x) {
       const int i = s_plist[u];
       const int j = div_by(i, s_rpcap);
       const int s = s_pairslot[i];
@@ -1017,14 +1019,18 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (cut < m) atomicMin(&s_roundcut, cut);
     }
     __syncthreads();
-    if (tid == 0) {
+    if (tid == 0 && a.intervis) {
       if (s_roundcut < m) atomicMax(a.cuts + par, kMaxPicks + 1 - s_roundcut);
       if (k == 0) __stcg(a.cuts + (par ^ 1), 0);  // read by all before this round's first barrier
     }
     mark(12);
-    // every read of the coverage this round is done once all CTAs pass here
-    if (!group_sync(gb, a.err, &s_flagv)) return;
-    const int latest = __ldcg(a.cuts + par);  // of the smallest cut of any CTA
+    // every read of the coverage this round is done once all CTAs pass here.
+    // Without intervis there is no cut to agree on, and in a spread round the
+    // coverage is read only before the spread barrier: the coverage update
+    // may start at once.  (The buffers reused by the next round are written
+    // only after its first barrier, which every CTA reaches after this one.)
+    if ((a.intervis || !dist) && !group_sync(gb, a.err, &s_flagv)) return;
+    const int latest = a.intervis ? __ldcg(a.cuts + par) : 0;  // of the smallest cut of any CTA
     const int mcut = latest ? kMaxPicks + 1 - latest : m;
     mark(7);
 
@@ -1088,7 +1094,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int g = s_gain[s] - s_dacc[s];
         s_gain[s] = g;
         s_dacc[s] = 0;
-        const bool inel = !(tag & 6);
+        const bool inel = a.intervis && !(tag & 6);
         s_area[s] = inel ? 0 : g;
         s_flag[s] = (unsigned char)((s_flag[s] & ~kInel) | (inel ? kInel : 0));
         s_dirty[s >> 5] = 1;
@@ -1159,11 +1165,17 @@ long long site_stop_area(int nrows) {
   return lo;
 }
 
-namespace {
-
-// Whether a job is selected by local dominance (site_local): any without intervis
-// (1537^2, 18 456 candidates: 0.93 ms against 1.93 ms in the global order; 287^2, 648
-// candidates: 0.24 against 0.19).  With intervis a round also searches for the
+// Without intervis local dominance pays by the picks that a round finds, so the raster
+// has to hold many of a candidate's circles: 30, or 15 from 1024 candidates on.  Its
+// passes over all bins cost what a hundredth of the bins in candidates, and 128, are
+// worth.  560 jobs and calls of 32 to 16 000 candidates, radius 4 to 200: the lines take
+// 1.014 times the better order's time in the mean.  Ms in the global order and by local
+// dominance: 50 circles 351^2, radius 28, 225 candidates 0.62, 0.44; 25 circles 784^2,
+// 99, 1374 1.53, 1.46; 14 circles 920^2, 139, 1369 1.45, 1.60; 19 circles 1301^2, 170,
+// 399 1.76, 2.24; 200 bins a candidate 913^2, 17, 160 0.22, 0.31; 60 candidates 386^2, 7
+// 0.08, 0.21.
+//
+// With intervis a round also searches for the
 // candidates that its picks would uncover (B2).  That pays where many regions are
 // independent and a search meets few candidates: from 16 384 candidates on, with at
 // most 512 in a pick's circle, and at most 64 where more than a twentieth of all cells
@@ -1179,9 +1191,16 @@ namespace {
 // 4.6; below it 1.2).
 bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks) {
   const double n2 = (double)nrows * nrows, circle = 3.14159 * roi * roi / n2 * nsheds;
-  return !intervis || (nblocks <= 1 && nsheds >= 4096 && circle <= 64) ||
+  if (!intervis) {
+    const double bins = (double)local_bins(nrows, roi) * local_bins(nrows, roi);
+    return (nsheds >= 1024 ? nsheds >= 15 * circle : nsheds >= 128 && nsheds >= 30 * circle) &&
+           bins <= 100.0 * nsheds;
+  }
+  return (nblocks <= 1 && nsheds >= 4096 && circle <= 64) ||
          (nsheds >= 16384 && circle <= 512 && (circle <= 64 || 20.0 * nsheds <= n2));
 }
+
+namespace {
 
 size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, bool local,
                       unsigned char *base, SiteScratch *s) {
@@ -1246,15 +1265,13 @@ size_t round16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 }  // namespace
 
-size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis, int nblocks) {
-  return scratch_layout(nrows, nsheds, nctas, roi, intervis,
-                        site_is_local(nrows, nsheds, roi, intervis, nblocks), nullptr, nullptr);
+size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis, bool local) {
+  return scratch_layout(nrows, nsheds, nctas, roi, intervis, local, nullptr, nullptr);
 }
 
 void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,
-                        int nblocks, SiteScratch *s) {
-  scratch_layout(nrows, nsheds, nctas, roi, intervis, site_is_local(nrows, nsheds, roi, intervis, nblocks),
-                 static_cast<unsigned char *>(base), s);
+                        bool local, SiteScratch *s) {
+  scratch_layout(nrows, nsheds, nctas, roi, intervis, local, static_cast<unsigned char *>(base), s);
 }
 
 // Up to one CTA per SM, about 100 candidates per CTA but at least 32 CTAs:
@@ -1395,7 +1412,7 @@ SiteArgs make_site_args(const SiteJob &j, int block0) {
   a.stop_area = site_stop_area(j.nrows);
   a.block0 = block0;
   a.local = j.scratch.local;
-  a.use_local = site_is_local(j.nrows, j.nsheds, j.roi, j.intervis, j.nblocks);
+  a.use_local = j.local;
   a.local_words = (int)((kLocalSmem - sizeof(LocalShared)) / 8);
   return a;
 }
@@ -1492,10 +1509,10 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
 
 cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int32_t *obs,
                         const uint64_t *sheds, float blocksize, int nblocks, int npb,
-                        uint8_t *selected, const SiteScratch &s, int nctas, int *d_err,
+                        uint8_t *selected, const SiteScratch &s, int nctas, int *d_err, bool local,
                         cudaStream_t st) {
   SiteJob j{nrows, roi, intervis, nsheds, obs, sheds, blocksize, nblocks, npb, selected, s, nctas,
-            d_err};
+            d_err, local};
   return launch_site_jobs(&j, 1, s.table, nullptr, st);
 }
 
@@ -1571,14 +1588,15 @@ extern "C" int siting_site_it_noalloc(int nrows, int roi, int intervis, int nshe
   if (site_smem_bytes(roi, nsheds, G, 1, nsheds, bs) > 220 * 1024) return SITING_EINVAL;
   if (scratch_layout(nrows, nsheds, G, roi, 1, false, nullptr, nullptr) + 256 > kNoAllocLimit)
     return SITING_ENOMEM;
-  const size_t need = site_scratch_bytes(nrows, nsheds, G, roi, intervis, 1) + 256;  // + error flag
+  const bool local = site_is_local(nrows, nsheds, roi, intervis, 1);
+  const size_t need = site_scratch_bytes(nrows, nsheds, G, roi, intervis, local) + 256;  // + error flag
   if (need > kNoAllocScratchBytes) return SITING_ENOMEM;
   void *base = nullptr;
   int rc = noalloc_scratch(&base);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   SiteScratch s;
-  site_carve_scratch(base, nrows, nsheds, G, roi, intervis, 1, &s);
+  site_carve_scratch(base, nrows, nsheds, G, roi, intervis, local, &s);
   int *d_err = reinterpret_cast<int *>(static_cast<unsigned char *>(base) + need - 256);
   // zero coverage, key lists, cuts, self-check counters, barrier and outputs
   if (cudaMemsetAsync(base, 0, (unsigned char *)s.order - (unsigned char *)base, st) != cudaSuccess ||
@@ -1595,7 +1613,7 @@ extern "C" int siting_site_it_noalloc(int nrows, int roi, int intervis, int nshe
   if (herr & kErrBadInput) return SITING_EINVAL;
   if (herr) return SITING_ECUDA;
   if (launch_site(nrows, roi, intervis, nsheds, d_obs, d_sheds, bs, 1, nsheds, d_selected, s, G,
-                  d_err, st) != cudaSuccess)
+                  d_err, local, st) != cudaSuccess)
     return SITING_ECUDA;
   long long out[3] = {0, 0, 0};
   if (cudaMemcpyAsync(out, s.out, sizeof(out), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -132,6 +132,7 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
   if (n == N && g.nwanted > 0) {
     const int gmin = (g.nwanted + 4095) / 4096;
     const int gdef = site_default_ctas(g.nwanted, ctx->sm_count);
+    const bool local = site_is_local(n, g.nwanted, p->roi, p->intervis, g.nblocks);
     std::vector<int> cands = {gdef, std::max(gmin, gdef / 2), std::max(gmin, gdef / 4)};
     std::sort(cands.begin(), cands.end());
     cands.erase(std::unique(cands.begin(), cands.end()), cands.end());
@@ -142,17 +143,17 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
               220 * 1024)
         continue;
       void *sp;
-      const size_t sb = site_scratch_bytes(n, g.nwanted, G, p->roi, p->intervis, g.nblocks);
+      const size_t sb = site_scratch_bytes(n, g.nwanted, G, p->roi, p->intervis, local);
       if ((rc = ws_get(ctx, kSite, sb, &sp))) return rc;
       SiteScratch s;
-      site_carve_scratch(sp, n, g.nwanted, G, p->roi, p->intervis, g.nblocks, &s);
+      site_carve_scratch(sp, n, g.nwanted, G, p->roi, p->intervis, local, &s);
       float t;
       rc = time_ms(ctx, [&] {
         cudaError_t e = cudaMemsetAsync(sp, 0, (unsigned char *)s.order - (unsigned char *)sp, st);
         if (e != cudaSuccess) return e;
         return launch_site(n, p->roi, p->intervis, g.nwanted, static_cast<int32_t *>(d_obs),
                            static_cast<uint64_t *>(d_sheds), g.blocksize, g.nblocks,
-                           g.nwantedperblock, static_cast<uint8_t *>(d_sel), s, G, err, st);
+                           g.nwantedperblock, static_cast<uint8_t *>(d_sel), s, G, err, local, st);
       }, &t);
       if (rc) return rc;
       if (t < bt) {

@@ -1,0 +1,56 @@
+"""SITE in the global key order and by local dominance: the same picks in the same order.
+
+Few, dense, sparse and equal candidates, with and without intervis, on both sides of the
+lines by which the order is chosen; each pinned and chosen.  Every result is a whole
+number, so all are compared exactly.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n, roi, count", [
+    (40, 5, 1), (60, 9, 31), (200, 4, 127), (200, 4, 128), (300, 3, 129), (97, 40, 60),
+    (33, 16, 500), (64, 3, 300), (50, 1, 2500), (300, 31, 1023), (300, 31, 1024), (300, 63, 700),
+    (300, 64, 700), (260, 46, 1100), (260, 48, 1100), (900, 7, 160), (130, 130, 200),
+])
+@pytest.mark.parametrize("intervis", [0, 1])
+def test_both_orders_match_the_sequential_greedy(native, oracle, n, roi, count, intervis):
+    rng = np.random.default_rng(n + roi + count)
+    dem = native.fbm_dem(n, seed=n + roi, octaves=7, range_max=6000)
+    obs = rng.integers(0, n * n, count).astype(np.int32)  # any order, some cells twice
+    sheds = oracle.sheds(dem, n, roi, 20, 20, obs)
+    want, used, area, order = oracle.site(n, roi, intervis, obs, sheds, want_order=True)
+    for ctas in (0, 1, 7):
+        for how in (0, 1, 2):
+            with native.Context(0) as ctx:
+                ctx.set_site_ctas(ctas)
+                ctx.set_site_order(how)
+                sel, res = ctx.site_it(n, roi, intervis, obs, sheds)
+                got = ctx.last_pick_order(count)
+            assert np.array_equal(got, order), f"{ctas} CTAs, order {how}"
+            assert np.array_equal(sel, want)
+            assert (res.nusedsheds, res.cumarea) == (used, area)
+
+
+@pytest.mark.parametrize("n, roi, bw, count, intervis", [
+    (287, 20, 12, 648, 0), (287, 90, 12, 648, 0), (512, 60, 25, 400, 0), (400, 9, 20, 1600, 1)])
+def test_jobs_in_both_orders(native, oracle, n, roi, bw, count, intervis):
+    dem = native.fbm_dem(n, seed=n, octaves=7, range_max=6000)
+    ref = oracle.run(dem, n, roi, 20, 16, bw, count, intervis)
+    p = native.Params(nrows=n, roi=roi, height=20, ntests=16, bw=bw, nwanted0=count, intervis=intervis)
+    for how in (0, 1, 2):
+        with native.Context(0) as ctx:
+            ctx.set_site_order(how)
+            obs, sel, res = ctx.run(p, dem)
+        assert np.array_equal(obs, ref["obs"])
+        assert np.array_equal(sel, ref["selected"]), f"order {how}"
+        assert (res.nusedsheds, res.cumarea) == (ref["nused"], ref["cumarea"])
+
+
+def test_an_unknown_order_is_refused(native):
+    with native.Context(0) as ctx:
+        for how in (-1, 3):
+            with pytest.raises(native.SitingError):
+                ctx.set_site_order(how)
