@@ -64,6 +64,7 @@ constexpr int kMaxSlots = 4096;  // candidates owned by one CTA
 // rounds with 3, 4, 6 or 8), and fewer keys make each merge cheaper.
 constexpr int kTopK = 3;
 constexpr int kFewKeys = 256;     // published keys that one warp orders
+constexpr int kFewPicks = 4;      // where the round before took at most so many picks
 constexpr int kMaxPicks = 64;    // picks accepted in one round at most
 constexpr int kSmallRecip = 128; // reciprocals tabled in shared memory (>= kMaxPicks)
 constexpr int kMaxPairs = 8192;  // (candidate, pick) pairs one CTA updates per round
@@ -175,7 +176,11 @@ __global__ void __launch_bounds__(256) site_score_kernel(const uint64_t *sheds, 
 // B for few published keys, by one warp: it takes the largest again and again, a
 // handful a round, where the general form below ranks all of them (SITE ms ranked and so:
 // 256^2, 1024 candidates 0.74, 0.72; 370^2, 1152 0.66, 0.63; 743^2, 8649 0.69, 0.66;
-// 1741^2, 23 762 3.33, 3.16).  A function of its own: inside the round's loop its code
+// 1741^2, 23 762 3.33, 3.16).  A pick costs a turn, so rounds of many are ranked: sparse
+// candidates give 30 and more (of 140 jobs, the 65 with more than 100 circles on the raster
+// took 1.01 times their time before this form where every round took it by turns up to 12
+// picks, 1.07 with no such limit, and 1.00 with a limit of 4; the other 75 0.96 in each).
+// A function of its own: inside the round's loop its code
 // costs the larger jobs 2-4%.  Returns the number of picks and, from bit 8 on, that at
 // the 95% stop plus one.
 __device__ __noinline__ int few_picks(const SiteArgs &a, int par, int max_m, long long cumv,
@@ -371,7 +376,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   mark(0);
 
   uint64_t *cum = a.cum0;
-  int npicks = 0, rounds = 0, nprev = 0;
+  int npicks = 0, rounds = 0, nprev = kMaxPicks;
   const int lim2 = 4 * roi * roi;
 
   for (;;) {
@@ -432,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (!group_sync(gb, a.err, &s_flagv)) return;
     mark(2);
     // ---- B. merge the published lists; accept the exact prefix --------------
-    if (GK <= kFewKeys) {
+    if (GK <= kFewKeys && nprev <= kFewPicks) {
       if (warp == 0) {
         const int got = few_picks(a, par, min(kMaxPicks, a.pair_cap / max(pcap, 1)), s_cum, s_pk,
                                   s_ppos, s_pkey, s_pbox, s_rrun);
