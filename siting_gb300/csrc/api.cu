@@ -234,9 +234,10 @@ int site_ctas_for(siting_ctx *ctx, int roi, int nsheds, int nb, int npb, float b
 
 // Enqueues SITE on device buffers, then copies its outputs and the error flag
 // into the context's pinned readout (collected by site_collect after a sync).
+// `foreign`: the viewsheds are the caller's, so bits beyond roi are looked for.
 int site_enqueue(siting_ctx *ctx, int nrows, int roi, int intervis, int nsheds,
                  const int32_t *d_obs, const uint64_t *d_sheds, float bs, int nb, int npb,
-                 uint8_t *d_selected, int *d_err) {
+                 uint8_t *d_selected, int *d_err, bool foreign) {
   if (!ctx->h_out) CK(cudaMallocHost(&ctx->h_out, 16 * sizeof(long long)));
   memset(ctx->h_out, 0, 16 * sizeof(long long));
   if (nsheds <= 0) return SITING_OK;
@@ -257,7 +258,7 @@ int site_enqueue(siting_ctx *ctx, int nrows, int roi, int intervis, int nsheds,
   CK(cudaMemsetAsync(p, 0, (unsigned char *)s.order - (unsigned char *)p, ctx->stream));
   CK(cudaMemsetAsync(d_selected, 0, nsheds, ctx->stream));
   CK(launch_site(nrows, roi, intervis, nsheds, d_obs, d_sheds, bs, nb, npb, d_selected, s, G,
-                 d_err, local, ctx->stream));
+                 d_err, local, foreign, ctx->stream));
   CK(cudaMemcpyAsync(ctx->h_out, s.out, (3 + kSitePhases) * sizeof(long long), cudaMemcpyDeviceToHost,
                      ctx->stream));
   ctx->d_last_order = s.order;
@@ -513,7 +514,7 @@ int siting_site_it_dev(siting_ctx *ctx, int nrows, int roi, int intervis, int ns
   CK(launch_check_obs(d_obs, nsheds, nrows, d_err, ctx->stream));
   if ((rc = check_err_flag(ctx, d_err))) return rc;
   rc = site_enqueue(ctx, nrows, roi, intervis, nsheds, d_obs, d_sheds, (float)nrows, 1, nsheds,
-                    d_selected, d_err);
+                    d_selected, d_err, true);
   if (rc) return rc;
   if ((rc = check_err_flag(ctx, d_err))) return rc;
   site_collect(ctx, nrows, res);
@@ -669,7 +670,7 @@ static int run_pipeline(siting_ctx *ctx, const siting_params *p, const DemView &
   CK(cudaEventRecord(ctx->ev[3], st));
   if ((rc = site_enqueue(ctx, n, p->roi, p->intervis, g.nwanted, d_obs,
                         static_cast<const uint64_t *>(d_sheds), g.blocksize, g.nblocks,
-                        g.nwantedperblock, d_selected, d_err)))
+                        g.nwantedperblock, d_selected, d_err, false)))
     return rc;
   CK(cudaEventRecord(ctx->ev[4], st));
   if ((rc = check_err_flag(ctx, d_err))) return rc;  // synchronizes the stream

@@ -387,7 +387,7 @@ int run_batch(siting_ctx *ctx, int njobs, const siting_params *params,
       sj.push_back(SiteJob{J.n, J.p.roi, J.p.intervis, J.g.nwanted, obs_of(j),
                            reinterpret_cast<const uint64_t *>(base + J.o_sheds), J.g.blocksize,
                            J.g.nblocks, J.g.nwantedperblock, sel_of(j), s, J.G,
-                           reinterpret_cast<int *>(base + J.o_err), J.local});
+                           reinterpret_cast<int *>(base + J.o_err), J.local, false});
     }
     CK(launch_site_jobs(sj.data(), (int)sj.size(), base + o_wtabs + o_wtab[w],
                         stage + s_wtabs + o_wtab[w], st2));

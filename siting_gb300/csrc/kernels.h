@@ -96,6 +96,7 @@ cudaError_t launch_findmax_queue(const StageJob *jobs, int njobs, cudaStream_t s
 // ---- SITE -----------------------------------------------------------------------
 // Device scratch of a selection (site_local.cuh).
 struct LocalScratch {
+  unsigned *leave;             // nonzero: in the global order after all; zeroed
   unsigned *count;             // [bins+1]: candidates of each bin, then their ranges' starts; zeroed
   unsigned *fill;              // [bins]; zeroed
   unsigned long long *gmax;    // [2]: the round's largest key; zeroed
@@ -120,14 +121,14 @@ struct SiteScratch {
   uint64_t *nbits;           // the round's new bits of each pick: [64][nr][nwpr+1] words
   unsigned char *nmask;      // [64][nr]: bit j set when word j of that new-bit row is nonzero
   unsigned long long *topk;  // [2][nctas][top-K] x {key, cell}: published top keys
-  int *cuts;                 // [2] of [2][nctas]: the smallest cut of the round's prefix (intervis)
+  int *cuts;                 // [2]: the smallest cut of the round's prefix (intervis)
   int *ncount;               // [2][64]: popcount of each pick's new bits (self-check)
   unsigned *bar;             // group barrier counter, zeroed
   long long *out;            // [0] nused, [1] cumarea, [2] rounds, [3..15] phase cycles
   int32_t *order;            // nsheds: picks in order
   int32_t *gains;            // nsheds: round-1 gains (site_score_kernel)
   void *table;               // job table of a one-job launch (site_job_table_bytes)
-  LocalScratch local;        // without intervis
+  LocalScratch local;        // of a job by local dominance
 };
 
 // Phases of the SITE tracing clocks (siting_last_site_phase_cycles).
@@ -145,6 +146,7 @@ struct SiteJob {
   int nctas;
   int *err;
   bool local;  // by local dominance (as its scratch was laid out)
+  bool check;  // the viewsheds may have bits beyond roi: then in the global order
 };
 // Device bytes of a job table for `njobs` jobs and `total_ctas` CTAs.
 size_t site_job_table_bytes(int njobs, int total_ctas);
@@ -171,6 +173,6 @@ bool site_supported(int roi, int nsheds, int nctas);
 cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int32_t *obs,
                         const uint64_t *sheds, float blocksize, int nblocks, int npb,
                         uint8_t *selected, const SiteScratch &s, int nctas, int *d_err, bool local,
-                        cudaStream_t st);
+                        bool check, cudaStream_t st);
 
 }  // namespace siting

@@ -320,7 +320,7 @@ int siting_server::launch_site(long long id, Request &r) {
   CK(cudaStreamWaitEvent(site, r.staged, 0));
   CK(cudaMemsetAsync(d_sel, 0, J.g.nwanted, site));
   SiteJob sj{J.n, J.p.roi, J.p.intervis, J.g.nwanted, d_obs, d_sheds, J.g.blocksize,
-             J.g.nblocks, J.g.nwantedperblock, d_sel, s, J.G, err, J.local};
+             J.g.nblocks, J.g.nwantedperblock, d_sel, s, J.G, err, J.local, false};
   CK(launch_site_jobs(&sj, 1, base + bp.o_wtabs + bp.o_wtab[0], pin + L.wtab, site));
   long long *hout = reinterpret_cast<long long *>(pin + L.out);
   CK(cudaMemcpyAsync(hout, s.out, 3 * sizeof(long long), cudaMemcpyDeviceToHost, site));

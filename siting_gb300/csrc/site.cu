@@ -151,8 +151,31 @@ constexpr unsigned char kUsed = 1, kInel = 4;
 // Round 1 (siting.cpp:537-549 with nusedsheds == 0): the gain of every
 // candidate against an empty coverage is the popcount of its shed.  One warp
 // per shed, 128-bit loads, grid-stride: a pure HBM stream over all sheds.
+// kBeyond: *beyond is set where a shed has a bit farther than roi from its observer.
+template <bool kBeyond>
 __global__ void __launch_bounds__(256) site_score_kernel(const uint64_t *sheds, int nsheds,
-                                                         int per, int *gains) {
+                                                         int per, int *gains, int roi,
+                                                         unsigned *beyond) {
+  extern __shared__ int s_half[];  // half the disc's width at each row distance
+  const int nwpr = (2 * roi + 64) / 64;
+  if constexpr (kBeyond) {
+    for (int d = threadIdx.x; d <= roi; d += blockDim.x) {
+      const int left = roi * roi - d * d;
+      int h = (int)sqrtf((float)left);
+      while (h * h > left) h--;
+      while ((h + 1) * (h + 1) <= left) h++;
+      s_half[d] = h;
+    }
+    __syncthreads();
+  }
+  uint64_t out = 0;  // bits beyond the disc
+  auto look = [&](int i, uint64_t v) {
+    if constexpr (kBeyond) {
+      const int row = i / nwpr, c0 = 64 * (i - row * nwpr), h = s_half[abs(row - roi)];
+      const int lo = max(roi - h - c0, 0), hi = min(roi + h - c0, 63);  // the disc's columns
+      out |= lo <= hi ? v & ~((~0ull >> lo) & (~0ull << (63 - hi))) : v;
+    }
+  };
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nsheds; c += warps) {
@@ -163,14 +186,21 @@ __global__ void __launch_bounds__(256) site_score_kernel(const uint64_t *sheds, 
       for (int i = lane; i < per / 2; i += 32) {
         const ulonglong2 q = __ldg(v + i);
         cnt += __popcll(q.x) + __popcll(q.y);
+        look(2 * i, q.x);
+        look(2 * i + 1, q.y);
       }
     } else {
-      for (int i = lane; i < per; i += 32) cnt += __popcll(__ldg(sh + i));
+      for (int i = lane; i < per; i += 32) {
+        const uint64_t q = __ldg(sh + i);
+        cnt += __popcll(q);
+        look(i, q);
+      }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0) gains[c] = cnt;
   }
+  if (kBeyond && out) atomicOr(beyond, 1u);
 }
 
 // B for few published keys, by one warp: it takes the largest again and again, a
@@ -277,10 +307,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < kSitePhases; i++) s_ph[i] = 0;
     s_tmark = clock64();
   }
-  if (a.use_local) {
-    site_local(a, *reinterpret_cast<LocalShared *>(sm), (int)blockIdx.x - a.block0, s_ph, &s_tmark);
+  GroupBarrier gb{a.bar, (unsigned)a.G, 0u};
+  if (a.use_local && site_local(a, *reinterpret_cast<LocalShared *>(sm), (int)blockIdx.x - a.block0,
+                                gb, s_ph, &s_tmark))
     return;
-  }
   __shared__ int s_m, s_stop_at, s_done, s_flagv, s_roundcut, s_npair, s_nvalid;
   __shared__ long long s_cum;
   __shared__ int s_poff[kMaxPicks + 1];
@@ -344,7 +374,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t *s_N = reinterpret_cast<uint64_t *>(take((size_t)a.ncap_words * 8));
   unsigned char *s_nmask = take(kMaskCap);
 
-  GroupBarrier gb{a.bar, (unsigned)G, 0u};
   auto mark = [&](int i) {
     if (k == 0 && tid == 0) {
       const long long now = clock64();
@@ -1229,7 +1258,11 @@ size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, b
   const size_t bins = local ? (size_t)local_bins(nrows, roi) * local_bins(nrows, roi) : 0;
   const size_t cells = local ? (size_t)local_cells(nrows, roi) * local_cells(nrows, roi) : 0;
   const int cap = local ? local_cap(roi) : kMaxPicks;
+  carve(t.topk, (size_t)2 * nctas * kTopK * 2 * 8);
+  carve(t.cuts, (size_t)2 * 4);
+  carve(t.ncount, (size_t)2 * kMaxPicks * 4);
   if (local) {
+    carve(l.leave, 4);
     carve(l.count, (bins + 1) * 4);
     carve(l.fill, bins * 4);
     carve(l.gmax, 16);
@@ -1237,14 +1270,11 @@ size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, b
     carve(l.npick, 8);
     carve(l.ncount, (size_t)2 * cap * 4);
     if (intervis) carve(l.bad, 2 * cells * 4);
-  } else {
-    carve(t.topk, (size_t)2 * nctas * kTopK * 2 * 8);
-    carve(t.cuts, (size_t)2 * nctas * 4);
-    carve(t.ncount, (size_t)2 * kMaxPicks * 4);
   }
   carve(t.order, (size_t)nsheds * 4);
   carve(t.gains, (size_t)nsheds * 4);
   carve(t.nbits, cap * nr * row);  // every row is written before it is read
+  carve(t.nmask, (size_t)kMaxPicks * nr + 16);  // + the 16-byte loads' tail
   if (local) {
     carve(l.binkey, bins * 8);
     carve(l.binat, bins * 8);
@@ -1258,8 +1288,6 @@ size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, b
       carve(l.preach, (size_t)nsheds * 8);
       carve(l.pparent, (size_t)nsheds * 4);
     }
-  } else {
-    carve(t.nmask, (size_t)kMaxPicks * nr + 16);  // + the 16-byte loads' tail
   }
   t.table = take(site_job_table_bytes(1, nctas));
   if (s) *s = t;
@@ -1438,10 +1466,9 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
     args[i] = make_site_args(jobs[i], total);
     for (int b = 0; b < jobs[i].nctas; b++) block_job.push_back(i);
     total += jobs[i].nctas;
-    shm = std::max(shm, args[i].use_local
-                            ? kLocalSmem
-                            : site_smem_bytes(jobs[i].roi, jobs[i].nsheds, jobs[i].nctas,
-                                              jobs[i].nblocks, jobs[i].npb, jobs[i].blocksize));
+    shm = std::max(shm, site_smem_bytes(jobs[i].roi, jobs[i].nsheds, jobs[i].nctas, jobs[i].nblocks,
+                                        jobs[i].npb, jobs[i].blocksize));
+    if (jobs[i].local) shm = std::max(shm, kLocalSmem);
   }
   if (total == 0) return cudaSuccess;
   // job table: arguments, then the CTA -> job map
@@ -1481,7 +1508,10 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
     sc.stream = st;
     sc.attrs = &prio;
     sc.numAttrs = 1;
-    e = cudaLaunchKernelEx(&sc, site_score_kernel, j.sheds, j.nsheds, per, j.scratch.gains);
+    const bool check = j.local && j.check;
+    sc.dynamicSmemBytes = check ? (size_t)(j.roi + 1) * 4 : 0;
+    e = cudaLaunchKernelEx(&sc, check ? site_score_kernel<true> : site_score_kernel<false>, j.sheds,
+                           j.nsheds, per, j.scratch.gains, j.roi, j.scratch.local.leave);
     if (e != cudaSuccess) return e;
   }
   int threads = 512;
@@ -1515,9 +1545,9 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
 cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int32_t *obs,
                         const uint64_t *sheds, float blocksize, int nblocks, int npb,
                         uint8_t *selected, const SiteScratch &s, int nctas, int *d_err, bool local,
-                        cudaStream_t st) {
+                        bool check, cudaStream_t st) {
   SiteJob j{nrows, roi, intervis, nsheds, obs, sheds, blocksize, nblocks, npb, selected, s, nctas,
-            d_err, local};
+            d_err, local, check};
   return launch_site_jobs(&j, 1, s.table, nullptr, st);
 }
 
@@ -1618,7 +1648,7 @@ extern "C" int siting_site_it_noalloc(int nrows, int roi, int intervis, int nshe
   if (herr & kErrBadInput) return SITING_EINVAL;
   if (herr) return SITING_ECUDA;
   if (launch_site(nrows, roi, intervis, nsheds, d_obs, d_sheds, bs, 1, nsheds, d_selected, s, G,
-                  d_err, local, st) != cudaSuccess)
+                  d_err, local, true, st) != cudaSuccess)
     return SITING_ECUDA;
   long long out[3] = {0, 0, 0};
   if (cudaMemcpyAsync(out, s.out, sizeof(out), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

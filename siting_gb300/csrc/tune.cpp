@@ -153,7 +153,8 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
         if (e != cudaSuccess) return e;
         return launch_site(n, p->roi, p->intervis, g.nwanted, static_cast<int32_t *>(d_obs),
                            static_cast<uint64_t *>(d_sheds), g.blocksize, g.nblocks,
-                           g.nwantedperblock, static_cast<uint8_t *>(d_sel), s, G, err, local, st);
+                           g.nwantedperblock, static_cast<uint8_t *>(d_sel), s, G, err, local, false,
+                           st);
       }, &t);
       if (rc) return rc;
       if (t < bt) {
