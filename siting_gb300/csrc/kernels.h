@@ -96,7 +96,7 @@ cudaError_t launch_findmax_queue(const StageJob *jobs, int njobs, cudaStream_t s
 // ---- SITE -----------------------------------------------------------------------
 // Device scratch of a selection (site_local.cuh).
 struct LocalScratch {
-  unsigned *leave;             // nonzero: in the global order after all; zeroed
+  unsigned long long *near;    // pairs of candidates in one bin, each counted twice, and kBeyond; zeroed
   unsigned *count;             // [bins+1]: candidates of each bin, then their ranges' starts; zeroed
   unsigned *fill;              // [bins]; zeroed
   unsigned long long *gmax;    // [2]: the round's largest key; zeroed
@@ -145,7 +145,7 @@ struct SiteJob {
   SiteScratch scratch;  // zeroed as site_dev does before the launch
   int nctas;
   int *err;
-  bool local;  // by local dominance (as its scratch was laid out)
+  int local;   // 1 by local dominance unless its candidates are crowded, 2 in any case (scratch as laid out)
   bool check;  // the viewsheds may have bits beyond roi: then in the global order
 };
 // Device bytes of a job table for `njobs` jobs and `total_ctas` CTAs.
@@ -172,7 +172,7 @@ size_t site_smem_bytes(int roi, int nsheds, int nctas, int nblocks, int npb, flo
 bool site_supported(int roi, int nsheds, int nctas);
 cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int32_t *obs,
                         const uint64_t *sheds, float blocksize, int nblocks, int npb,
-                        uint8_t *selected, const SiteScratch &s, int nctas, int *d_err, bool local,
+                        uint8_t *selected, const SiteScratch &s, int nctas, int *d_err, int local,
                         bool check, cudaStream_t st);
 
 }  // namespace siting

@@ -95,6 +95,7 @@ struct SiteArgs {
   LocalScratch local;   // of site_local
   int use_local;        // the selection by local dominance
   int local_words;      // shared-memory words for the picks' new bits
+  unsigned long long max_near;  // most pairs in a bin, over all bins and counted twice
 };
 
 }  // namespace
@@ -151,14 +152,19 @@ constexpr unsigned char kUsed = 1, kInel = 4;
 // Round 1 (siting.cpp:537-549 with nusedsheds == 0): the gain of every
 // candidate against an empty coverage is the popcount of its shed.  One warp
 // per shed, 128-bit loads, grid-stride: a pure HBM stream over all sheds.
-// kBeyond: *beyond is set where a shed has a bit farther than roi from its observer.
-template <bool kBeyond>
+// For a job by local dominance it also counts the candidates of each bin and the pairs
+// of candidates that share one (kBins), and looks for bits farther than roi from their
+// observer (kLook); *near then tells whether the job stays one (site_kernel).
+constexpr unsigned long long kBeyond = 1ull << 63;
+
+template <bool kBins, bool kLook>
 __global__ void __launch_bounds__(256) site_score_kernel(const uint64_t *sheds, int nsheds,
-                                                         int per, int *gains, int roi,
-                                                         unsigned *beyond) {
+                                                         int per, int *gains, const int32_t *obs,
+                                                         int n, int roi, unsigned *count,
+                                                         unsigned long long *near) {
   extern __shared__ int s_half[];  // half the disc's width at each row distance
   const int nwpr = (2 * roi + 64) / 64;
-  if constexpr (kBeyond) {
+  if constexpr (kLook) {
     for (int d = threadIdx.x; d <= roi; d += blockDim.x) {
       const int left = roi * roi - d * d;
       int h = (int)sqrtf((float)left);
@@ -169,8 +175,9 @@ __global__ void __launch_bounds__(256) site_score_kernel(const uint64_t *sheds, 
     __syncthreads();
   }
   uint64_t out = 0;  // bits beyond the disc
+  unsigned long long shared_bin = 0;
   auto look = [&](int i, uint64_t v) {
-    if constexpr (kBeyond) {
+    if constexpr (kLook) {
       const int row = i / nwpr, c0 = 64 * (i - row * nwpr), h = s_half[abs(row - roi)];
       const int lo = max(roi - h - c0, 0), hi = min(roi + h - c0, 63);  // the disc's columns
       out |= lo <= hi ? v & ~((~0ull >> lo) & (~0ull << (63 - hi))) : v;
@@ -199,8 +206,14 @@ __global__ void __launch_bounds__(256) site_score_kernel(const uint64_t *sheds, 
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0) gains[c] = cnt;
+    if (kBins && lane == 0) {
+      int pos;
+      const int b = local_bin_of(__ldg(obs + c), n, local_bin_side(n, roi), local_bins(n, roi), &pos);
+      shared_bin += 2ull * atomicAdd(count + b, 1u);
+    }
   }
-  if (kBeyond && out) atomicOr(beyond, 1u);
+  if (kBins && shared_bin) atomicAdd(near, shared_bin);
+  if (kLook && out) atomicOr(near, kBeyond);
 }
 
 // B for few published keys, by one warp: it takes the largest again and again, a
@@ -307,10 +320,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < kSitePhases; i++) s_ph[i] = 0;
     s_tmark = clock64();
   }
-  GroupBarrier gb{a.bar, (unsigned)a.G, 0u};
-  if (a.use_local && site_local(a, *reinterpret_cast<LocalShared *>(sm), (int)blockIdx.x - a.block0,
-                                gb, s_ph, &s_tmark))
+  // Bits beyond roi: a cell may then be covered by two picks that are more than 2*roi
+  // apart, and by one that no search meets.  Pairs in a bin: site_local_limit.
+  if (a.use_local && __ldcg(a.local.near) <= a.max_near) {
+    site_local(a, *reinterpret_cast<LocalShared *>(sm), (int)blockIdx.x - a.block0, s_ph, &s_tmark);
     return;
+  }
   __shared__ int s_m, s_stop_at, s_done, s_flagv, s_roundcut, s_npair, s_nvalid;
   __shared__ long long s_cum;
   __shared__ int s_poff[kMaxPicks + 1];
@@ -374,6 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t *s_N = reinterpret_cast<uint64_t *>(take((size_t)a.ncap_words * 8));
   unsigned char *s_nmask = take(kMaskCap);
 
+  GroupBarrier gb{a.bar, (unsigned)G, 0u};
   auto mark = [&](int i) {
     if (k == 0 && tid == 0) {
       const long long now = clock64();
@@ -1223,15 +1239,36 @@ long long site_stop_area(int nrows) {
 // candidate is a possible neighbour of a pick: there the line is 4096 candidates with 64 in a
 // circle (17 jobs up to 16 384: 0.62 of its time; 1500^2, radius 60, 8836: 3.1 ms against
 // 4.6; below it 1.2).
-bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks) {
-  const double n2 = (double)nrows * nrows, circle = 3.14159 * roi * roi / n2 * nsheds;
+//
+// These lines are on the candidates in a circle.  The host knows their mean over the
+// raster; where they lie close together, the scoring kernel's count of them leaves the
+// job to the global order.
+namespace {
+
+// The most candidates in a pick's circle that local dominance is used for.
+double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblocks) {
   if (!intervis) {
     const double bins = (double)local_bins(nrows, roi) * local_bins(nrows, roi);
-    return (nsheds >= 1024 ? nsheds >= 15 * circle : nsheds >= 128 && nsheds >= 30 * circle) &&
-           bins <= 100.0 * nsheds;
+    if (nsheds < 128 || bins > 100.0 * nsheds) return 0;
+    return nsheds / (nsheds >= 1024 ? 15.0 : 30.0);
   }
-  return (nblocks <= 1 && nsheds >= 4096 && circle <= 64) ||
-         (nsheds >= 16384 && circle <= 512 && (circle <= 64 || 20.0 * nsheds <= n2));
+  const double twentieth = 3.14159 * roi * roi / 20;
+  if (nsheds >= 16384) return std::max(64.0, std::min(512.0, twentieth));
+  return nblocks <= 1 && nsheds >= 4096 ? 64 : 0;
+}
+
+// The same as pairs of candidates in one bin, each counted twice: nsheds times the
+// candidates that one shares its bin with in the mean.
+unsigned long long site_max_near(int nrows, int nsheds, int roi, double limit) {
+  const double side = local_bin_side(nrows, roi);
+  return (unsigned long long)(limit * nsheds * side * side / (3.14159 * roi * roi));
+}
+
+}  // namespace
+
+bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks) {
+  const double circle = 3.14159 * roi * roi / ((double)nrows * nrows) * nsheds;
+  return circle <= site_local_limit(nrows, nsheds, roi, intervis, nblocks);
 }
 
 namespace {
@@ -1262,7 +1299,7 @@ size_t scratch_layout(int nrows, int nsheds, int nctas, int roi, int intervis, b
   carve(t.cuts, (size_t)2 * 4);
   carve(t.ncount, (size_t)2 * kMaxPicks * 4);
   if (local) {
-    carve(l.leave, 4);
+    carve(l.near, 8);
     carve(l.count, (bins + 1) * 4);
     carve(l.fill, bins * 4);
     carve(l.gmax, 16);
@@ -1445,7 +1482,11 @@ SiteArgs make_site_args(const SiteJob &j, int block0) {
   a.stop_area = site_stop_area(j.nrows);
   a.block0 = block0;
   a.local = j.scratch.local;
-  a.use_local = j.local;
+  a.use_local = j.local != 0;
+  a.max_near = j.local == 2 ? kBeyond - 1
+                            : site_max_near(j.nrows, j.nsheds, j.roi,
+                                            site_local_limit(j.nrows, j.nsheds, j.roi, j.intervis,
+                                                             j.nblocks));
   a.local_words = (int)((kLocalSmem - sizeof(LocalShared)) / 8);
   return a;
 }
@@ -1508,10 +1549,13 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
     sc.stream = st;
     sc.attrs = &prio;
     sc.numAttrs = 1;
-    const bool check = j.local && j.check;
-    sc.dynamicSmemBytes = check ? (size_t)(j.roi + 1) * 4 : 0;
-    e = cudaLaunchKernelEx(&sc, check ? site_score_kernel<true> : site_score_kernel<false>, j.sheds,
-                           j.nsheds, per, j.scratch.gains, j.roi, j.scratch.local.leave);
+    sc.dynamicSmemBytes = j.local && j.check ? (size_t)(j.roi + 1) * 4 : 0;
+    e = cudaLaunchKernelEx(&sc,
+                           !j.local  ? site_score_kernel<false, false>
+                           : j.check ? site_score_kernel<true, true>
+                                     : site_score_kernel<true, false>,
+                           j.sheds, j.nsheds, per, j.scratch.gains, j.obs, j.nrows, j.roi,
+                           j.scratch.local.count, j.scratch.local.near);
     if (e != cudaSuccess) return e;
   }
   int threads = 512;
@@ -1544,7 +1588,7 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
 
 cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int32_t *obs,
                         const uint64_t *sheds, float blocksize, int nblocks, int npb,
-                        uint8_t *selected, const SiteScratch &s, int nctas, int *d_err, bool local,
+                        uint8_t *selected, const SiteScratch &s, int nctas, int *d_err, int local,
                         bool check, cudaStream_t st) {
   SiteJob j{nrows, roi, intervis, nsheds, obs, sheds, blocksize, nblocks, npb, selected, s, nctas,
             d_err, local, check};

@@ -476,10 +476,17 @@ __device__ __noinline__ void local_threat(const SiteArgs &a, LocalShared &s, uns
   __syncthreads();
 }
 
+// The bin of a cell, and the cell as row and column.
+__device__ __forceinline__ int local_bin_of(int cell, int n, int side, int nbin, int *pos) {
+  const int x = cell / n, y = cell - x * n;
+  *pos = (int)((unsigned)x << 16) | y;
+  return (x / side) * nbin + y / side;
+}
+
 // The whole selection of one job by the G CTAs of its group; k is this CTA's
-// place in it.  False: nothing is selected, the job is one for the global order.
-__device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, int k,
-                                           GroupBarrier &gb, long long *phase, long long *tmark) {
+// place in it.
+__device__ __forceinline__ void site_local(const SiteArgs &a, LocalShared &s, int k,
+                                           long long *phase, long long *tmark) {
   const LocalScratch &L = a.local;
   const int G = a.G, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int T = blockDim.x, nwarps = T >> 5;
@@ -492,6 +499,7 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
   const int cap = local_cap(roi);
   uint64_t *N = reinterpret_cast<uint64_t *>(&s + 1);
   const bool iv = a.intervis;
+  GroupBarrier gb{a.bar, (unsigned)G, 0u};
   auto mark = [&](int i) {
     if (k == 0 && tid == 0) {
       const long long now = clock64();
@@ -500,21 +508,7 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
     }
   };
 
-  // Viewsheds with bits beyond roi: a cell may then be covered by two picks that are more
-  // than 2*roi apart, and by one that no search meets.
-  if (__ldcg(L.leave)) return false;
-
-  // ---- candidates into bins ------------------------------------------------------
-  auto bin_of = [&](int cell, int *pos) {
-    const int x = cell / n, y = cell - x * n;
-    *pos = (int)((unsigned)x << 16) | y;
-    return (x / side) * nbin + y / side;
-  };
-  for (int c = gtid; c < a.nsheds; c += gthreads) {
-    int pos;
-    atomicAdd(L.count + bin_of(__ldg(a.obs + c), &pos), 1u);
-  }
-  if (!group_sync(gb, a.err, &s.flag)) return true;
+  // ---- candidates into bins (counted with the round-1 gains) ---------------------------
   if (k == 0) {  // exclusive prefix sums, in place
     const int each = (nbins + T - 1) / T, b0 = min(tid * each, nbins), b1 = min(b0 + each, nbins);
     unsigned sum = 0;
@@ -536,17 +530,17 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
     }
     if (tid == 0) __stcg(L.count + nbins, (unsigned)a.nsheds);
   }
-  if (!group_sync(gb, a.err, &s.flag)) return true;
+  if (!group_sync(gb, a.err, &s.flag)) return;
   for (int c = gtid; c < a.nsheds; c += gthreads) {
     int pos;
-    const int b = bin_of(__ldg(a.obs + c), &pos);
+    const int b = local_bin_of(__ldg(a.obs + c), n, side, nbin, &pos);
     const unsigned at = __ldcg(L.count + b) + atomicAdd(L.fill + b, 1u);
     __stcg(L.rec + at, make_int4(pos, __ldcg(a.gains + c), c, 0));
   }
   if (tid == 0) s.total = 0;
   if (iv)
     for (int i = gtid; i < G * kLocalSearch; i += gthreads) __stcg(L.search + i, 0u);
-  if (!group_sync(gb, a.err, &s.flag)) return true;
+  if (!group_sync(gb, a.err, &s.flag)) return;
   mark(0);
 
   uint64_t *cum = a.cum0;
@@ -611,7 +605,7 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
       if (mine) atomicMax(L.gmax + par, mine);
     }
     mark(1);
-    if (!group_sync(gb, a.err, &s.flag)) return true;
+    if (!group_sync(gb, a.err, &s.flag)) return;
     mark(2);
     // ---- the end: no area left, or every pick before the stop is taken ------------
     const unsigned long long M = __ldcg(L.gmax + par);
@@ -724,7 +718,7 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
       }
     }
     mark(3);
-    if (!group_sync(gb, a.err, &s.flag)) return true;
+    if (!group_sync(gb, a.err, &s.flag)) return;
     mark(4);
     int m = iv ? (int)__ldcg(L.ndom + par) : min((int)__ldcg(L.npick + par), cap);
     int *bad = L.bad + par * ncell * ncell;
@@ -754,7 +748,7 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
                               nbin, d / m, parts);
       }
       mark(10);
-      if (!group_sync(gb, a.err, &s.flag)) return true;
+      if (!group_sync(gb, a.err, &s.flag)) return;
       if (parts > 1)
         for (int i = gtid; i < m * kLocalSearch; i += gthreads) __stcg(L.search + i, 0u);
       mark(11);
@@ -865,7 +859,7 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
       if (tid == 0) s.prefix[0] = 0;
     }
     mark(5);
-    if (!group_sync(gb, a.err, &s.flag)) return true;
+    if (!group_sync(gb, a.err, &s.flag)) return;
     mark(6);
     // ---- D. the neighbours' gains, the coverage ---------------------------------------
     for (int i = gtid; i < m * nr * nb2; i += gthreads) {
@@ -969,7 +963,7 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
     if (tid == 0) s.total += areas;
     np += m;
     mark(7);
-    if (!group_sync(gb, a.err, &s.flag)) return true;
+    if (!group_sync(gb, a.err, &s.flag)) return;
     mark(8);
   }
 
@@ -1041,7 +1035,6 @@ __device__ __forceinline__ bool site_local(const SiteArgs &a, LocalShared &s, in
       for (int i = 0; i < kSitePhases; i++) a.out[3 + i] = phase[i];
     }
   }
-  return true;
 }
 
 }  // namespace
