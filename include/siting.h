@@ -121,7 +121,8 @@ int siting_ctx_set_site_ctas(siting_ctx *ctx, int nctas);
 /* Tuning knob: how SITE of single jobs takes its picks (batches and servers choose
  * for each job).  1 = in the global key order, the longest prefix of it without a
  * conflict a round, 2 = by local dominance, every candidate that nothing within 2*roi
- * can precede a round, 0 = automatic, by the number and the spread of the candidates.
+ * can precede a round (where it applies: radius at most 992, no viewshed bits farther
+ * than roi), 0 = automatic, by the number and the spread of the candidates.
  * Results do not depend on it. */
 int siting_ctx_set_site_order(siting_ctx *ctx, int order);
 /* Tuning knob of the batched form (no counterpart in the reference): how a

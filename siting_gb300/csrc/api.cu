@@ -247,7 +247,7 @@ int site_enqueue(siting_ctx *ctx, int nrows, int roi, int intervis, int nsheds,
   if (site_smem_bytes(roi, nsheds, G, nb, npb, bs) > 220 * 1024)
     return fail(ctx, SITING_EINVAL, "SITE: shared-memory plan exceeds 220 KB");
   void *p;
-  const int local = ctx->site_order == kOrderLocal ? 2
+  const int local = ctx->site_order == kOrderLocal ? 2 * site_may_be_local(roi)
                     : ctx->site_order == kOrderAuto && site_is_local(nrows, nsheds, roi, intervis, nb);
   const size_t sb = site_scratch_bytes(nrows, nsheds, G, roi, intervis, local);
   int rc = ws_get(ctx, kSite, sb, &p);

@@ -157,7 +157,9 @@ size_t site_job_table_bytes(int njobs, int total_ctas);
 // kept unchanged until the copy has run; NULL stages through pageable memory.
 cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void *h_stage,
                              cudaStream_t st);
-// Whether a job is faster by local dominance than in the global key order.
+// Whether a job can be selected by local dominance, and is faster so than in the global
+// key order.
+bool site_may_be_local(int roi);
 bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks);
 size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis, bool local);
 void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,

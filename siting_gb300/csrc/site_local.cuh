@@ -88,6 +88,8 @@ __host__ __device__ __forceinline__ int local_bins(int n, int roi) {
 __host__ __device__ __forceinline__ int local_cells(int n, int roi) {
   return (local_bins(n, roi) + kLocalCell - 1) / kLocalCell;
 }
+// Whether a placed row of a window has a lane of a warp for each word (radius <= 992).
+__host__ __device__ __forceinline__ bool local_width(int roi) { return (2 * roi + 64) / 64 + 1 <= 32; }
 // Picks a round takes at most: while their new bits take at most 8 MB (4 MB of it
 // is 256 picks at radius 64), and 64 in any case.
 __host__ __device__ __forceinline__ int local_cap(int roi) {
@@ -191,20 +193,17 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v,
 // |placed(shed of u) n N_p| over the rows and words that the two windows share, by
 // one warp, consecutive lanes on consecutive words (a lane a row reads each line
 // of the shed once a word: 2.8 times the wavefronts); kShared: N_p in shared memory.
-// Of the shared words only 32 from the 32*part-th on: from radius 993 on there can be
-// more (bits of so wide a window are never in shared memory).
+// The windows share at most 32 words of a row (local_width).
 template <bool kShared>
 __device__ __forceinline__ int local_pair(const uint64_t *shed, const uint64_t *nbits, int n, int cw,
-                                          int roi, int cpos, int ppos, int lane, int part) {
+                                          int roi, int cpos, int ppos, int lane) {
   const int nr = 2 * roi + 1, nwpr = (nr + 63) / 64, nb2 = nwpr + 1;
   const int cx = row_of(cpos), cy = cpos & 0xffff, px = row_of(ppos), py = ppos & 0xffff;
   // rows of u's shed inside the pick's window and the DEM, words of the row in both
   const int r0 = max(max(0, px - cx), roi - cx);
   const int r1 = min(min(nr - 1, px - cx + 2 * roi), n - 1 - cx + roi);
   const int fwc = (cy - roi) >> 6, fbc = (cy - roi) & 63, fwp = (py - roi) >> 6;
-  const int lo = max(max(fwc, fwp), 0) + (kShared ? 0 : 32 * part);
-  const int last = min(min((cy + roi) >> 6, fwp + nwpr), cw - 1);
-  const int hi = kShared ? last : min(last, lo + 31);
+  const int lo = max(max(fwc, fwp), 0), hi = min(min((cy + roi) >> 6, fwp + nwpr), cw - 1);
   const int nw = hi - lo + 1, total = nw > 0 ? max(0, r1 - r0 + 1) * nw : 0;
   if (total == 0) return 0;
   // A lane keeps its word of the row and takes every `rows`-th row.  u's word uq
@@ -249,11 +248,9 @@ __device__ __forceinline__ void local_pairs(const SiteArgs &a, LocalShared &s, c
     j = __shfl_sync(0xffffffffu, j, 0);
     if (j >= s.n) break;
     const int p = s.pair_pick[j];
-    int d = 0;
-    for (int part = 0; part < (kShared ? 1 : (nwpr + 32) / 32); part++)
-      d += local_pair<kShared>(a.sheds + (size_t)s.pair_cand[j] * per,
-                               N + (size_t)(p - first) * nper, a.n, cw, a.roi, s.pair_pos[j],
-                               s.pos[p], lane, part);
+    const int d = local_pair<kShared>(a.sheds + (size_t)s.pair_cand[j] * per,
+                                      N + (size_t)(p - first) * nper, a.n, cw, a.roi,
+                                      s.pair_pos[j], s.pos[p], lane);
     if (d && lane == 0) atomicSub(&a.local.rec[s.pair_at[j]].y, d);
   }
 }

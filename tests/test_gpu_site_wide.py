@@ -43,8 +43,9 @@ def test_windows_of_more_words_than_lanes(native, oracle, n, roi, intervis):
     want, used, area, order = oracle.site(n, roi, intervis, obs, sheds, want_order=True)
     assert used > 1  # later picks' areas have lost the earlier ones' cells
     with native.Context(0) as ctx:
-        sel, res = ctx.site_it(n, roi, intervis, obs, sheds)
-        got = ctx.last_pick_order(len(obs))
-    assert np.array_equal(got, order)
-    assert np.array_equal(sel, want)
-    assert (res.nusedsheds, res.cumarea) == (used, area)
+        for how in (2, 1):
+            ctx.set_site_order(how)
+            sel, res = ctx.site_it(n, roi, intervis, obs, sheds)
+            assert np.array_equal(ctx.last_pick_order(len(obs)), order), f"order {how}"
+            assert np.array_equal(sel, want)
+            assert (res.nusedsheds, res.cumarea) == (used, area)
