@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ int s_rank[kMaxPicks], s_rpos[kMaxPicks];
 
   const int G = a.G, k = blockIdx.x - a.block0;
+  const bool iv = a.intervis;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int n = a.n, roi = a.roi, nr = 2 * roi + 1, nwpr = (nr + 63) / 64;
   const int nb2 = nwpr + 1;            // words of a placed row
@@ -719,7 +720,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           s_pairslot[pr] = s;
           s_pairdelta[pr] = 0;
           unsigned char cv = 0;
-          if (a.intervis)  // own cell already covered?
+          if (iv)  // own cell already covered?
             cv = (unsigned char)(((__ldcg(cum + (size_t)cx * cw + (cy >> 6)) >> (63 - (cy & 63))) & 1ull)
                                  << 1);
           s_paircov[pr] = cv;
@@ -811,7 +812,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(cy - roi, fwc, fbc);
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = s_N + (size_t)(pi * nr + prow) * nb2;
-        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
+        if (iv && r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((nrow[j] >> (63 - (cy & 63))) & 1ull))
             atomicOr(reinterpret_cast<unsigned *>(s_paircov + (pr & ~3)), 1u << (8 * (pr & 3)));
@@ -884,7 +885,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
         const unsigned rowm = masked ? s_nmask[pi * nr + prow] : 0xffu;
-        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
+        if (iv && r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((rowm >> j) & 1u) &&
               ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
@@ -940,7 +941,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
         const unsigned rowm = masked ? s_nmask[pi * nr + prow] : 0xffu;
-        if (a.intervis && r == roi) {  // own cell: newly covered by the pick?
+        if (iv && r == roi) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((rowm >> j) & 1u) &&
               ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
@@ -985,7 +986,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         shed_align(cy - roi, fwc, fbc);
         shed_align(py - roi, fwp, fbp);
         const uint64_t *nrow = a.nbits + (size_t)(pi * nr + prow) * nb2;
-        if (a.intervis && r == roi && ch == 0) {  // own cell: newly covered by the pick?
+        if (iv && r == roi && ch == 0) {  // own cell: newly covered by the pick?
           const int j = (cy >> 6) - fwp;
           if (j >= 0 && j < nb2 && ((__ldcg(nrow + j) >> (63 - (cy & 63))) & 1ull))
             atomicOr(reinterpret_cast<unsigned *>(s_paircov + (pr & ~3)), 1u << (8 * (pr & 3)));
@@ -1019,7 +1020,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---- E. intervis: where would a newly covered candidate overtake? --------
     if (tid == 0) s_roundcut = m;
     __syncthreads();
-    for (int u = a.intervis ? tid : npair; u < npair; u += blockDim.x) {
+    for (int u = iv ? tid : npair; u < npair; u += blockDim.x) {
       const int i = s_plist[u];
       const int j = div_by(i, s_rpcap);
       const int s = s_pairslot[i];
@@ -1069,7 +1070,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (cut < m) atomicMin(&s_roundcut, cut);
     }
     __syncthreads();
-    if (tid == 0 && a.intervis) {
+    if (tid == 0 && iv) {
       if (s_roundcut < m) atomicMax(a.cuts + par, kMaxPicks + 1 - s_roundcut);
       if (k == 0) __stcg(a.cuts + (par ^ 1), 0);  // read by all before this round's first barrier
     }
@@ -1079,8 +1080,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     // coverage is read only before the spread barrier: the coverage update
     // may start at once.  (The buffers reused by the next round are written
     // only after its first barrier, which every CTA reaches after this one.)
-    if ((a.intervis || !dist) && !group_sync(gb, a.err, &s_flagv)) return;
-    const int latest = a.intervis ? __ldcg(a.cuts + par) : 0;  // of the smallest cut of any CTA
+    if ((iv || !dist) && !group_sync(gb, a.err, &s_flagv)) return;
+    const int latest = iv ? __ldcg(a.cuts + par) : 0;  // of the smallest cut of any CTA
     const int mcut = latest ? kMaxPicks + 1 - latest : m;
     mark(7);
 
@@ -1144,7 +1145,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int g = s_gain[s] - s_dacc[s];
         s_gain[s] = g;
         s_dacc[s] = 0;
-        const bool inel = a.intervis && !(tag & 6);
+        const bool inel = iv && !(tag & 6);
         s_area[s] = inel ? 0 : g;
         s_flag[s] = (unsigned char)((s_flag[s] & ~kInel) | (inel ? kInel : 0));
         s_dirty[s >> 5] = 1;
