@@ -205,10 +205,9 @@ int siting_last_site_phase_cycles(siting_ctx *ctx, long long *cycles, int n);
  * the reference: it is for callers that cannot allocate device memory on
  * their call path (a serving loop that reserves its HBM budget at start-up,
  * or an application whose memory pool already owns the device's memory).
- * Scratch comes from a 48 MiB array in the library's device image, held by
+ * Scratch comes from a 16 MiB array in the library's device image, held by
  * every GPU that loads the library until the process exits; a job whose
- * coverage bitmap, new-bit rows and pick lists (as of a selection in the global
- * key order) take more than 16 MiB returns SITING_ENOMEM, and invalid arguments return
+ * scratch would exceed it returns SITING_ENOMEM, and invalid arguments return
  * SITING_EINVAL (an observer index outside the DEM is found before SITE
  * reads through it).  Runs on `stream` (a cudaStream_t, NULL = default
  * stream) of the current device, synchronises that stream twice and returns
@@ -256,7 +255,8 @@ int siting_run_batch_dev(siting_ctx *ctx, int njobs, const siting_params *params
                          const siting_plan *plans);
 
 /* Device workspace siting_run_batch would take for these jobs (no device
- * work; plans may be NULL).  No counterpart in the reference. */
+ * work; plans may be NULL); in less, down to that of selections in the global
+ * order alone, it runs without local dominance.  No counterpart in the reference. */
 int siting_batch_workspace_bytes(siting_ctx *ctx, int njobs,
                                  const siting_params *params,
                                  const siting_plan *plans, size_t *bytes);

@@ -94,6 +94,19 @@ int ws_get(siting_ctx *ctx, Slot s, size_t bytes, void **out) {
   return SITING_OK;
 }
 
+int site_scratch_get(siting_ctx *ctx, int nrows, int nsheds, int nctas, int roi, int intervis,
+                     int *local, void **base, SiteScratch *s) {
+  int rc = ws_get(ctx, kSite, site_scratch_bytes(nrows, nsheds, nctas, roi, intervis, *local), base);
+  if (rc == SITING_ENOMEM && *local) {
+    *local = 0;
+    rc = ws_get(ctx, kSite, site_scratch_bytes(nrows, nsheds, nctas, roi, intervis, false), base);
+    if (rc == SITING_OK) ctx->err.clear();
+  }
+  if (rc) return rc;
+  site_carve_scratch(*base, nrows, nsheds, nctas, roi, intervis, *local, s);
+  return SITING_OK;
+}
+
 bool geometry_of(int nrows, int bw, int nwanted0, siting_geometry *g) {
   // siting.cpp:689-695
   const float bs = (float)nrows / (int)((float)nrows / bw + 0.5f);
@@ -247,13 +260,11 @@ int site_enqueue(siting_ctx *ctx, int nrows, int roi, int intervis, int nsheds,
   if (site_smem_bytes(roi, nsheds, G, nb, npb, bs) > 220 * 1024)
     return fail(ctx, SITING_EINVAL, "SITE: shared-memory plan exceeds 220 KB");
   void *p;
-  const int local = ctx->site_order == kOrderLocal ? 2 * site_may_be_local(roi)
-                    : ctx->site_order == kOrderAuto && site_is_local(nrows, nsheds, roi, intervis, nb);
-  const size_t sb = site_scratch_bytes(nrows, nsheds, G, roi, intervis, local);
-  int rc = ws_get(ctx, kSite, sb, &p);
-  if (rc) return rc;
+  int local = ctx->site_order == kOrderLocal ? 2 * site_may_be_local(roi)
+              : ctx->site_order == kOrderAuto && site_is_local(nrows, nsheds, roi, intervis, nb);
   SiteScratch s;
-  site_carve_scratch(p, nrows, nsheds, G, roi, intervis, local, &s);
+  int rc = site_scratch_get(ctx, nrows, nsheds, G, roi, intervis, &local, &p, &s);
+  if (rc) return rc;
   // zero coverage, slots, barrier and outputs (order is written before read)
   CK(cudaMemsetAsync(p, 0, (unsigned char *)s.order - (unsigned char *)p, ctx->stream));
   CK(cudaMemsetAsync(d_selected, 0, nsheds, ctx->stream));

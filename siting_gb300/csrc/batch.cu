@@ -34,8 +34,8 @@ size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 // 48.8, 46.0, 45.4; 20 of 500^2 to 2000^2, dense 51.4, 47.7, 50.2; 24 of 512^2 to 2048^2
 // 43.7, 37.3, 37.3; 24 of 300^2 to 900^2 11.0, 11.0, 10.2; 12 of 256^2 to 2200^2 23.5,
 // 21.3, 22.5).
-int batch_site_ctas(int nsheds, int sm_count) {
-  const int g = std::max(1, (nsheds + 2047) / 2048);
+int batch_site_ctas(int nsheds, int sm_count, bool lean) {
+  const int each = lean ? 4096 : 2048, g = std::max(1, (nsheds + each - 1) / each);
   return std::min(std::min(g, std::max(1, nsheds)), sm_count);
 }
 
@@ -53,7 +53,7 @@ namespace siting {
 // Launch plan and workspace layout of a batch: pure host arithmetic (no
 // device work), so that admission control can size a batch before running it.
 int plan_batch(int sm_count, int njobs, const siting_params *params, const siting_plan *plans,
-               BatchPlan *bp, std::string *err) {
+               bool lean, BatchPlan *bp, std::string *err) {
   auto bad = [&](int j, const std::string &m) {
     *err = "job " + std::to_string(j) + ": " + m;
     return SITING_EINVAL;
@@ -82,7 +82,7 @@ int plan_batch(int sm_count, int njobs, const siting_params *params, const sitin
     J.vp = vix_plan_for(grid_rows, J.p.roi, J.p.ntests, pl ? pl->vix_tile : 0, pl ? pl->vix_smem : -1);
     J.sp = shed_plan_for(J.p.roi, pl ? pl->shed_smem : -1);
     J.G = (pl && pl->site_ctas > 0) ? std::min(pl->site_ctas, sm_count)
-                                     : batch_site_ctas(J.g.nwanted, sm_count);
+                                     : batch_site_ctas(J.g.nwanted, sm_count, lean);
     if (!site_supported(J.p.roi, J.g.nwanted, J.G)) return bad(j, "beyond the SITE kernel's limits");
     J.auto_G = !(pl && pl->site_ctas > 0);
     if (!site_fits(J, J.G)) return bad(j, "SITE shared-memory plan too large");
@@ -155,7 +155,7 @@ int plan_batch(int sm_count, int njobs, const siting_params *params, const sitin
     J.o_tab = tab_bytes;
     tab_bytes += align256(vix_table_bytes(J.p.roi, J.p.ntests));
     J.o_site = ws;
-    J.local = site_is_local(J.n, J.g.nwanted, J.p.roi, J.p.intervis, J.g.nblocks);
+    J.local = !lean && site_is_local(J.n, J.g.nwanted, J.p.roi, J.p.intervis, J.g.nblocks);
     ws += align256(site_scratch_bytes(J.n, J.g.nwanted, J.G, J.p.roi, J.p.intervis, J.local));
     J.o_err = ws;
     ws += 256;
@@ -206,19 +206,28 @@ int run_batch(siting_ctx *ctx, int njobs, const siting_params *params,
   }
   BatchPlan plan;
   std::string perr;
-  if (int prc = plan_batch(ctx->sm_count, njobs, params, plans, &plan, &perr))
+  if (int prc = plan_batch(ctx->sm_count, njobs, params, plans, false, &plan, &perr))
     return fail(ctx, prc, perr);
+  void *base_v;
+  bool lean = false;
+  int rc = ws_get(ctx, kBatch, plan.ws, &base_v);
+  if (rc == SITING_ENOMEM) {  // beyond the budget or the device's free memory
+    lean = true;
+    plan = BatchPlan();
+    if (int prc = plan_batch(ctx->sm_count, njobs, params, plans, lean, &plan, &perr))
+      return fail(ctx, prc, perr);
+    rc = ws_get(ctx, kBatch, plan.ws, &base_v);
+  }
+  if (rc) return rc;
+  if (lean) ctx->err.clear();
   std::vector<Job> &jobs = plan.jobs;
   const auto &waves = plan.waves;
   const auto &wave_ctas = plan.wave_ctas;
   const auto &o_wtab = plan.o_wtab;
-  const size_t ws = plan.ws, tab_bytes = plan.tab_bytes, wtab_bytes = plan.wtab_bytes;
+  const size_t tab_bytes = plan.tab_bytes, wtab_bytes = plan.wtab_bytes;
   const size_t o_tabs = plan.o_tabs, o_wtabs = plan.o_wtabs;
   (void)wave_ctas;
 
-  void *base_v;
-  int rc = ws_get(ctx, kBatch, ws, &base_v);
-  if (rc) return rc;
   unsigned char *base = static_cast<unsigned char *>(base_v);
   // pinned staging: VIX tables, wave job tables, then per-job readback
   const size_t s_tabs = 0, s_wtabs = align256(tab_bytes);
@@ -282,6 +291,7 @@ int run_batch(siting_ctx *ctx, int njobs, const siting_params *params,
       put(&pl, sizeof(pl));
     }
     put(&base, sizeof(base));
+    put(&lean, sizeof(lean));
     put(&ctx->batch_mode, sizeof(ctx->batch_mode));
   }
   unsigned char *stage;
@@ -494,7 +504,7 @@ int siting_batch_workspace_bytes(siting_ctx *ctx, int njobs, const siting_params
     return fail(ctx, SITING_EINVAL, "batch_workspace_bytes: null argument");
   BatchPlan plan;
   std::string perr;
-  if (int rc = plan_batch(ctx->sm_count, njobs, params, plans, &plan, &perr))
+  if (int rc = plan_batch(ctx->sm_count, njobs, params, plans, false, &plan, &perr))
     return fail(ctx, rc, perr);
   *bytes = plan.ws;
   return SITING_OK;

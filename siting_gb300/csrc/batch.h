@@ -37,9 +37,11 @@ struct BatchPlan {
 };
 
 // Plans a batch for a device of sm_count SMs: host arithmetic only, safe to
-// call from any thread.  SITING_EINVAL and a message for an invalid job.
+// call from any thread.  SITING_EINVAL and a message for an invalid job.  `lean`: the
+// smallest workspace (every SITE in the global order, by the fewest CTAs), for a memory
+// budget that the usual plan exceeds.
 int plan_batch(int sm_count, int njobs, const siting_params *params, const siting_plan *plans,
-               BatchPlan *bp, std::string *err);
+               bool lean, BatchPlan *bp, std::string *err);
 
 // Drops the context's captured batch graph (its workspace may be gone).
 void batch_graph_reset(siting_ctx *ctx);

@@ -68,6 +68,10 @@ int fail(siting_ctx *ctx, int code, const std::string &msg);
 int cuda_fail(siting_ctx *ctx, cudaError_t e, const char *what);
 // Grows workspace slot `s` to at least `bytes` (contents not preserved).
 int ws_get(siting_ctx *ctx, Slot s, size_t bytes, void **out);
+// The scratch of a SITE job from the context's workspace.  *local: as in SiteJob; 0 on
+// return where the scratch of local dominance is beyond the budget.
+int site_scratch_get(siting_ctx *ctx, int nrows, int nsheds, int nctas, int roi, int intervis,
+                     int *local, void **base, SiteScratch *s);
 // Pinned host staging of at least `bytes`.
 int stage_get(siting_ctx *ctx, size_t bytes, unsigned char **out);
 bool geometry_of(int nrows, int bw, int nwanted0, siting_geometry *g);

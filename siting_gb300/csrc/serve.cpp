@@ -497,7 +497,12 @@ int siting_server_submit(siting_server *s, const siting_params *p, const uint16_
   // (planning is host-only)
   BatchPlan plan;
   std::string e;
-  const int rc = plan_batch(s->ctx->sm_count, 1, p, serve_plan(s->ctx->sm_count, p), &plan, &e);
+  const siting_plan *sp = serve_plan(s->ctx->sm_count, p);
+  int rc = plan_batch(s->ctx->sm_count, 1, p, sp, false, &plan, &e);
+  if (!rc && plan.ws > s->budget) {
+    plan = BatchPlan();
+    rc = plan_batch(s->ctx->sm_count, 1, p, sp, true, &plan, &e);
+  }
   std::lock_guard<std::mutex> g(s->mu);
   const size_t pin = rc ? 0 : pin_layout(plan).total;
   if (rc || plan.ws > s->budget || pin > s->h_size) {

@@ -1622,10 +1622,9 @@ cudaError_t launch_site(int nrows, int roi, int intervis, int nsheds, const int3
 // it and must be serialised by the caller.
 namespace {
 
-// Jobs are admitted by the scratch that a selection in the global order takes (16 MiB at
-// most); site_local takes up to 36 bytes a candidate and 12 MiB more.
-constexpr size_t kNoAllocLimit = size_t(16) << 20;
-constexpr size_t kNoAllocScratchBytes = size_t(48) << 20;  // per device
+// A selection by local dominance takes up to 36 bytes a candidate and 12 MiB more than
+// one in the global order: where that is too much, the global order takes the job.
+constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;  // 16 MiB per device
 
 }  // namespace
 
@@ -1673,11 +1672,12 @@ extern "C" int siting_site_it_noalloc(int nrows, int roi, int intervis, int nshe
   // candidates are taken in any order: one block row holding them all
   const float bs = (float)nrows;
   if (site_smem_bytes(roi, nsheds, G, 1, nsheds, bs) > 220 * 1024) return SITING_EINVAL;
-  if (scratch_layout(nrows, nsheds, G, roi, 1, false, nullptr, nullptr) + 256 > kNoAllocLimit)
-    return SITING_ENOMEM;
-  const bool local = site_is_local(nrows, nsheds, roi, intervis, 1);
-  const size_t need = site_scratch_bytes(nrows, nsheds, G, roi, intervis, local) + 256;  // + error flag
-  if (need > kNoAllocScratchBytes) return SITING_ENOMEM;
+  auto need_of = [&](bool local) {  // + error flag
+    return site_scratch_bytes(nrows, nsheds, G, roi, intervis, local) + 256;
+  };
+  const bool local = site_is_local(nrows, nsheds, roi, intervis, 1) && need_of(true) <= kNoAllocScratchBytes;
+  const size_t need = need_of(local);
+  if (need > kNoAllocScratchBytes) return SITING_ENOMEM;  // beyond the 16 MiB array
   void *base = nullptr;
   int rc = noalloc_scratch(&base);
   if (rc) return rc;

@@ -132,7 +132,6 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
   if (n == N && g.nwanted > 0) {
     const int gmin = (g.nwanted + 4095) / 4096;
     const int gdef = site_default_ctas(g.nwanted, ctx->sm_count);
-    const bool local = site_is_local(n, g.nwanted, p->roi, p->intervis, g.nblocks);
     std::vector<int> cands = {gdef, std::max(gmin, gdef / 2), std::max(gmin, gdef / 4)};
     std::sort(cands.begin(), cands.end());
     cands.erase(std::unique(cands.begin(), cands.end()), cands.end());
@@ -143,10 +142,9 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
               220 * 1024)
         continue;
       void *sp;
-      const size_t sb = site_scratch_bytes(n, g.nwanted, G, p->roi, p->intervis, local);
-      if ((rc = ws_get(ctx, kSite, sb, &sp))) return rc;
+      int local = site_is_local(n, g.nwanted, p->roi, p->intervis, g.nblocks);
       SiteScratch s;
-      site_carve_scratch(sp, n, g.nwanted, G, p->roi, p->intervis, local, &s);
+      if ((rc = site_scratch_get(ctx, n, g.nwanted, G, p->roi, p->intervis, &local, &sp, &s))) return rc;
       float t;
       rc = time_ms(ctx, [&] {
         cudaError_t e = cudaMemsetAsync(sp, 0, (unsigned char *)s.order - (unsigned char *)sp, st);
