@@ -144,6 +144,13 @@ __device__ __forceinline__ int elevation(const uint16_t *dem, int at) {
   }
 }
 
+// A table entry that the compiler cannot fold; ordered with the stores and barriers before.
+__device__ __forceinline__ float ld_shared_f32(uint32_t at) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+
 constexpr float kNoHorizon = -99999.f;
 
 // The steps k..k1 of a pair of rays: A and B are mirror images about the
@@ -397,8 +404,7 @@ __global__ void __launch_bounds__(448, 2)
     r.nalt = f2_pack(nalt, nalt);
     // A product times 1 plus a sum keeps the product's own rounding: ptxas 13.0
     // contracts mul.rn.f32x2 into an add.rn.f32x2 that it feeds.
-    float one;
-    asm("ld.shared.f32 %0, [%1];" : "=f"(one) : "r"(smem_u32(tab + 1)));  // RN(1/1)
+    const float one = ld_shared_f32(smem_u32(tab + 1));  // RN(1/1)
     r.one = f2_pack(one, one);
     r.img = smem_u32(img + ((kHalves == 2 && half ? 2 : 0) + (xm ? 0 : 1)) * ximg);
     r.near = smem_u32(near + ((kHalves == 2 && half ? 2 : 0) + (xm ? 0 : 1)) * 2 * near_map(kNearSteps));
@@ -576,8 +582,7 @@ __global__ void __cluster_dims__(2) __launch_bounds__(kQuadMaxThreads, 2)
         r.sl = sl;
         const float nalt = -i2f(elevation<true>(a.dem, p0) + a.oht), tht = i2f(a.tht);
         r.nalt = f2_pack(nalt, nalt);
-        float one;
-        asm("ld.shared.f32 %0, [%1];" : "=f"(one) : "r"(smem_u32(tab + 1)));  // RN(1/1)
+        const float one = ld_shared_f32(smem_u32(tab + 1));  // RN(1/1)
         r.one = f2_pack(one, one);
         r.img = smem_u32(img);
         r.near = smem_u32(near);
