@@ -691,7 +691,8 @@ ShedPlan shed_staged_plan(int roi, bool half) {
       (roi + 1 + 31) / 32 * 32 <= kQuadMaxThreads && quad_smem_bytes(roi, kNearSteps) <= kMaxSmem;
   if (roi >= kQuadMinRoi && quad_smem_bytes(roi, kNearSteps) <= kTwoCtaSmem)
     return shed_quad_plan(roi);
-  if (pair_smem_bytes(roi, 1, true) <= kMaxSmem)
+  // a thread for every pair, as a staged CTA sweeps one each
+  if (2 * roi + 1 <= kPairMaxThreads && pair_smem_bytes(roi, 1, true) <= kMaxSmem)
     return ShedPlan{pair_threads(2 * roi + 1), true, true, false};
   return quad_fits ? shed_quad_plan(roi) : shed_l1_plan(roi);
 }
