@@ -323,7 +323,9 @@ __device__ __forceinline__ void near_bits(const unsigned char *map, int line, un
   }
 }
 
-template <int kHalves, bool kStaged, bool kRcp>
+// kSmall: a CTA of one warp for a small radius (kSmallMinRoi), whose pairs are a few more
+// than its lanes.  It takes the straight y-major pair a lane a step and loops over the rest.
+template <int kHalves, bool kStaged, bool kRcp, bool kSmall = false>
 __global__ void __launch_bounds__(448, 2)
     shed_kernel(const __grid_constant__ CUtensorMap map, const ShedArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
@@ -371,7 +373,8 @@ __global__ void __launch_bounds__(448, 2)
 
   // ---- rays: roi+1 x-major pairs and then the y-major ones of each side; the
   // straight y-major ray (minor offset 0) belongs to the upper side
-  const int up = 2 * roi + 1, npairs = kHalves == 2 ? 4 * roi + 1 : half0 ? 2 * roi : up;
+  constexpr int kStraight = kSmall ? 0 : 1;
+  const int up = 2 * roi + kStraight, npairs = kHalves == 2 ? 4 * roi + kStraight : half0 ? 2 * roi : up;
   // (a staged CTA has a thread for every pair: as a loop over pairs, the compiler
   // lets a warp's rays part at their ends, 15% more instructions)
   for (int t0 = tid; t0 < npairs; t0 += blockDim.x) {
@@ -381,8 +384,9 @@ __global__ void __launch_bounds__(448, 2)
     // adjacent lanes take every second ray of their group: half as many meet in
     // one image word (2048^2, roi 100: 1.018 -> 0.980 ms; every third 0.992, as the
     // lengths of a warp's rays then differ more)
-    const int mt = xm ? t : t - (roi + 1), evens = ((xm ? roi + 1 : roi - half) + 1) / 2;
-    const int m = (mt < evens ? 2 * mt : 2 * (mt - evens) + 1) + (xm ? 0 : half);
+    const int first = kSmall ? 1 : half;  // the least minor offset of the y-major rays
+    const int mt = xm ? t : t - (roi + 1), evens = ((xm ? roi + 1 : roi - first) + 1) / 2;
+    const int m = (mt < evens ? 2 * mt : 2 * (mt - evens) + 1) + (xm ? 0 : first);
     const int rowlim = half ? n - 1 - ox : ox;  // rows on this side of the observer
     const int collimA = n - 1 - oy, collimB = oy;
     const float sl = kRcp ? step_slope(tab[roi], m) : fdiv(i2f(m), i2f(roi));
@@ -413,7 +417,27 @@ __global__ void __launch_bounds__(448, 2)
     r.hs = f2_pack(kNoHorizon, kNoHorizon);
     r.tht = f2_pack(tht, tht);
     pair_sweep<kStaged, kRcp, kNearSteps>(r, kA, kB);
-    if (kStaged) break;
+    if (kStaged && !kSmall) break;
+  }
+  if constexpr (kSmall) {
+    // the observer's row: lanes 0..15 the steps to the right, 16..31 to the left, the
+    // horizon a running maximum over the lanes
+    const int side = lane >> 4, k = (lane & 15) + 1;
+    const bool on = k <= min(roi, side ? oy : n - 1 - oy);
+    const int p0 = (int)win + (ox - hx0) * W2 + 2 * (oy - hy0);
+    const float e = i2f(elevation<true>(a.dem, on ? p0 + (side ? -2 : 2) * k : p0));
+    const float nalt = -i2f(elevation<true>(a.dem, p0) + a.oht);
+    const float4 t = tab[min(k, roi)];
+    const float d = fadd(e, nalt), q = fmul(d, t.x);
+    float hs = on ? __fmaf_rn(__fmaf_rn(q, t.z, d), t.x, q) : kNoHorizon;
+    hs = fmaxf(hs, kNoHorizon);
+    for (int o = 1; o < 16; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, hs, o, 16);
+      if ((lane & 15) >= o) hs = fmaxf(hs, v);
+    }
+    // elev + tht >= oalt + hs*k, as in pair_group
+    if (on && fadd(e, i2f(a.tht)) >= -fadd(fmul(hs, t.z), nalt))
+      near[(2 + side) * near_map(kNearSteps) + k - 1] = 1;
   }
   __syncthreads();
 
@@ -450,7 +474,7 @@ __global__ void __launch_bounds__(448, 2)
   // A thread keeps one word column q, so that its string positions are fixed.
   const int S = 64 * nwpr - 1 - roi;
   auto by_nwpr = [&](int t) { return (int)((unsigned)t * a.rw >> 16); };
-  const int per = by_nwpr(blockDim.x);  // rows a pass (blockDim >= 64 > nwpr)
+  const int per = by_nwpr(blockDim.x);  // rows a pass (blockDim > nwpr)
   const int tr = by_nwpr(tid), q = tid - tr * nwpr, z = 2 * (nwpr - 1 - q);  // bits 32z..32z+63
   const int l0 = 32 * z - (S + 1), r0 = S - 1 - 32 * z - 31;
   const int li = l0 >> 5, ri = r0 >> 5, lsh = l0 & 31, rsh = r0 & 31;
@@ -675,6 +699,13 @@ ShedPlan shed_quad_plan(int roi) {
   return ShedPlan{(roi + 1 + 31) / 32 * 32, true, false, true};
 }
 
+// Radii whose whole windows have more pairs of rays than a warp has lanes, by so few that
+// most of a second warp idles, and the observers from which one warp that loops is faster
+// (2048^2, 102 400 observers, ms with a thread a ray, a thread a pair, and so: radius 8
+// 0.154, 0.222, 0.144; 10 0.205, 0.222, 0.196; 12 0.226, 0.247, 0.209; 15 0.332, 0.247,
+// 0.222; 4096 observers of radius 12 16, 17, 17 us, 1024 9, 9, 11).
+constexpr int kSmallMinRoi = 8, kSmallMaxRoi = 15, kSmallMinObs = 4096;
+
 // The staged form of a radius.  The SM holds few CTAs of a large window, so the
 // window shrinks with the radius (ms at 2048^2, 1.6 G cells of rays; whole, half,
 // quarter): roi 30 0.454, 0.484; 60 1.016, 1.021, 1.233; 70 1.018, 1.056, 1.240;
@@ -749,13 +780,17 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
     const WinGeom g = eff.quad ? quad_geom(roi) : win_geom(roi, eff.half ? 1 : 2, true);
     if (!make_dem_tensor_map(&map, dem, g.w, g.box_rows)) return cudaErrorInvalidValue;
   }
+  const bool small = eff.use_smem && !eff.quad && !eff.half && roi >= kSmallMinRoi &&
+                     roi <= kSmallMaxRoi && (roi == kSmallMinRoi || nsheds >= kSmallMinObs);
   auto kern = !eff.use_smem ? (rcp ? shed_kernel<1, false, true> : shed_kernel<1, false, false>)
               : eff.quad    ? (quad_near(roi) == kNearSteps ? shed_quad_kernel<kNearSteps>
                                                             : shed_quad_kernel<kFarNearSteps>)
               : eff.half    ? shed_kernel<1, true, true>
+              : small       ? shed_kernel<2, true, true, true>
                             : shed_kernel<2, true, true>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
   if (e != cudaSuccess) return e;
+  const int threads = small ? 32 : eff.threads;
   int grid = nsheds * (eff.half ? 2 : 1);
   if (eff.quad) {
     // One CTA an SM has nothing to run while a window arrives: there a cluster takes up
@@ -768,7 +803,7 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
     if (shm > kTwoCtaSmem) a.chunk = std::max(1, std::min(4, a.items / (8 * std::max(1, sms / 2))));
     grid = 2 * ceil_div(a.items, a.chunk);
   }
-  kern<<<grid, eff.threads, shm, st>>>(map, a);
+  kern<<<grid, threads, shm, st>>>(map, a);
   return cudaGetLastError();
 }
 
