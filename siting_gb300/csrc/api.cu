@@ -94,6 +94,10 @@ int ws_get(siting_ctx *ctx, Slot s, size_t bytes, void **out) {
   return SITING_OK;
 }
 
+int dem_pitch(const siting_ctx *ctx, int nrows, int roi, int nsheds) {
+  return ctx->budget ? (nrows + 7) & ~7 : shed_dem_pitch(nrows, roi, nsheds, ctx->sm_count);
+}
+
 int site_scratch_get(siting_ctx *ctx, int nrows, int nsheds, int nctas, int roi, int intervis,
                      int *local, void **base, SiteScratch *s) {
   int rc = ws_get(ctx, kSite, site_scratch_bytes(nrows, nsheds, nctas, roi, intervis, *local), base);
@@ -173,15 +177,15 @@ int check_device(siting_ctx *ctx) {
 }
 
 // Prepares a DemView for a device DEM with pitch n; if its layout cannot be
-// tiled by TMA (row bytes not a multiple of 16, or unaligned base), copies it
+// tiled by TMA (row bytes not a multiple of 16, or unaligned base), or a VIEWSHED of that
+// radius and so many observers wants another pitch (shed_dem_pitch), copies it
 // into the context's pitched DEM buffer.
-int dem_view(siting_ctx *ctx, const uint16_t *d_elevs, int nrows, DemView *v) {
-  const bool aligned = (nrows % 8 == 0) && ((uintptr_t)d_elevs % 16 == 0);
-  if (aligned) {
+int dem_view(siting_ctx *ctx, const uint16_t *d_elevs, int nrows, int roi, int nsheds, DemView *v) {
+  const int pitch = dem_pitch(ctx, nrows, roi, nsheds);
+  if (pitch == nrows && (uintptr_t)d_elevs % 16 == 0) {
     *v = DemView{d_elevs, nrows, nrows, true};
     return SITING_OK;
   }
-  const int pitch = (nrows + 7) & ~7;
   void *p;
   int rc = ws_get(ctx, kDem, (size_t)pitch * nrows * 2, &p);
   if (rc) return rc;
@@ -473,7 +477,7 @@ int siting_calc_vix_dev(siting_ctx *ctx, int nrows, const uint16_t *d_elevs, int
   if (rc) return rc;
   CK(cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
   DemView dem;
-  if ((rc = dem_view(ctx, d_elevs, nrows, &dem))) return rc;
+  if ((rc = dem_view(ctx, d_elevs, nrows, 0, 0, &dem))) return rc;
   return vix_dev(ctx, dem, roi, oht, tht, ntests, d_vix, d_err);
 }
 
@@ -499,7 +503,7 @@ int siting_calc_sheds_dev(siting_ctx *ctx, int nrows, const uint16_t *d_elevs, i
   if (rc) return rc;
   CK(cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
   DemView dem;
-  if ((rc = dem_view(ctx, d_elevs, nrows, &dem))) return rc;
+  if ((rc = dem_view(ctx, d_elevs, nrows, roi, nsheds, &dem))) return rc;
   return sheds_dev(ctx, dem, roi, oht, tht, nsheds, d_obs, d_sheds, d_err);
 }
 
@@ -582,10 +586,10 @@ int siting_calc_sheds(siting_ctx *ctx, int nrows, const uint16_t *elevs, int roi
   if (!obs_in_range(obs, nsheds, nrows))
     return fail(ctx, SITING_EINVAL, "calc_sheds: observer index outside the DEM");
   cudaSetDevice(ctx->device);
-  const int pitch = (nrows + 7) & ~7;
   const int nr = 2 * roi + 1, nwpr = (nr + 63) / 64;
   const size_t shed_bytes = (size_t)nsheds * nr * nwpr * 8;
   void *d_dem, *d_obs, *d_sheds;
+  const int pitch = dem_pitch(ctx, nrows, roi, nsheds);
   int rc;
   if ((rc = ws_get(ctx, kDem, (size_t)pitch * nrows * 2, &d_dem))) return rc;
   if ((rc = ws_get(ctx, kObs, (size_t)std::max(nsheds, 1) * 4, &d_obs))) return rc;
@@ -704,7 +708,9 @@ int siting_run_dev(siting_ctx *ctx, const siting_params *p, const uint16_t *d_el
   if (validate(p, 1, &m)) return fail(ctx, SITING_EINVAL, m);
   cudaSetDevice(ctx->device);
   DemView dem;
-  int rc = dem_view(ctx, d_elevs, p->nrows, &dem);
+  siting_geometry g;
+  geometry_of(p->nrows, p->bw, p->nwanted0, &g);
+  int rc = dem_view(ctx, d_elevs, p->nrows, p->roi, g.nwanted, &dem);
   if (rc) return rc;
   return run_pipeline(ctx, p, dem, d_obs, d_selected, res);
 }
@@ -717,8 +723,9 @@ int siting_run(siting_ctx *ctx, const siting_params *p, const uint16_t *elevs, i
   cudaSetDevice(ctx->device);
   siting_geometry g;
   geometry_of(p->nrows, p->bw, p->nwanted0, &g);
-  const int n = p->nrows, pitch = (n + 7) & ~7;
+  const int n = p->nrows;
   void *d_dem, *d_obs, *d_sel;
+  const int pitch = dem_pitch(ctx, n, p->roi, g.nwanted);
   int rc;
   if ((rc = ws_get(ctx, kDem, (size_t)pitch * n * 2, &d_dem))) return rc;
   if ((rc = ws_get(ctx, kObs, (size_t)g.nwanted * 4, &d_obs))) return rc;

@@ -73,7 +73,7 @@ int plan_batch(int sm_count, int njobs, const siting_params *params, const sitin
     if (validate(&J.p, 1, &m)) return bad(j, m);
     geometry_of(J.p.nrows, J.p.bw, J.p.nwanted0, &J.g);
     J.n = J.p.nrows;
-    J.pitch = (J.n + 7) & ~7;
+    J.pitch = lean ? (J.n + 7) & ~7 : shed_dem_pitch(J.n, J.p.roi, J.g.nwanted, sm_count);
     J.nr = 2 * J.p.roi + 1;
     J.nwpr = (J.nr + 63) / 64;
     J.per = (size_t)J.nr * J.nwpr;
@@ -319,7 +319,7 @@ int run_batch(siting_ctx *ctx, int njobs, const siting_params *params,
   for (int j = 0; j < njobs; j++) {  // inputs, VIX tables, zeroed scratch
     Job &J = jobs[j];
     const size_t sp = (size_t)(src_pitch && src_pitch[j] ? src_pitch[j] : J.n) * 2;
-    if (host_io || J.n % 8 || (uintptr_t)elevs[j] % 16 || sp != (size_t)J.n * 2)
+    if (host_io || J.pitch != J.n || (uintptr_t)elevs[j] % 16 || sp != (size_t)J.n * 2)
       CK(cudaMemcpy2DAsync(base + J.o_dem, (size_t)J.pitch * 2, elevs[j], sp, (size_t)J.n * 2, J.n,
                            host_io ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
     vix_fill_tables(stage + s_tabs + J.o_tab, J.p.roi, J.p.ntests);
@@ -334,7 +334,7 @@ int run_batch(siting_ctx *ctx, int njobs, const siting_params *params,
   CK(cudaEventRecordWithFlags(ctx->ev[0], st, rec_flags));
   auto dem_of = [&](int j) {
     const Job &J = jobs[j];
-    const bool own = host_io || J.n % 8 || (uintptr_t)elevs[j] % 16 ||
+    const bool own = host_io || J.pitch != J.n || (uintptr_t)elevs[j] % 16 ||
                      (src_pitch && src_pitch[j] && src_pitch[j] != J.n);
     return own ? DemView{reinterpret_cast<const uint16_t *>(base + J.o_dem), J.n, J.pitch, true}
                : DemView{elevs[j], J.n, J.n, true};

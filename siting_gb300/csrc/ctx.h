@@ -72,6 +72,9 @@ int ws_get(siting_ctx *ctx, Slot s, size_t bytes, void **out);
 // return where the scratch of local dominance is beyond the budget.
 int site_scratch_get(siting_ctx *ctx, int nrows, int nsheds, int nctas, int roi, int intervis,
                      int *local, void **base, SiteScratch *s);
+// The row pitch of a copy of the DEM for a VIEWSHED of that radius and so many observers;
+// the least under a memory budget, which the rest of a job may need.
+int dem_pitch(const siting_ctx *ctx, int nrows, int roi, int nsheds);
 // Pinned host staging of at least `bytes`.
 int stage_get(siting_ctx *ctx, size_t bytes, unsigned char **out);
 bool geometry_of(int nrows, int bw, int nwanted0, siting_geometry *g);

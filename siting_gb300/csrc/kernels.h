@@ -63,10 +63,14 @@ struct ShedPlan {
   bool use_smem;  // stage the window by TMA
   bool half;      // two CTAs an observer, one for the rows on each side of it
   bool quad;      // four CTAs an observer, one for each quadrant
+  bool any;       // launch_sheds may read the window through L1 instead
 };
 ShedPlan shed_default_plan(int roi);
 ShedPlan shed_plan_for(int roi, int smem);
 size_t shed_smem_bytes(const ShedPlan &p, int roi);
+// The row pitch (elements) for a copy of the DEM: a multiple of 8 (TMA), and not of 32 for
+// a job whose windows the default plan then reads through L1.
+int shed_dem_pitch(int nrows, int roi, int nsheds, int sm_count);
 cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nsheds,
                          const int32_t *obs, uint64_t *sheds, const ShedPlan &plan, int *d_err,
                          cudaStream_t st);

@@ -693,10 +693,12 @@ int pair_threads(int pairs) {
   return ((pairs + rounds - 1) / rounds + 31) / 32 * 32;
 }
 
-ShedPlan shed_l1_plan(int roi) { return ShedPlan{pair_threads(2 * roi + 1), false, true, false}; }
+ShedPlan shed_l1_plan(int roi) {
+  return ShedPlan{pair_threads(2 * roi + 1), false, true, false, false};
+}
 
 ShedPlan shed_quad_plan(int roi) {
-  return ShedPlan{(roi + 1 + 31) / 32 * 32, true, false, true};
+  return ShedPlan{(roi + 1 + 31) / 32 * 32, true, false, true, false};
 }
 
 // Radii whose whole windows have more pairs of rays than a warp has lanes, by so few that
@@ -712,19 +714,19 @@ constexpr int kSmallMinRoi = 8, kSmallMaxRoi = 15, kSmallMinObs = 4096;
 // 90 1.018, 0.987, 0.945; 100 1.032, 0.981, 1.067; 118 -, 0.956, 0.957; 125 -,
 // 1.039, 0.904; 140 -, 1.056, 0.962; 200 -, 1.390, 1.138.  From roi 209 quarters
 // are one CTA an SM and halves are faster while they fit (212: 1.344, 1.744).
-constexpr int kHalfMinRoi = 75, kQuadMinRoi = 119;
+constexpr int kHalfMinRoi = 75, kQuadMinRoi = 119, kOneCtaMinRoi = 209, kOutsideMinRoi = 16;
 
 ShedPlan shed_staged_plan(int roi, bool half) {
   if (roi < 1) return shed_l1_plan(roi);
   if (!half && 4 * roi + 1 <= kPairMaxThreads && pair_smem_bytes(roi, 2, true) <= kMaxSmem)
-    return ShedPlan{pair_threads(4 * roi + 1), true, false, false};
+    return ShedPlan{pair_threads(4 * roi + 1), true, false, false, false};
   const bool quad_fits =
       (roi + 1 + 31) / 32 * 32 <= kQuadMaxThreads && quad_smem_bytes(roi, kNearSteps) <= kMaxSmem;
   if (roi >= kQuadMinRoi && quad_smem_bytes(roi, kNearSteps) <= kTwoCtaSmem)
     return shed_quad_plan(roi);
   // a thread for every pair, as a staged CTA sweeps one each
   if (2 * roi + 1 <= kPairMaxThreads && pair_smem_bytes(roi, 1, true) <= kMaxSmem)
-    return ShedPlan{pair_threads(2 * roi + 1), true, true, false};
+    return ShedPlan{pair_threads(2 * roi + 1), true, true, false, false};
   return quad_fits ? shed_quad_plan(roi) : shed_l1_plan(roi);
 }
 
@@ -748,7 +750,32 @@ size_t shed_smem_bytes(const ShedPlan &p, int roi) {
   return p.quad ? quad_smem_bytes(roi, quad_near(roi)) : pair_smem_bytes(roi, p.half ? 1 : 2, p.use_smem);
 }
 
-ShedPlan shed_default_plan(int roi) { return shed_staged_plan(roi, roi >= kHalfMinRoi); }
+ShedPlan shed_default_plan(int roi) {
+  ShedPlan p = shed_staged_plan(roi, roi >= kHalfMinRoi);
+  p.any = p.use_smem;
+  return p;
+}
+
+namespace {
+
+// Whether the default plan reads a job's windows through L1, where its DEM's row pitch
+// allows: staged CTAs of radius 209 and more are alone on their SM, 7 to 14 warps whose
+// starts and ends nothing overlaps, and a window that lies mostly outside the DEM is staged
+// and cleared for short rays.  Few observers do not fill the SMs: quarters are more CTAs.
+// Ms of 4000 observers with one ray a thread through L1, staged, and so: radius 216, 432^2
+// 1.23, 1.79, 1.15; 1296^2 1.48, 1.80, 1.23; 260, 1560^2 2.41, 2.53, 1.72; 200, 240^2 0.92,
+// 1.01, 0.86; 60, 72^2 0.20, 0.20, 0.11.
+bool shed_prefers_l1(int n, int roi, int nsheds, int sms) {
+  return nsheds >= sms && (roi >= kOneCtaMinRoi || (roi >= kOutsideMinRoi && 4 * n <= 5 * roi));
+}
+
+}  // namespace
+
+int shed_dem_pitch(int nrows, int roi, int nsheds, int sm_count) {
+  const int pitch = (nrows + 7) & ~7;
+  return pitch % 32 == 0 && nrows < 7 * roi && shed_prefers_l1(nrows, roi, nsheds, sm_count) ? pitch + 8
+                                                                                          : pitch;
+}
 
 // smem: 1 half windows staged, 2 the whole window staged (as 1 where it does
 // not fit), 0 the window read through L1 (as 1 and 2 are where half a window
@@ -772,7 +799,14 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
   // the reciprocal-table division is exhaustively checked for |a| <= 2^21
   // (heights up to 10^6 over 16-bit elevations) and steps up to 2048
   const bool rcp = oht >= 0 && oht <= 1000000;
-  const ShedPlan eff = plan.use_smem && !(rcp && dem.tma_ok) ? shed_l1_plan(roi) : plan;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // a pitch of whole cache lines puts a column's cells at one place of their lines, and
+  // lanes on one column then leave theirs together (2048^2, radius 225, 3000 observers:
+  // 1.75 ms at a pitch of 2048, 0.98 at 2056)
+  const bool l1 = plan.any && dem.pitch % 64 && shed_prefers_l1(dem.nrows, roi, nsheds, sms);
+  const ShedPlan eff = l1 || (plan.use_smem && !(rcp && dem.tma_ok)) ? shed_l1_plan(roi) : plan;
   const size_t shm = shed_smem_bytes(eff, roi);
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
@@ -797,9 +831,6 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
     // to 4 halves in turn and asks for the next window when the rays of one are done (roi
     // 216 1.69 -> 1.63 ms, 240 1.56 -> 1.46, 300 1.46 -> 1.37), in 8 or more rounds of
     // clusters.  With two CTAs an SM their ends overlap anyhow (200: 1.08, 1.15).
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (shm > kTwoCtaSmem) a.chunk = std::max(1, std::min(4, a.items / (8 * std::max(1, sms / 2))));
     grid = 2 * ceil_div(a.items, a.chunk);
   }

@@ -60,3 +60,48 @@ def test_quarters_of_two_boxes(native, oracle, roi):
             if plan >= 0:
                 ctx.autotune_set(roi, 1, native.Plan(0, -1, plan, 0))
             assert np.array_equal(ctx.calc_sheds(n, dem, roi, 40, 8, obs), want), f"plan {plan}"
+
+
+@pytest.mark.parametrize("n, roi, count", [(128, 110, 400), (128, 100, 400), (448, 216, 400), (512, 209, 151),
+                                           (512, 209, 152), (384, 240, 400), (200, 180, 400), (20, 16, 300)])
+def test_windows_through_l1_and_the_pitch_of_the_dem(native, oracle, n, roi, count):
+    """Large radii and rasters smaller than a window: through L1 from one observer an SM on,
+    from a copy of the DEM where its rows are whole cache lines; without one in a budget."""
+    dem = native.fbm_dem(n, seed=n + roi, octaves=6, range_max=20000)
+    obs = np.random.default_rng(n).integers(0, n * n, count).astype(np.int32)
+    want = oracle.sheds(dem, n, roi, 30, 10, obs)
+    for budget in (0, 1 << 30):
+        with native.Context(0, hbm_budget=budget) as ctx:
+            assert np.array_equal(ctx.calc_sheds(n, dem, roi, 30, 10, obs), want)
+            got = _sheds_dev(native, ctx, n, dem, roi, 30, 10, obs)
+            assert np.array_equal(got.ravel(), want)
+
+
+def test_jobs_whose_dem_is_copied(native, oracle):
+    torch = pytest.importorskip("torch")
+    job = dict(nrows=320, roi=212, height=40, ntests=8, bw=16, nwanted0=400, intervis=1)
+    dem = native.fbm_dem(320, seed=2, octaves=7, range_max=20000)
+    ref = oracle.run(dem, *(job[k] for k in ("nrows", "roi", "height", "ntests", "bw", "nwanted0", "intervis")))
+    p = native.Params(**job)
+    d_dem = torch.from_numpy(dem.view(np.int16)).cuda()
+    d_obs = [torch.empty(len(ref["obs"]), dtype=torch.int32, device="cuda") for _ in range(2)]
+    d_sel = [torch.empty(len(ref["obs"]), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+
+    def same(obs, sel, res):
+        assert np.array_equal(obs, ref["obs"]) and np.array_equal(sel, ref["selected"])
+        assert (res.nusedsheds, res.cumarea) == (ref["nused"], ref["cumarea"])
+
+    with native.Context(0) as ctx:
+        same(*ctx.run(p, dem))
+        res = ctx.run_dev(p, d_dem, d_obs[0], d_sel[0])
+        same(d_obs[0].cpu().numpy(), d_sel[0].cpu().numpy(), res)
+        for got in ctx.run_batch([p, p], [dem, dem]):
+            same(*got)
+        for _ in range(2):  # captured, then replayed
+            rs = ctx.run_batch_dev([p, p], [d_dem, d_dem], d_obs, d_sel)
+            for o, s, res in zip(d_obs, d_sel, rs):
+                same(o.cpu().numpy(), s.cpu().numpy(), res)
+    with native.Server(0) as srv:
+        obs, sel, info = srv.wait(srv.submit(p, dem))
+        same(obs, sel, info.result)
