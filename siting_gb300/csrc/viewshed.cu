@@ -697,6 +697,12 @@ ShedPlan shed_l1_plan(int roi) {
   return ShedPlan{pair_threads(2 * roi + 1), false, true, false, false};
 }
 
+// Halves where they fit, with a thread for every pair, as a staged CTA sweeps one each.
+ShedPlan shed_half_plan(int roi) {
+  if (2 * roi + 1 > kPairMaxThreads || pair_smem_bytes(roi, 1, true) > kMaxSmem) return shed_l1_plan(roi);
+  return ShedPlan{pair_threads(2 * roi + 1), true, true, false, false};
+}
+
 ShedPlan shed_quad_plan(int roi) {
   return ShedPlan{(roi + 1 + 31) / 32 * 32, true, false, true, false};
 }
@@ -724,10 +730,8 @@ ShedPlan shed_staged_plan(int roi, bool half) {
       (roi + 1 + 31) / 32 * 32 <= kQuadMaxThreads && quad_smem_bytes(roi, kNearSteps) <= kMaxSmem;
   if (roi >= kQuadMinRoi && quad_smem_bytes(roi, kNearSteps) <= kTwoCtaSmem)
     return shed_quad_plan(roi);
-  // a thread for every pair, as a staged CTA sweeps one each
-  if (2 * roi + 1 <= kPairMaxThreads && pair_smem_bytes(roi, 1, true) <= kMaxSmem)
-    return ShedPlan{pair_threads(2 * roi + 1), true, true, false, false};
-  return quad_fits ? shed_quad_plan(roi) : shed_l1_plan(roi);
+  const ShedPlan half_plan = shed_half_plan(roi);
+  return half_plan.use_smem || !quad_fits ? half_plan : shed_quad_plan(roi);
 }
 
 }  // namespace
@@ -806,7 +810,8 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
   // lanes on one column then leave theirs together (2048^2, radius 225, 3000 observers:
   // 1.75 ms at a pitch of 2048, 0.98 at 2056)
   const bool l1 = plan.any && dem.pitch % 64 && shed_prefers_l1(dem.nrows, roi, nsheds, sms);
-  const ShedPlan eff = l1 || (plan.use_smem && !(rcp && dem.tma_ok)) ? shed_l1_plan(roi) : plan;
+  ShedPlan eff = l1 || (plan.use_smem && !dem.tma_ok) ? shed_l1_plan(roi) : plan;
+  if (eff.quad && !rcp) eff = shed_half_plan(roi);  // quarters have no build that divides
   const size_t shm = shed_smem_bytes(eff, roi);
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
@@ -814,14 +819,15 @@ cudaError_t launch_sheds(const DemView &dem, int roi, int oht, int tht, int nshe
     const WinGeom g = eff.quad ? quad_geom(roi) : win_geom(roi, eff.half ? 1 : 2, true);
     if (!make_dem_tensor_map(&map, dem, g.w, g.box_rows)) return cudaErrorInvalidValue;
   }
-  const bool small = eff.use_smem && !eff.quad && !eff.half && roi >= kSmallMinRoi &&
+  const bool small = rcp && eff.use_smem && !eff.quad && !eff.half && roi >= kSmallMinRoi &&
                      roi <= kSmallMaxRoi && (roi == kSmallMinRoi || nsheds >= kSmallMinObs);
   auto kern = !eff.use_smem ? (rcp ? shed_kernel<1, false, true> : shed_kernel<1, false, false>)
               : eff.quad    ? (quad_near(roi) == kNearSteps ? shed_quad_kernel<kNearSteps>
                                                             : shed_quad_kernel<kFarNearSteps>)
-              : eff.half    ? shed_kernel<1, true, true>
+              : eff.half    ? (rcp ? shed_kernel<1, true, true> : shed_kernel<1, true, false>)
               : small       ? shed_kernel<2, true, true, true>
-                            : shed_kernel<2, true, true>;
+              : rcp         ? shed_kernel<2, true, true>
+                            : shed_kernel<2, true, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
   if (e != cudaSuccess) return e;
   const int threads = small ? 32 : eff.threads;

@@ -105,3 +105,19 @@ def test_jobs_whose_dem_is_copied(native, oracle):
     with native.Server(0) as srv:
         obs, sel, info = srv.wait(srv.submit(p, dem))
         same(obs, sel, info.result)
+
+
+@pytest.mark.parametrize("roi", [7, 12, 80, 130, 215, 216, 320])
+@pytest.mark.parametrize("oht, tht", [(-3, 5), (1500000, 0)])
+def test_heights_that_divide_in_every_form(native, oracle, roi, oht, tht):
+    """Observer heights outside 0..10^6 divide: whole and half windows, and through L1."""
+    n = 2 * roi + 45
+    dem = native.fbm_dem(n, seed=roi, octaves=7, range_max=60000)
+    obs = np.random.default_rng(roi).integers(0, n * n, 160).astype(np.int32)
+    want = oracle.sheds(dem, n, roi, oht, tht, obs)
+    with native.Context(0) as ctx:
+        for plan in (-1, 1, 2, 0):
+            ctx.autotune_clear()
+            if plan >= 0:
+                ctx.autotune_set(roi, 1, native.Plan(0, -1, plan, 0))
+            assert np.array_equal(ctx.calc_sheds(n, dem, roi, oht, tht, obs), want), f"plan {plan}"
