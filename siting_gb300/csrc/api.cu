@@ -226,8 +226,9 @@ int vix_dev(siting_ctx *ctx, const DemView &dem, int roi, int oht, int tht, int 
     ctx->tab_ntests = ntests;
   }
   const siting_plan *tp = tuned_plan(ctx, roi, ntests);
-  const VixPlan plan = tp ? vix_plan_for(dem.nrows, roi, ntests, tp->vix_tile, tp->vix_smem)
-                          : vix_default_plan(dem.nrows, roi, ntests);
+  const VixPlan plan = tp ? vix_plan_for(dem.nrows, roi, ntests, tp->vix_tile, tp->vix_smem,
+                                       ctx->sm_count)
+                          : vix_default_plan(dem.nrows, roi, ntests, ctx->sm_count);
   CK(launch_vix(dem, roi, oht, tht, ntests, d_vix, tab, plan, d_err, ctx->stream));
   return SITING_OK;
 }

@@ -79,7 +79,8 @@ int plan_batch(int sm_count, int njobs, const siting_params *params, const sitin
     J.per = (size_t)J.nr * J.nwpr;
     const siting_plan *pl = plans ? &plans[j] : nullptr;
     const int grid_rows = shared_grid ? (int)std::min(std::sqrt(cells), 20000.0) : J.n;
-    J.vp = vix_plan_for(grid_rows, J.p.roi, J.p.ntests, pl ? pl->vix_tile : 0, pl ? pl->vix_smem : -1);
+    J.vp = vix_plan_for(grid_rows, J.p.roi, J.p.ntests, pl ? pl->vix_tile : 0, pl ? pl->vix_smem : -1,
+                        sm_count);
     J.sp = shed_plan_for(J.p.roi, pl ? pl->shed_smem : -1);
     J.G = (pl && pl->site_ctas > 0) ? std::min(pl->site_ctas, sm_count)
                                      : batch_site_ctas(J.g.nwanted, sm_count, lean);

@@ -35,15 +35,16 @@ struct VixPlan {
   int tile;       // cells per tile side
   int threads;    // threads per CTA
   bool use_smem;  // stage the whole halo by TMA (else the cells within 64 of the tile)
+  bool bare;      // else not even these: the tile alone
 };
 // Device tables of the VIX stage (host-computed with the reference's
 // expressions): jump[2k], jump[2k+1] = LCG multiplier/increment of k+1 steps
 // for k < 2*ntests; rtab[d] = (float)(1.0/d); vtab[v] = VIX byte of v hits.
 size_t vix_table_bytes(int roi, int ntests);
 void vix_fill_tables(void *host_buf, int roi, int ntests);
-VixPlan vix_default_plan(int nrows, int roi, int ntests);
+VixPlan vix_default_plan(int nrows, int roi, int ntests, int sm_count);
 // A caller's plan (tile 16/32/64, smem 1/0/-1), corrected to one that fits.
-VixPlan vix_plan_for(int nrows, int roi, int ntests, int tile, int smem);
+VixPlan vix_plan_for(int nrows, int roi, int ntests, int tile, int smem, int sm_count);
 size_t vix_smem_bytes(const VixPlan &p, int roi, int ntests);
 cudaError_t launch_vix(const DemView &dem, int roi, int oht, int tht, int ntests,
                        uint8_t *vix, const void *d_tables, const VixPlan &plan, int *d_err,

@@ -83,7 +83,7 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
   float bt = 1e30f;
   for (int tile : {16, 32, 64})
     for (int sm : {1, 0}) {
-      const VixPlan vp = vix_plan_for(n, p->roi, p->ntests, tile, sm);
+      const VixPlan vp = vix_plan_for(n, p->roi, p->ntests, tile, sm, ctx->sm_count);
       if (std::any_of(seen.begin(), seen.end(), [&](const VixPlan &q) {
             return q.tile == vp.tile && q.use_smem == vp.use_smem;
           }))
@@ -103,7 +103,8 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
     }
   // observers of the sample for the VIEWSHED trials
   CK(launch_vix(dem, p->roi, p->oht, p->tht, p->ntests, static_cast<uint8_t *>(d_vix), tab,
-                vix_plan_for(n, p->roi, p->ntests, out.vix_tile, out.vix_smem), err, st));
+                vix_plan_for(n, p->roi, p->ntests, out.vix_tile, out.vix_smem, ctx->sm_count), err,
+                st));
   CK(launch_findmax(static_cast<uint8_t *>(d_vix), n, g.blocksize, g.nblocks, g.nwantedperblock,
                     static_cast<int32_t *>(d_obs), st));
   bt = 1e30f;

@@ -41,6 +41,9 @@ namespace {
 // Staged samples of the far form.
 constexpr int kFarNear = 7;
 
+// The whole halo staged, the cells near the tile, or the tile alone.
+constexpr int kStagedForm = 0, kFarForm = 1, kBareForm = 2, kForms = 3;
+
 struct VixArgs {
   const uint16_t *dem;
   int pitch, n, roi, oht, tht, ntests;
@@ -86,6 +89,9 @@ struct VixArgs {
       : "=f"(over)                                                                  \
       : "r"(ad), "f"(slope), "f"(zslope), "f"(foz), "f"(0x1.fffffep-2f), "r"(ob2), \
         "r"(smaj), "r"(smin))
+#define VIX_S1 VIX_SAMPLE("d0", "1", "0f3F800000")
+#define VIX_S3                                                                        \
+  VIX_S1 VIX_SAMPLE("d1", "2", "0f40000000") VIX_MAX VIX_SAMPLE("d0", "4", "0f40800000")
 #define VIX_S5                                                                        \
   VIX_SAMPLE("d0", "1", "0f3F800000") VIX_SAMPLE("d1", "2", "0f40000000") VIX_MAX       \
   VIX_SAMPLE("d0", "4", "0f40800000") VIX_SAMPLE("d1", "8", "0f41000000") VIX_MAX       \
@@ -98,6 +104,8 @@ template <int kNear>
 __device__ __forceinline__ int near_samples(int ad, float slope, float zslope, float foz,
                                             uint32_t ob2, int smaj, int smin) {
   float over;
+  if constexpr (kNear == 1) VIX_SAMPLES(VIX_S1);
+  if constexpr (kNear == 3) VIX_SAMPLES(VIX_S3);
   if constexpr (kNear == 5) VIX_SAMPLES(VIX_S5);
   if constexpr (kNear == 6) VIX_SAMPLES(VIX_S6);
   if constexpr (kNear == 7) VIX_SAMPLES(VIX_S7);
@@ -174,7 +182,8 @@ __device__ __forceinline__ int vix_target(const VixArgs &a, const VixCell &c, in
   const float slope = fmul(i2f(am), r), zslope = fmul(i2f(ev + c.ctz), r);
   // every staged sample is tested: a blocked target's lane would idle until
   // its warp's other lanes finish anyway
-  const int vis = near_samples<kNear>(ad, slope, zslope, c.foz, c.ob2, smaj, smin);
+  int vis = 1;
+  if constexpr (kNear > 0) vis = near_samples<kNear>(ad, slope, zslope, c.foz, c.ob2, smaj, smin);
   if constexpr (kFar) {
     if (ad > (1 << kNear) && vis) {
       const int P = a.pitch;
@@ -237,7 +246,7 @@ __device__ __forceinline__ void vix_tile_work(const VixArgs &a, const uint16_t *
 // tile's index (row-major over tiles_per_row^2), `sm` the CTA's dynamic
 // shared memory (vix_smem_bytes), `mbar` the window's mbarrier (shared
 // memory).  Every thread of the CTA calls it.
-template <bool kFar>
+template <int kForm>
 __device__ __forceinline__ void vix_tile(const CUtensorMap *map, const VixArgs &a, int tile,
                                          unsigned char *sm, uint64_t *mbar) {
   const int T = a.tile;
@@ -277,15 +286,22 @@ __device__ __forceinline__ void vix_tile(const CUtensorMap *map, const VixArgs &
   }
   auto work = [&](auto near) {
     constexpr int kNear = decltype(near)::value;
+    constexpr bool kFar = kForm != kStagedForm;
     if (interior)
       vix_tile_work<kNear, kFar, true>(a, halo, tx0, ty0, hx0, hy0, jump, rtab, vtab);
     else
       vix_tile_work<kNear, kFar, false>(a, halo, tx0, ty0, hx0, hy0, jump, rtab, vtab);
   };
-  if constexpr (kFar) {
+  if constexpr (kForm == kBareForm) {
+    work(std::integral_constant<int, 0>());
+  } else if constexpr (kForm == kFarForm) {
     work(std::integral_constant<int, kFarNear>());
   } else {  // the fewest samples that reach offsets below roi
-    if (a.roi <= 32)
+    if (a.roi <= 2)
+      work(std::integral_constant<int, 1>());
+    else if (a.roi <= 8)
+      work(std::integral_constant<int, 3>());
+    else if (a.roi <= 32)
       work(std::integral_constant<int, 5>());
     else if (a.roi <= 64)
       work(std::integral_constant<int, 6>());
@@ -296,12 +312,12 @@ __device__ __forceinline__ void vix_tile(const CUtensorMap *map, const VixArgs &
   }
 }
 
-template <bool kFar>
+template <int kForm>
 __global__ void __launch_bounds__(1024, 2) vix_kernel(const __grid_constant__ CUtensorMap map,
                                                      const VixArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
   const uint32_t halo_bytes = (uint32_t)a.nboxes * a.box_rows * a.halo_w * 2u;
-  vix_tile<kFar>(&map, a, blockIdx.x, sm, reinterpret_cast<uint64_t *>(sm + halo_bytes));
+  vix_tile<kForm>(&map, a, blockIdx.x, sm, reinterpret_cast<uint64_t *>(sm + halo_bytes));
 }
 
 // ---- VIX of many jobs in one launch (batched form) ---------------------------
@@ -323,10 +339,9 @@ struct VixQTable {
 };
 static_assert(sizeof(VixQTable) <= 32000, "kernel parameters are limited to 32 KB");
 
-// One CTA per (job, tile) item.  kFar: every job of the launch reads its far
-// targets through L1 (else none does): one kernel per form keeps each within
+// One CTA per (job, tile) item, all of one form: one kernel per form keeps each within
 // 32 registers a thread.
-template <bool kFar>
+template <int kForm>
 __global__ void __launch_bounds__(1024, 2) vixq_kernel(const __grid_constant__ VixQTable tab) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ __align__(8) uint64_t mbar;
@@ -340,7 +355,7 @@ __global__ void __launch_bounds__(1024, 2) vixq_kernel(const __grid_constant__ V
       hi = mid - 1;
   }
   const VixQJob &J = tab.jobs[lo];
-  vix_tile<kFar>(&J.map, J.a, (int)(it - J.first), sm, &mbar);
+  vix_tile<kForm>(&J.map, J.a, (int)(it - J.first), sm, &mbar);
 }
 
 int round8(int v) { return (v + 7) & ~7; }
@@ -348,6 +363,10 @@ int round8(int v) { return (v + 7) & ~7; }
 // Samples of the near window of the far form: offsets 1..64, so the window
 // reaches kFarHalo cells around the tile.
 constexpr int kFarHalo = 1 << (kFarNear - 1);
+// Targets a cell up to which not even that window pays: the tile alone is staged (us at
+// radius 120, 1 and 2 targets: 1000^2 26.7 and 30.8 with
+// the window, 20.8 and 26.8 without).
+constexpr int kBareTests = 2;
 
 // Two 1024-thread CTAs share an SM when each takes at most half of its 228 KB
 // shared memory (at most 32 registers a thread); the second CTA fills the
@@ -365,7 +384,9 @@ size_t tables_tail_bytes(int roi, int ntests) {
   return 16 + (size_t)ntests * 8 + (size_t)(roi + 1) * 4 + ntests + 1;
 }
 
-int plan_halo(const VixPlan &p, int roi) { return p.use_smem ? roi : kFarHalo; }
+int vix_form(const VixPlan &p) { return p.use_smem ? kStagedForm : p.bare ? kBareForm : kFarForm; }
+
+int plan_halo(const VixPlan &p, int roi) { return p.use_smem ? roi : p.bare ? 0 : kFarHalo; }
 
 // The window of a tile: its columns start at a multiple of 8 at or before the
 // halo's first (tiles start at multiples of 16).
@@ -421,23 +442,27 @@ size_t vix_smem_bytes(const VixPlan &p, int roi, int ntests) {
 // longer to load for a quarter of the cells: 2048^2, roi 96, staged 16x16 takes
 // 0.32 ms + 12.2 us a target, 32x32 with the near window alone 0.04 ms + 16.1
 // us, so few targets take the far form.  64x64 tiles (four cells a thread)
-// never won.  A grid of 32x32 tiles that is not two waves of the 152 SMs' CTA
+// never won.  A grid of 32x32 tiles that is not two waves of the SMs' CTA
 // pairs leaves SMs idle: 16x16 tiles then (us at 32 and 16, 256^2 roi 20: 23,
-// 15; 400^2 roi 200: 100, 69; 700^2 roi 200: 198, 176; 1000^2 roi 50: 187, 207).
-VixPlan vix_default_plan(int nrows, int roi, int ntests) {
+// 15; 400^2 roi 200: 100, 69; 700^2 roi 200: 198, 176; 1000^2 roi 50: 187, 207),
+// unless the targets are so few that four threads a cell and four halos for one cost
+// more, an eighth of the tiles (roi 45: 300^2, 8 targets 14.6, 16.8, 16 18.6, 19.7, 32
+// 27.3, 26.0; 700^2, 16 46.9, 57.1, 32 77.6, 79.6, 64 142, 128).
+VixPlan vix_default_plan(int nrows, int roi, int ntests, int sm_count) {
   const int t32 = (nrows + 31) / 32;
-  const bool few = t32 * t32 < 4 * 152;
-  const VixPlan s32{32, 1024, true}, s16{16, 1024, true};
+  const bool few = t32 * t32 < 4 * sm_count && 8 * ntests >= t32 * t32;
+  const VixPlan s32{32, 1024, true, false}, s16{16, 1024, true, false};
   if (!few && vix_smem_bytes(s32, roi, ntests) <= kVixTwoCtaSmem) return s32;
   if ((few || ntests >= 72) && vix_smem_bytes(s16, roi, ntests) <= kVixTwoCtaSmem) return s16;
-  return VixPlan{few ? 16 : 32, 1024, false};
+  return VixPlan{few ? 16 : 32, 1024, false, ntests <= kBareTests};
 }
 
-VixPlan vix_plan_for(int nrows, int roi, int ntests, int tile, int smem) {
-  VixPlan p = vix_default_plan(nrows, roi, ntests);
+VixPlan vix_plan_for(int nrows, int roi, int ntests, int tile, int smem, int sm_count) {
+  VixPlan p = vix_default_plan(nrows, roi, ntests, sm_count);
   if (tile == 16 || tile == 32 || tile == 64) {
     p.tile = tile;
     p.use_smem = smem != 0;
+    p.bare = false;
     if (p.use_smem &&
         (halo_geom(p, roi, ntests).w > 2048 || vix_smem_bytes(p, roi, ntests) > kVixMaxSmem))
       p.use_smem = false;
@@ -489,7 +514,10 @@ cudaError_t launch_vix(const DemView &dem, int roi, int oht, int tht, int ntests
     return cudaErrorInvalidValue;
   const size_t shm = vix_smem_bytes(plan, roi, ntests);
   const int grid = a.tiles_per_row * a.tiles_per_row;
-  auto kern = plan.use_smem ? vix_kernel<false> : vix_kernel<true>;
+  const int form = vix_form(plan);
+  auto kern = form == kStagedForm ? vix_kernel<kStagedForm>
+              : form == kFarForm  ? vix_kernel<kFarForm>
+                                  : vix_kernel<kBareForm>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
   if (e != cudaSuccess) return e;
   kern<<<grid, plan.threads, shm, st>>>(map, a);
@@ -497,10 +525,9 @@ cudaError_t launch_vix(const DemView &dem, int roi, int oht, int tht, int ntests
 }
 
 cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st) {
-  // jobs whose halo is staged, then the far form's: one launch for
-  // each kind, at most kStageQueueMaxJobs jobs a launch
+  // one launch for the jobs of each form, at most kStageQueueMaxJobs jobs a launch
   static thread_local VixQTable tab;  // 20 KB: not on the host stack
-  for (int kind = 0; kind < 2; kind++) {
+  for (int kind = 0; kind < kForms; kind++) {
     int j = 0;
     while (j < njobs) {
       tab.njobs = 0;
@@ -510,7 +537,7 @@ cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st) {
         const StageJob &J = jobs[j];
         VixQJob &q = tab.jobs[tab.njobs];
         memset(&q, 0, sizeof(q));
-        if ((J.vplan.use_smem ? 0 : 1) != kind) continue;
+        if (vix_form(J.vplan) != kind) continue;
         if (!vix_args(J.dem, J.roi, J.oht, J.tht, J.ntests, J.vix, J.vix_tables, J.vplan, J.err,
                       &q.a, &q.map))
           return cudaErrorInvalidValue;
@@ -520,7 +547,9 @@ cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st) {
         tab.njobs++;
       }
       if (!tab.njobs) continue;
-      auto kern = kind == 0 ? vixq_kernel<false> : vixq_kernel<true>;
+      auto kern = kind == kStagedForm ? vixq_kernel<kStagedForm>
+                  : kind == kFarForm  ? vixq_kernel<kFarForm>
+                                      : vixq_kernel<kBareForm>;
       cudaError_t e =
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
       if (e != cudaSuccess) return e;
