@@ -1238,8 +1238,13 @@ long long site_stop_area(int nrows) {
 // against 1.3).
 // Observers in no block order (one block) cost the global order more, since every
 // candidate is a possible neighbour of a pick: there the line is 4096 candidates with 64 in a
-// circle (17 jobs up to 16 384: 0.62 of its time; 1500^2, radius 60, 8836: 3.1 ms against
-// 4.6; below it 1.2).
+// circle, 180 circles on the raster, and candidates in a fiftieth of the cells, a twentieth
+// from 400 circles on and any share from 1000.  Below 10 000 candidates a bin may be no larger
+// than the radius, as a round finds one pick in 4x4 bins.  Of 58 selections of 4096 to 16 384
+// candidates and at most 64 in a circle, the 47 within these lines took 0.43 of the global
+// order's time in the mean (500^2, radius 6, 9388: 5.2 ms against 21.6; the slowest 1.1
+// times), the others 1.17 (289^2, 7, 7045: 3.9 against 2.6; 375^2, 15, 5588: 1.5 against 1.1;
+// 1988^2, 7, 5027: 4.0 against 2.8).
 //
 // Radii beyond 992 are for the global order, whose items are 4 words of a row (rows taken
 // 32 words at a time by local dominance: 10500^2, radius 1000, 150 candidates 8.3 ms
@@ -1260,7 +1265,11 @@ double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblock
   }
   const double twentieth = 3.14159 * roi * roi / 20;
   if (nsheds >= 16384) return std::max(64.0, std::min(512.0, twentieth));
-  return nblocks <= 1 && nsheds >= 4096 ? 64 : 0;
+  const double n2 = (double)nrows * nrows, circles = n2 / (20 * twentieth);
+  const double share = circles >= 1000 ? 1 : circles >= 400 ? 20 : 50;
+  const bool spread = circles >= 180 && share * nsheds <= n2;
+  const bool fine = nsheds >= 10000 || local_bin_side(nrows, roi) <= roi;
+  return nblocks <= 1 && nsheds >= 4096 && spread && fine ? 64 : 0;
 }
 
 // The same as pairs of candidates in one bin, each counted twice: nsheds times the

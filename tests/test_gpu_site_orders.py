@@ -54,3 +54,26 @@ def test_an_unknown_order_is_refused(native):
         for how in (-1, 3):
             with pytest.raises(native.SitingError):
                 ctx.set_site_order(how)
+
+
+@pytest.mark.parametrize("n, roi, count, local", [
+    (460, 19, 4096, True), (460, 19, 4095, False), (451, 19, 4096, False), (452, 12, 10000, True),
+    (440, 12, 10000, False), (200, 3, 5000, True), (600, 3, 4500, True), (800, 3, 4500, False)])
+def test_the_line_for_observers_in_no_block_order(native, oracle, n, roi, count, local):
+    """Intervis, one block: 180 circles on the raster, the share of cells, the bins' size."""
+    side = int(np.ceil(np.sqrt(count)))
+    i = np.arange(count)
+    jitter = np.random.default_rng(n).random((2, count)) * 0.9
+    x = ((i // side + jitter[0]) * (n / side)).astype(int)  # one in each square of a grid
+    y = ((i % side + jitter[1]) * (n / side)).astype(int)
+    obs = (np.clip(x, 0, n - 1) * n + np.clip(y, 0, n - 1)).astype(np.int32)
+    dem = native.fbm_dem(n, seed=n, octaves=7, range_max=6000)
+    sheds = oracle.sheds(dem, n, roi, 20, 20, obs)
+    want, used, area, order = oracle.site(n, roi, 1, obs, sheds, want_order=True)
+    with native.Context(0) as ctx:
+        sel, res = ctx.site_it(n, roi, 1, obs, sheds)
+        assert np.array_equal(ctx.last_pick_order(count), order)
+        # the clock of the cut runs in the global order alone
+        assert (ctx.last_site_phase_cycles()[12] == 0) == local
+    assert np.array_equal(sel, want)
+    assert (res.nusedsheds, res.cumarea) == (used, area)
