@@ -77,3 +77,22 @@ def test_the_line_for_observers_in_no_block_order(native, oracle, n, roi, count,
         assert (ctx.last_site_phase_cycles()[12] == 0) == local
     assert np.array_equal(sel, want)
     assert (res.nusedsheds, res.cumarea) == (used, area)
+
+
+@pytest.mark.parametrize("n, roi, count, top", [(700, 3, 6000, 6000), (1600, 35, 4000, 9000), (330, 1, 20000, 1),
+                                                (900, 12, 9000, 3000), (520, 4, 1030, 6000)])
+@pytest.mark.parametrize("intervis", [0, 1])
+def test_the_order_of_many_picks(native, oracle, n, roi, count, top, intervis):
+    """More than 1024 picks are put in order by buckets: small and large areas, equal ones."""
+    dem = native.fbm_dem(n, seed=n, octaves=7, range_max=top)
+    obs = np.random.default_rng(n).integers(0, n * n, count).astype(np.int32)
+    sheds = oracle.sheds(dem, n, roi, 3, 3, obs)
+    want, used, area, order = oracle.site(n, roi, intervis, obs, sheds, want_order=True)
+    for ctas in (0, 5):
+        with native.Context(0) as ctx:
+            ctx.set_site_ctas(ctas)
+            ctx.set_site_order(2)
+            sel, res = ctx.site_it(n, roi, intervis, obs, sheds)
+            assert np.array_equal(ctx.last_pick_order(count), order), f"{ctas} CTAs"
+        assert np.array_equal(sel, want)
+        assert (res.nusedsheds, res.cumarea) == (used, area)
