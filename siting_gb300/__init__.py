@@ -534,11 +534,15 @@ class Server:
             raise SitingError(rc, f"siting_server_create(device={device}) failed: "
                                   f"{self._lib.siting_status_string(rc).decode()}")
         self.h = h
+        # buffers of the jobs not yet waited for: the worker reads and writes them, whether
+        # their tickets are kept or not
+        self._held = {}
 
     def close(self):
         if getattr(self, "h", None):
-            self._lib.siting_server_destroy(self.h)
+            self._lib.siting_server_destroy(self.h)  # after the jobs in flight
             self.h = None
+            self._held.clear()
 
     def __enter__(self):
         return self
@@ -570,6 +574,7 @@ class Server:
                                             obs.ctypes.data, sel.ctypes.data, C.byref(tid))
         if rc:
             raise SitingError(rc, f"submit refused: {self._lib.siting_status_string(rc).decode()}")
+        self._held[tid.value] = (dem, obs, sel)
         return Ticket(tid.value, p, obs, sel, dem)
 
     def wait(self, t: Ticket, timeout: float | None = None):
@@ -582,6 +587,7 @@ class Server:
             raise TimeoutError(f"job {t.id} not done within {timeout} s")
         if rc:
             raise SitingError(rc, f"wait({t.id}) failed")
+        self._held.pop(t.id, None)
         ji = JobInfo(info.status, Result.of(info.result), info.t_submit, info.t_start,
                      info.t_done, info.batch_id, info.batch_jobs, info.error.decode())
         if ji.status:
