@@ -49,21 +49,25 @@ def test_a_single_job(native, oracle, job):
 
 
 def test_a_batch_and_a_server(native, oracle):
-    dems, refs = _oracle_of(native, oracle, JOBS)
-    params = [native.Params(**j) for j in JOBS]
+    # the last job's SITE takes 1024 threads a CTA, in one launch with the others
+    jobs = JOBS + [dict(nrows=420, roi=130, height=60, ntests=8, bw=20, nwanted0=900, intervis=1)]
+    dems, refs = _oracle_of(native, oracle, jobs)
+    params = [native.Params(**j) for j in jobs]
     with native.Context(0) as ctx:
         usual = ctx.batch_workspace_bytes(params)
         one = ctx.batch_workspace_bytes(params[:1])
-    with native.Context(0, hbm_budget=usual - (1 << 20)) as ctx:
-        for _ in range(2):
-            for ref, got in zip(refs, ctx.run_batch(params, dems)):
-                _same(ref, *got)
-        assert ctx.workspace_bytes() < usual
-    with native.Server(0, hbm_budget=one - (1 << 20)) as srv:
-        tickets = [srv.submit(p, d) for p, d in zip(params, dems)]
-        for ref, t in zip(refs, tickets):
-            obs, sel, info = srv.wait(t)
-            _same(ref, obs, sel, info.result)
+    for budget in (0, usual - (1 << 20)):
+        with native.Context(0, hbm_budget=budget) as ctx:
+            for _ in range(2):
+                for ref, got in zip(refs, ctx.run_batch(params, dems)):
+                    _same(ref, *got)
+            assert budget == 0 or ctx.workspace_bytes() < usual
+    for budget in (1 << 30, one - (1 << 20)):
+        with native.Server(0, hbm_budget=budget) as srv:
+            tickets = [srv.submit(p, d) for p, d in zip(params[:3], dems)]
+            for ref, t in zip(refs, tickets):
+                obs, sel, info = srv.wait(t)
+                _same(ref, obs, sel, info.result)
 
 
 def test_noalloc_takes_what_does_not_fit_in_the_global_order(native, oracle):
