@@ -26,14 +26,6 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ float i2f(int v) { return __int2float_rn(v); }
 __device__ __forceinline__ int f2i(float v) { return __float2int_rz(v); }
-// (int)roundf(v), half away from zero, for |v| < 2^31: truncation of
-// v + copysign(pred(0.5), v), with pred(0.5) = 0.5 - 2^-25 the float just
-// below one half (the usual trunc-based round: adding 0.5 itself would round
-// 0.5 - 2^-25 up to 1).  Checked against roundf over every float in range.
-__device__ __forceinline__ int round_i(float v) {
-  const float h = __uint_as_float((__float_as_uint(v) & 0x80000000u) | 0x3effffffu);
-  return __float2int_rz(__fadd_rn(v, h));
-}
 
 // Packed FP32 pairs (low half, high half) for the f32x2 instructions of
 // sm_100 and later: each half is an IEEE round-to-nearest operation of its
@@ -76,10 +68,6 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
   unsigned long long d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
-}
-// copysign(pred(0.5), v): the addend of round_i for v's sign
-__device__ __forceinline__ float round_addend(float v) {
-  return __uint_as_float((__float_as_uint(v) & 0x80000000u) | 0x3effffffu);
 }
 
 // ---- memory-order helpers --------------------------------------------------

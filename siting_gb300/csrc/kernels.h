@@ -91,9 +91,8 @@ struct StageJob {
 };
 // Jobs per multi-job launch (the job table is the kernel's parameters).
 constexpr int kStageQueueMaxJobs = 64;
-// VIX of every tile of `jobs`: one grid over the (job, tile) items of the
-// jobs whose halo is staged and one over the others (more when a kind has
-// over kStageQueueMaxJobs jobs).
+// VIX of every tile of `jobs`: one grid over the (job, tile) items of the jobs of each
+// form of halo (more when a form has over kStageQueueMaxJobs jobs).
 cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st);
 // FINDMAX of every block of `jobs`: one grid over the (job, block) items.
 cudaError_t launch_findmax_queue(const StageJob *jobs, int njobs, cudaStream_t st);
@@ -123,11 +122,11 @@ struct LocalScratch {
 // Scratch layout of one SITE job (device, carved from one allocation).
 struct SiteScratch {
   uint64_t *cum;             // nrows * ceil(nrows/64) words, zeroed before launch
-  uint64_t *nbits;           // the round's new bits of each pick: [64][nr][nwpr+1] words
+  uint64_t *nbits;           // the round's new bits of each pick: [64, or local_cap][nr][nwpr+1] words
   unsigned char *nmask;      // [64][nr]: bit j set when word j of that new-bit row is nonzero
   unsigned long long *topk;  // [2][nctas][top-K] x {key, cell}: published top keys
   int *cuts;                 // [2]: the smallest cut of the round's prefix (intervis)
-  int *ncount;               // [2][64]: popcount of each pick's new bits (self-check)
+  int *ncount;               // [2][64]: popcount of each pick's new bits (self-check); zeroed
   unsigned *bar;             // group barrier counter, zeroed
   long long *out;            // [0] nused, [1] cumarea, [2] rounds, [3..15] phase cycles
   int32_t *order;            // nsheds: picks in order

@@ -54,9 +54,10 @@ namespace {
 
 // Threads a CTA: 512 allow 128 registers a thread and suit jobs with few
 // candidates per CTA and narrow sheds; 1024 (64 registers) keep more items
-// in flight for many candidates per CTA or wide sheds (measured, SITE ms at
-// 512 and 1024 threads: 4096^2/roi 100 7.41 vs 7.65; 16384^2/roi 200 51.5 vs
-// 42.7).
+// in flight for many candidates per CTA or wide sheds (SITE ms at 512 and 1024
+// threads.  By local dominance: 2048^2, roi 60, intervis 1.84, 2.19; 4096^2, roi 100 4.00,
+// 3.94; 16384^2, roi 200, without 32.2, 21.9.  In the global order: 256^2, roi 20 0.68,
+// 0.73; 1000^2, roi 150 1.62, 1.55; 1152^2, roi 61, 147 456 candidates 5.11, 4.60).
 int site_threads_for(int nslots, int roi) { return (nslots > 1024 || roi > 127) ? 1024 : 512; }
 constexpr int kMaxSlots = 4096;  // candidates owned by one CTA
 // Keys each CTA publishes per round.  Rounds end at distance conflicts and
@@ -1363,8 +1364,11 @@ void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, i
 
 // Up to one CTA per SM, about 100 candidates per CTA but at least 32 CTAs:
 // each round's work is spread widely, while mid-size jobs keep fewer CTAs in
-// their barriers (1000^2, 10 000 candidates: 1.79 ms at 96-100 CTAs against
-// 1.99 ms at 152; 256^2, 512 candidates: 0.34 ms at 32 CTAs, 0.43 ms at 5).
+// their barriers (ms in the global order, 256^2, 1024 candidates, at 16, 32, 48 and 100
+// CTAs: 0.78, 0.73, 0.69, 0.70; 1000^2, 10 000, at 64, 80, 120 and 152: 1.88, 1.83, 1.76,
+// 1.78).  Local dominance, whose work does not go by owner, takes the same CTAs (1000^2,
+// 10 000, at 64, 100 and 152: 0.52, 0.46, 0.44; 4096^2, 65 536, at 64, 100 and 152: 6.35,
+// 4.93, 3.99).
 // The merged top-K lists (G * kTopK keys) stay small enough to walk with one
 // warp.
 int site_default_ctas(int nsheds, int sm_count) {

@@ -92,8 +92,8 @@ __host__ __device__ __forceinline__ int local_cells(int n, int roi) {
 }
 // Whether a placed row of a window has a lane of a warp for each word (radius <= 992).
 __host__ __device__ __forceinline__ bool local_width(int roi) { return (2 * roi + 64) / 64 + 1 <= 32; }
-// Picks a round takes at most: while their new bits take at most 8 MB (4 MB of it
-// is 256 picks at radius 64), and 64 in any case.
+// Picks a round takes at most: 256 while their new bits take at most 8 MB (radius 227),
+// 128 while these do (radius 340), else 64.
 __host__ __device__ __forceinline__ int local_cap(int roi) {
   const size_t nr = 2 * (size_t)roi + 1, one = nr * ((nr + 63) / 64 + 1) * 8;
   return kLocalMaxPicks * one <= (size_t)8 << 20   ? kLocalMaxPicks

@@ -17,11 +17,11 @@
 // read through L1 by the same code.  Visible cells are marked in a shared-memory
 // image of the shed, which is then written to HBM with coalesced stores.
 //
-// Bound by instruction issue and shared-memory wavefronts alike (75% and 78% of
-// their peaks at roi 100).  2048^2, ms before (one ray a thread) and after: 65536
-// observers of roi 20 0.330, 0.318; roi 30 0.632, 0.454; roi 50 1.523, 1.144;
-// 45511 of roi 60 1.490, 1.016; 16384 of roi 100 1.240, 0.981; 7281 of roi 150
-// 1.314, 1.008; 4096 of roi 200 1.604, 1.138 (1.02-1.2 T ray steps/s).
+// Bound by instruction issue and shared-memory wavefronts alike (76% and 82% of
+// their peaks at roi 100).  2048^2, ms before (one ray a thread) and after: 102400
+// observers of roi 10 0.205, 0.195; roi 20 0.512, 0.451; roi 30 0.982, 0.646; 65536 of roi
+// 50 1.523, 1.070; 45511 of roi 60 1.490, 0.959; 16384 of roi 100 1.241, 0.934; 6400 of
+// roi 160 1.488, 0.999; 4096 of roi 200 1.604, 1.044; 2844 of roi 240 1.872, 1.431.
 //
 // Half windows: every ray to a target row tx <= ox stays in rows ox-roi..ox,
 // every other ray in rows ox..ox+roi, so the sides can be swept apart.  The
@@ -33,7 +33,8 @@
 // straight rays along it.
 //
 // Bit-exactness: separately rounded FP32 operations, IEEE division for the
-// slopes (of which the sign goes with the strides, as rounding is symmetric), round-half-away-from-zero for the minor coordinate.  The horizon
+// slopes (of which the sign goes with the strides, as rounding is symmetric),
+// round-half-away-from-zero for the minor coordinate.  The horizon
 // slope s = RN(a/k) (a an integer elevation difference, k the step) is
 // q0 = RN(a*y), s = RN(q0 + RN(a - k*q0)*y) with y = RN(1/k) from a per-CTA
 // table: one fused correction of a quotient within an ulp, given a correctly
@@ -508,8 +509,8 @@ __global__ void __launch_bounds__(448, 2)
 // that word to the right one.  A cluster takes `chunk` halves (2o + lower of observer o)
 // in turn.
 //
-// At radius 200 two CTAs (14 warps) fill an SM: 58% of issue slots, shared-memory
-// pipe 68%, a quarter of the warps' time at the barriers between the sweep and the rows
+// At radius 200 two CTAs (14 warps) fill an SM: 59% of issue slots, shared-memory
+// pipe 64%, a quarter of the warps' time at the barriers between the sweep and the rows
 // out.  Reading a group's elevations ahead of the marks before them does not help (1.14
 // -> 1.17 ms).
 __host__ __device__ __forceinline__ WinGeom quad_geom(int roi) {
