@@ -1218,14 +1218,14 @@ long long site_stop_area(int nrows) {
 }
 
 // Without intervis local dominance pays by the picks that a round finds, so the raster
-// has to hold many of a candidate's circles: 30, or 15 from 1024 candidates on.  Its
-// passes over all bins cost what a hundredth of the bins in candidates, and 128, are
-// worth.  560 jobs and calls of 32 to 16 000 candidates, radius 4 to 200: the lines take
-// 1.014 times the better order's time in the mean.  Ms in the global order and by local
-// dominance: 50 circles 351^2, radius 28, 225 candidates 0.62, 0.44; 25 circles 784^2,
-// 99, 1374 1.53, 1.46; 14 circles 920^2, 139, 1369 1.45, 1.60; 19 circles 1301^2, 170,
-// 399 1.76, 2.24; 200 bins a candidate 913^2, 17, 160 0.22, 0.31; 60 candidates 386^2, 7
-// 0.08, 0.21.
+// has to hold several of a candidate's circles: 30, 8 from 400 candidates on, 3 from 2048.
+// Its passes over all bins cost what a hundredth of the bins in candidates, and 128, are
+// worth.  820 jobs and calls of 32 to 20 000 candidates, radius 4 to 200: these lines take
+// 1.006 times the better order's time in the mean.  Ms in the global order and by local
+// dominance: 50 circles 351^2, radius 28, 225 candidates 0.62, 0.44; 10 circles 612^2, 107,
+// 1236 0.34, 0.29; 5 circles 736^2, 179, 4232 0.82, 0.90 and 686^2, 179, 7396 0.63, 0.59; 19
+// circles 1301^2, 170, 399 1.76, 2.24; 2 circles 485^2, 174, 1125 0.24, 0.30; 200 bins a
+// candidate 913^2, 17, 160 0.22, 0.31; 60 candidates 386^2, 7 0.08, 0.21.
 //
 // With intervis a round also searches for the
 // candidates that its picks would uncover (B2).  That pays where many regions are
@@ -1239,13 +1239,13 @@ long long site_stop_area(int nrows) {
 // against 1.3).
 // Observers in no block order (one block) cost the global order more, since every
 // candidate is a possible neighbour of a pick: there the line is 4096 candidates with 64 in a
-// circle, 180 circles on the raster, and candidates in a fiftieth of the cells, a twentieth
+// circle, 80 circles on the raster, and candidates in a fiftieth of the cells, a twentieth
 // from 400 circles on and any share from 1000.  Below 10 000 candidates a bin may be no larger
-// than the radius, as a round finds one pick in 4x4 bins.  Of 58 selections of 4096 to 16 384
-// candidates and at most 64 in a circle, the 47 within these lines took 0.43 of the global
-// order's time in the mean (500^2, radius 6, 9388: 5.2 ms against 21.6; the slowest 1.1
-// times), the others 1.17 (289^2, 7, 7045: 3.9 against 2.6; 375^2, 15, 5588: 1.5 against 1.1;
-// 1988^2, 7, 5027: 4.0 against 2.8).
+// than the radius, as a round finds one pick in 4x4 bins.  Of 97 selections of 4096 to 16 384
+// candidates and at most 64 in a circle, the 84 within these lines took 0.53 of the global
+// order's time in the mean (500^2, radius 6, 9388: 5.2 ms against 21.6; the slowest, 906^2,
+// 25, 4663, 3.0 against 1.9), the others 1.26 (289^2, 7, 7045: 3.9 against 2.6; 241^2, 10,
+// 4786: 1.9 against 1.0; 1988^2, 7, 5027: 4.0 against 2.8).
 //
 // Radii beyond 992 are for the global order, whose items are 4 words of a row (rows taken
 // 32 words at a time by local dominance: 10500^2, radius 1000, 150 candidates 8.3 ms
@@ -1262,20 +1262,25 @@ double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblock
   if (!intervis) {
     const double bins = (double)local_bins(nrows, roi) * local_bins(nrows, roi);
     if (nsheds < 128 || bins > 100.0 * nsheds) return 0;
-    return nsheds / (nsheds >= 1024 ? 15.0 : 30.0);
+    return nsheds / (nsheds >= 2048 ? 3.0 : nsheds >= 400 ? 8.0 : 30.0);
   }
   const double twentieth = 3.14159 * roi * roi / 20;
   if (nsheds >= 16384) return std::max(64.0, std::min(512.0, twentieth));
   const double n2 = (double)nrows * nrows, circles = n2 / (20 * twentieth);
   const double share = circles >= 1000 ? 1 : circles >= 400 ? 20 : 50;
-  const bool spread = circles >= 180 && share * nsheds <= n2;
+  const bool spread = circles >= 80 && share * nsheds <= n2;
   const bool fine = nsheds >= 10000 || local_bin_side(nrows, roi) <= roi;
   return nblocks <= 1 && nsheds >= 4096 && spread && fine ? 64 : 0;
 }
 
-// The same as pairs of candidates in one bin, each counted twice: nsheds times the
-// candidates that one shares its bin with in the mean.
-unsigned long long site_max_near(int nrows, int nsheds, int roi, double limit) {
+// The most pairs of candidates in one bin, each counted twice: nsheds times the candidates
+// that one shares its bin with in the mean.  Crowded is what has more in a circle than the
+// line allows, without intervis a twelfth of all, and half as many again as anywhere at
+// random (20 000 candidates about one place of 1000^2, radius 20, with a 25th, a 12th and a
+// 6th of all in a circle: 1.45, 1.31 and 1.39 ms against 2.31, 1.56 and 1.23).
+unsigned long long site_max_near(int nrows, int nsheds, int roi, int intervis, double limit) {
+  const double circle = 3.14159 * roi * roi / ((double)nrows * nrows) * nsheds;
+  limit = std::max(intervis ? limit : std::min(limit, nsheds / 12.0), 1.5 * circle);
   const double side = local_bin_side(nrows, roi);
   return (unsigned long long)(limit * nsheds * side * side / (3.14159 * roi * roi));
 }
@@ -1505,7 +1510,7 @@ SiteArgs make_site_args(const SiteJob &j, int block0) {
   a.local = j.scratch.local;
   a.use_local = j.local != 0;
   a.max_near = j.local == 2 ? kBeyond - 1
-                            : site_max_near(j.nrows, j.nsheds, j.roi,
+                            : site_max_near(j.nrows, j.nsheds, j.roi, j.intervis,
                                             site_local_limit(j.nrows, j.nsheds, j.roi, j.intervis,
                                                              j.nblocks));
   a.local_words = (int)((kLocalSmem - sizeof(LocalShared)) / 8);

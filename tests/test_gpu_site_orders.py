@@ -57,10 +57,11 @@ def test_an_unknown_order_is_refused(native):
 
 
 @pytest.mark.parametrize("n, roi, count, local", [
-    (460, 19, 4096, True), (460, 19, 4095, False), (451, 19, 4096, False), (452, 12, 10000, True),
+    (460, 19, 4096, True), (460, 19, 4095, False), (450, 19, 4096, False), (454, 28, 4096, True),
+    (454, 29, 4096, False), (452, 12, 10000, True),
     (440, 12, 10000, False), (200, 3, 5000, True), (600, 3, 4500, True), (800, 3, 4500, False)])
 def test_the_line_for_observers_in_no_block_order(native, oracle, n, roi, count, local):
-    """Intervis, one block: 180 circles on the raster, the share of cells, the bins' size."""
+    """Intervis, one block: 80 circles on the raster, the share of cells, the bins' size."""
     side = int(np.ceil(np.sqrt(count)))
     i = np.arange(count)
     jitter = np.random.default_rng(n).random((2, count)) * 0.9
