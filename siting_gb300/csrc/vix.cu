@@ -41,8 +41,10 @@ namespace {
 // Staged samples of the far form.
 constexpr int kFarNear = 7;
 
-// The whole halo staged, the cells near the tile, or the tile alone.
-constexpr int kStagedForm = 0, kFarForm = 1, kBareForm = 2, kForms = 3;
+// The whole halo staged, also for radii up to 8 (a kernel of its own: as one more case of the
+// samples it costs radii up to 32 3%), the cells near the tile, or the tile alone.
+constexpr int kStagedForm = 0, kSmallForm = 1, kFarForm = 2, kBareForm = 3, kForms = 4;
+constexpr int kSmallRoi = 8;
 
 struct VixArgs {
   const uint16_t *dem;
@@ -286,7 +288,7 @@ __device__ __forceinline__ void vix_tile(const CUtensorMap *map, const VixArgs &
   }
   auto work = [&](auto near) {
     constexpr int kNear = decltype(near)::value;
-    constexpr bool kFar = kForm != kStagedForm;
+    constexpr bool kFar = kForm == kFarForm || kForm == kBareForm;
     if (interior)
       vix_tile_work<kNear, kFar, true>(a, halo, tx0, ty0, hx0, hy0, jump, rtab, vtab);
     else
@@ -296,12 +298,13 @@ __device__ __forceinline__ void vix_tile(const CUtensorMap *map, const VixArgs &
     work(std::integral_constant<int, 0>());
   } else if constexpr (kForm == kFarForm) {
     work(std::integral_constant<int, kFarNear>());
-  } else {  // the fewest samples that reach offsets below roi
+  } else if constexpr (kForm == kSmallForm) {
     if (a.roi <= 2)
       work(std::integral_constant<int, 1>());
-    else if (a.roi <= 8)
+    else
       work(std::integral_constant<int, 3>());
-    else if (a.roi <= 32)
+  } else {  // the fewest samples that reach offsets below roi
+    if (a.roi <= 32)
       work(std::integral_constant<int, 5>());
     else if (a.roi <= 64)
       work(std::integral_constant<int, 6>());
@@ -384,7 +387,10 @@ size_t tables_tail_bytes(int roi, int ntests) {
   return 16 + (size_t)ntests * 8 + (size_t)(roi + 1) * 4 + ntests + 1;
 }
 
-int vix_form(const VixPlan &p) { return p.use_smem ? kStagedForm : p.bare ? kBareForm : kFarForm; }
+int vix_form(const VixPlan &p, int roi) {
+  if (p.use_smem) return roi <= kSmallRoi ? kSmallForm : kStagedForm;
+  return p.bare ? kBareForm : kFarForm;
+}
 
 int plan_halo(const VixPlan &p, int roi) { return p.use_smem ? roi : p.bare ? 0 : kFarHalo; }
 
@@ -514,10 +520,11 @@ cudaError_t launch_vix(const DemView &dem, int roi, int oht, int tht, int ntests
     return cudaErrorInvalidValue;
   const size_t shm = vix_smem_bytes(plan, roi, ntests);
   const int grid = a.tiles_per_row * a.tiles_per_row;
-  const int form = vix_form(plan);
-  auto kern = form == kStagedForm ? vix_kernel<kStagedForm>
-              : form == kFarForm  ? vix_kernel<kFarForm>
-                                  : vix_kernel<kBareForm>;
+  const int form = vix_form(plan, roi);
+  auto kern = form == kStagedForm  ? vix_kernel<kStagedForm>
+              : form == kSmallForm ? vix_kernel<kSmallForm>
+              : form == kFarForm   ? vix_kernel<kFarForm>
+                                   : vix_kernel<kBareForm>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
   if (e != cudaSuccess) return e;
   kern<<<grid, plan.threads, shm, st>>>(map, a);
@@ -537,7 +544,7 @@ cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st) {
         const StageJob &J = jobs[j];
         VixQJob &q = tab.jobs[tab.njobs];
         memset(&q, 0, sizeof(q));
-        if (vix_form(J.vplan) != kind) continue;
+        if (vix_form(J.vplan, J.roi) != kind) continue;
         if (!vix_args(J.dem, J.roi, J.oht, J.tht, J.ntests, J.vix, J.vix_tables, J.vplan, J.err,
                       &q.a, &q.map))
           return cudaErrorInvalidValue;
@@ -547,9 +554,10 @@ cudaError_t launch_vix_queue(const StageJob *jobs, int njobs, cudaStream_t st) {
         tab.njobs++;
       }
       if (!tab.njobs) continue;
-      auto kern = kind == kStagedForm ? vixq_kernel<kStagedForm>
-                  : kind == kFarForm  ? vixq_kernel<kFarForm>
-                                      : vixq_kernel<kBareForm>;
+      auto kern = kind == kStagedForm  ? vixq_kernel<kStagedForm>
+                  : kind == kSmallForm ? vixq_kernel<kSmallForm>
+                  : kind == kFarForm   ? vixq_kernel<kFarForm>
+                                       : vixq_kernel<kBareForm>;
       cudaError_t e =
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
       if (e != cudaSuccess) return e;
