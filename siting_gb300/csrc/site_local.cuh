@@ -74,8 +74,11 @@ constexpr int kLocalSearch = (1 << kLocalSeenLog) + kLocalQueue + 64;  // words
 constexpr int kLocalShareMin = 2, kLocalShare = 16;
 constexpr int kLocalStride = 7919;   // order of a pick's candidates
 constexpr int kLocalLook = 12;       // 32s of bins within reach: at most 19 a side
-// Picks whose order is found by comparing each with all, and buckets for more of them.
-constexpr int kLocalDirect = 1024, kLocalBuckets = 4096;
+// Picks whose order is found by comparing each with all in shared memory, without and with
+// intervis, and buckets for more of them (thousand cycles so and by buckets: 4500 picks of
+// 2458^2, radius 26, without 76, 180; 2500 of 4096^2, radius 100, with 460, 50; 16384
+// buckets 152 and 122, for their sums).
+constexpr int kLocalDirect = 8192, kLocalDirectChains = 1024, kLocalBuckets = 4096;
 
 // Bins: side (cells of the DEM) and count a side.
 __host__ __device__ __forceinline__ int local_bin_side(int n, int roi) {
@@ -544,12 +547,19 @@ __device__ __forceinline__ void local_order(const SiteArgs &a, LocalShared &s, G
     const unsigned long long first = __ldcg(base + b);
     const int y0 = (int)(first >> 32), y1 = y0 + (int)(__ldcg(sum + b) >> 32);
     unsigned above = (unsigned)y0, before = (unsigned)first;
+    int same = 0;
+#pragma unroll 8
     for (int j = y0; j < y1; j++) {
       const ulonglong2 o = sorted[j];
-      bool ahead = o.x > me.x;
-      if (iv && o.x == me.x && j != i)
-        ahead = chain_before(L.plist, L.pparent, ~0ull, which[j], ~0ull, x);
-      if (ahead) {
+      above += o.x > me.x;
+      before += o.x > me.x ? (unsigned)(o.y >> 32) : 0u;
+      same += o.x == me.x;
+    }
+    for (int j = y0; same > 1 && j < y1; j++) {  // of one level (intervis): by their chains
+      const ulonglong2 o = sorted[j];
+      if (o.x != me.x || j == i) continue;
+      same--;
+      if (chain_before(L.plist, L.pparent, ~0ull, which[j], ~0ull, x)) {
         above++;
         before += (unsigned)(o.y >> 32);
       }
@@ -1065,7 +1075,7 @@ __device__ __forceinline__ void site_local(const SiteArgs &a, LocalShared &s, in
       area += mine >> 32;
     }
   };
-  if (np <= kLocalDirect) {  // against all picks, in shared memory
+  if (np <= (iv ? kLocalDirectChains : kLocalDirect)) {  // against all picks, in shared memory
     unsigned long long *key = reinterpret_cast<unsigned long long *>(N), *reach = key + np;
     int *parent = reinterpret_cast<int *>(reach + np);
     for (int i = tid; i < np; i += T) {

@@ -80,11 +80,12 @@ def test_the_line_for_observers_in_no_block_order(native, oracle, n, roi, count,
     assert (res.nusedsheds, res.cumarea) == (used, area)
 
 
-@pytest.mark.parametrize("n, roi, count, top", [(700, 3, 6000, 6000), (1600, 35, 4000, 9000), (330, 1, 20000, 1),
+@pytest.mark.parametrize("n, roi, count, top", [(700, 3, 6000, 6000), (1000, 3, 9000, 6000), (1600, 35, 4000, 9000), (330, 1, 20000, 1),
                                                 (900, 12, 9000, 3000), (520, 4, 1030, 6000)])
 @pytest.mark.parametrize("intervis", [0, 1])
 def test_the_order_of_many_picks(native, oracle, n, roi, count, top, intervis):
-    """More than 1024 picks are put in order by buckets: small and large areas, equal ones."""
+    """More than 8192 picks, 1024 with intervis, are put in order by buckets: small and large
+    areas, equal ones."""
     dem = native.fbm_dem(n, seed=n, octaves=7, range_max=top)
     obs = np.random.default_rng(n).integers(0, n * n, count).astype(np.int32)
     sheds = oracle.sheds(dem, n, roi, 3, 3, obs)
