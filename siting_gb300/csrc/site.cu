@@ -1218,14 +1218,16 @@ long long site_stop_area(int nrows) {
 }
 
 // Without intervis local dominance pays by the picks that a round finds, so the raster
-// has to hold several of a candidate's circles: 30, 8 from 400 candidates on, 3 from 2048.
-// Its passes over all bins cost what a hundredth of the bins in candidates, and 128, are
-// worth.  820 jobs and calls of 32 to 20 000 candidates, radius 4 to 200: these lines take
-// 1.006 times the better order's time in the mean.  Ms in the global order and by local
+// has to hold several of a candidate's circles: 16, 8 from 400 candidates on, 3 from 2048.
+// Its passes over all bins cost what a 300th of the bins in candidates, and 128, are
+// worth.  820 jobs and calls of 32 to 20 000 candidates that lie anywhere, radius 4 to 200,
+// take 1.01 times the better order's time in the mean within these lines, and 262 jobs
+// whose observers lie in heaps in large blocks 1.01.  Ms in the global order and by local
 // dominance: 50 circles 351^2, radius 28, 225 candidates 0.62, 0.44; 10 circles 612^2, 107,
 // 1236 0.34, 0.29; 5 circles 736^2, 179, 4232 0.82, 0.90 and 686^2, 179, 7396 0.63, 0.59; 19
-// circles 1301^2, 170, 399 1.76, 2.24; 2 circles 485^2, 174, 1125 0.24, 0.30; 200 bins a
-// candidate 913^2, 17, 160 0.22, 0.31; 60 candidates 386^2, 7 0.08, 0.21.
+// circles 1301^2, 170, 399 1.76, 2.24 and 409^2, 51, 338 0.36, 0.23; 2 circles 485^2, 174,
+// 1125 0.24, 0.30; 200 bins a candidate 913^2, 17, 160 anywhere 0.22, 0.31 and 1322^2, 11, 288
+// in heaps 0.94, 0.30; 60 candidates 386^2, 7 0.08, 0.21.
 //
 // With intervis a round also searches for the
 // candidates that its picks would uncover (B2).  That pays where many regions are
@@ -1261,8 +1263,8 @@ double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblock
   if (!local_width(roi)) return 0;
   if (!intervis) {
     const double bins = (double)local_bins(nrows, roi) * local_bins(nrows, roi);
-    if (nsheds < 128 || bins > 100.0 * nsheds) return 0;
-    return nsheds / (nsheds >= 2048 ? 3.0 : nsheds >= 400 ? 8.0 : 30.0);
+    if (nsheds < 128 || bins > 300.0 * nsheds) return 0;
+    return nsheds / (nsheds >= 2048 ? 3.0 : nsheds >= 400 ? 8.0 : 16.0);
   }
   const double twentieth = 3.14159 * roi * roi / 20;
   if (nsheds >= 16384) return std::max(64.0, std::min(512.0, twentieth));
@@ -1273,16 +1275,20 @@ double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblock
   return nblocks <= 1 && nsheds >= 4096 && spread && fine ? 64 : 0;
 }
 
-// The most pairs of candidates in one bin, each counted twice: nsheds times the candidates
-// that one shares its bin with in the mean.  Crowded is what has more in a circle than the
-// line allows, without intervis a twelfth of all, and half as many again as anywhere at
-// random (20 000 candidates about one place of 1000^2, radius 20, with a 25th, a 12th and a
-// 6th of all in a circle: 1.45, 1.31 and 1.39 ms against 2.31, 1.56 and 1.23).
-unsigned long long site_max_near(int nrows, int nsheds, int roi, int intervis, double limit) {
-  const double circle = 3.14159 * roi * roi / ((double)nrows * nrows) * nsheds;
-  limit = std::max(intervis ? limit : std::min(limit, nsheds / 12.0), 1.5 * circle);
-  const double side = local_bin_side(nrows, roi);
-  return (unsigned long long)(limit * nsheds * side * side / (3.14159 * roi * roi));
+// The most pairs of candidates in one bin, each counted twice.  Candidates on their own
+// share a bin with few; those in heaps are as if they lay evenly in nsheds^2 / (nsheds +
+// pairs) bins, and a round finds what that many bins hold.  That has to be 120 bins, 500
+// with intervis.  Local dominance takes these shares of the global order's time in the mean:
+//   bins                         to 70   120   200   350   600   1200   3000   more
+//   jobs, blocks of 8 to 600^2           0.9   0.7   0.65  0.56  0.31 (246)
+//   candidates in 1 to 60 heaps   2.0    1.5   1.24  1.06  0.87  0.56 (6150)
+//   with intervis, jobs                                          0.60   0.59   0.27 (130)
+//   with intervis, in heaps                          1.23  1.07  0.87   0.74   0.50 (380)
+// (1016^2, radius 11, 18 576 in blocks of 84^2, intervis: 4775 bins, 2.5 ms against 20.4;
+// 312^2, radius 41, 400 in blocks of 32^2, without: the job 0.39 ms against 0.46).
+unsigned long long site_max_near(int nsheds, int intervis) {
+  const double least = intervis ? 500 : 120;
+  return (unsigned long long)(nsheds * std::max(0.0, nsheds / least - 1));
 }
 
 }  // namespace
@@ -1510,9 +1516,7 @@ SiteArgs make_site_args(const SiteJob &j, int block0) {
   a.local = j.scratch.local;
   a.use_local = j.local != 0;
   a.max_near = j.local == 2 ? kBeyond - 1
-                            : site_max_near(j.nrows, j.nsheds, j.roi, j.intervis,
-                                            site_local_limit(j.nrows, j.nsheds, j.roi, j.intervis,
-                                                             j.nblocks));
+                            : site_max_near(j.nsheds, j.intervis);
   a.local_words = (int)((kLocalSmem - sizeof(LocalShared)) / 8);
   return a;
 }

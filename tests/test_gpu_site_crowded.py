@@ -20,7 +20,7 @@ def _observers(n, count, spread, seed):
 
 
 @pytest.mark.parametrize("n, roi, count, intervis, spread, crowded", [
-    (400, 6, 1500, 0, np.inf, False), (400, 6, 1500, 0, 8, True), (400, 6, 1500, 0, 0, True),
+    (400, 6, 1500, 0, np.inf, False), (400, 6, 1500, 0, 4, True), (400, 6, 1500, 0, 0, True),
     (500, 5, 5000, 1, np.inf, False), (500, 5, 5000, 1, 12, True), (600, 8, 17000, 1, np.inf, False),
     (600, 8, 17000, 1, 15, True), (90, 1, 400, 0, 0, True), (300, 70, 1200, 0, 3, None),
 ])
