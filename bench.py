@@ -323,7 +323,7 @@ NCU_TRAFFIC = {
 # were measured with.
 ISSUE_WORK = {
     ("vix", 100, 100): (1.739e9 / (2048 * 2048 * 100), "target"),
-    ("viewshed", 100, 100): (8.885e8 / 16384, "observer"),
+    ("viewshed", 100, 100): (8.911e8 / 16384, "observer"),
 }
 ISSUE_SLOTS_PER_SM = 4  # one warp instruction per cycle from each SM sub-partition
 

@@ -71,7 +71,9 @@ typedef struct siting_plan {
   int shed_smem;    /* VIEWSHED window staged by TMA: 1 in halves or quarters, a
                        CTA each, 2 whole in one CTA (as 1 above roi 111), 0 the
                        window read through L1, -1 default (2 below roi 75, else
-                       1; both read through L1 where a quarter does not fit) */
+                       1, read through L1 where a quarter does not fit, from
+                       radius 304, where the DEM is at most 1.25 radii wide
+                       and, with observers for every SM, from radius 209) */
   int site_ctas;    /* CTAs of the job's SITE group (0 = default) */
 } siting_plan;
 

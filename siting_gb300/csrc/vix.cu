@@ -447,7 +447,8 @@ size_t vix_smem_bytes(const VixPlan &p, int roi, int ntests) {
 // two CTAs share an SM, then 16x16 (four threads a cell), whose halo takes
 // longer to load for a quarter of the cells: 2048^2, roi 96, staged 16x16 takes
 // 0.32 ms + 12.2 us a target, 32x32 with the near window alone 0.04 ms + 16.1
-// us, so few targets take the far form.  64x64 tiles (four cells a thread)
+// us, so few targets take the far form (16x16 over it at 64 and 72 targets: 1024^2, radius
+// 100, 1.00, 0.97; 2001^2, 105, 1.01, 0.99; 3000^2, 110, 1.01, 0.99).  64x64 tiles (four cells a thread)
 // never won.  A grid of 32x32 tiles that is not two waves of the SMs' CTA
 // pairs leaves SMs idle: 16x16 tiles then (us at 32 and 16, 256^2 roi 20: 23,
 // 15; 400^2 roi 200: 100, 69; 700^2 roi 200: 198, 176; 1000^2 roi 50: 187, 207),
