@@ -266,7 +266,7 @@ int site_enqueue(siting_ctx *ctx, int nrows, int roi, int intervis, int nsheds,
     return fail(ctx, SITING_EINVAL, "SITE: shared-memory plan exceeds 220 KB");
   void *p;
   int local = ctx->site_order == kOrderLocal ? 2 * site_may_be_local(roi)
-              : ctx->site_order == kOrderAuto && site_is_local(nrows, nsheds, roi, intervis, nb);
+              : ctx->site_order == kOrderAuto && site_is_local(nrows, nsheds, roi, intervis, nb, G);
   SiteScratch s;
   int rc = site_scratch_get(ctx, nrows, nsheds, G, roi, intervis, &local, &p, &s);
   if (rc) return rc;

@@ -156,7 +156,7 @@ int plan_batch(int sm_count, int njobs, const siting_params *params, const sitin
     J.o_tab = tab_bytes;
     tab_bytes += align256(vix_table_bytes(J.p.roi, J.p.ntests));
     J.o_site = ws;
-    J.local = !lean && site_is_local(J.n, J.g.nwanted, J.p.roi, J.p.intervis, J.g.nblocks);
+    J.local = !lean && site_is_local(J.n, J.g.nwanted, J.p.roi, J.p.intervis, J.g.nblocks, J.G);
     ws += align256(site_scratch_bytes(J.n, J.g.nwanted, J.G, J.p.roi, J.p.intervis, J.local));
     J.o_err = ws;
     ws += 256;

@@ -164,7 +164,7 @@ cudaError_t launch_site_jobs(const SiteJob *jobs, int njobs, void *d_table, void
 // Whether a job can be selected by local dominance, and is faster so than in the global
 // key order.
 bool site_may_be_local(int roi);
-bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks);
+bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks, int nctas);
 size_t site_scratch_bytes(int nrows, int nsheds, int nctas, int roi, int intervis, bool local);
 void site_carve_scratch(void *base, int nrows, int nsheds, int nctas, int roi, int intervis,
                         bool local, SiteScratch *s);

@@ -1228,6 +1228,11 @@ long long site_stop_area(int nrows) {
 // circles 1301^2, 170, 399 1.76, 2.24 and 409^2, 51, 338 0.36, 0.23; 2 circles 485^2, 174,
 // 1125 0.24, 0.30; 200 bins a candidate 913^2, 17, 160 anywhere 0.22, 0.31 and 1322^2, 11, 288
 // in heaps 0.94, 0.30; 60 candidates 386^2, 7 0.08, 0.21.
+// In a narrow group (batches) the global order's rounds wait for the owners of a pick's
+// neighbours, so fewer circles do between 8 and 32 CTAs, and any up to 8: of 806 jobs of
+// 250^2 to 1200^2, radius 15 to 200, those of at most one circle took 1.68, 1.48, 1.23, 0.98
+// and 0.86 times as long in the global order with 2, 4, 8, 16 and 24 CTAs, those of two to
+// four 1.66, 1.57, 1.41, 1.21 and 1.09.
 //
 // With intervis a round also searches for the
 // candidates that its picks would uncover (B2).  That pays where many regions are
@@ -1258,13 +1263,16 @@ long long site_stop_area(int nrows) {
 // job to the global order.
 namespace {
 
+// The share of the lines without intervis that holds for a group.
+double site_narrow(int nctas) { return std::max(0.01, std::min(1.0, (nctas - 8) / 24.0)); }
+
 // The most candidates in a pick's circle that local dominance is used for.
-double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblocks) {
+double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblocks, int nctas) {
   if (!local_width(roi)) return 0;
   if (!intervis) {
     const double bins = (double)local_bins(nrows, roi) * local_bins(nrows, roi);
     if (nsheds < 128 || bins > 300.0 * nsheds) return 0;
-    return nsheds / (nsheds >= 2048 ? 3.0 : nsheds >= 400 ? 8.0 : 16.0);
+    return nsheds / ((nsheds >= 2048 ? 3.0 : nsheds >= 400 ? 8.0 : 16.0) * site_narrow(nctas));
   }
   const double twentieth = 3.14159 * roi * roi / 20;
   if (nsheds >= 16384) return std::max(64.0, std::min(512.0, twentieth));
@@ -1277,8 +1285,8 @@ double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblock
 
 // The most pairs of candidates in one bin, each counted twice.  Candidates on their own
 // share a bin with few; those in heaps are as if they lay evenly in nsheds^2 / (nsheds +
-// pairs) bins, and a round finds what that many bins hold.  That has to be 120 bins, 500
-// with intervis.  Local dominance takes these shares of the global order's time in the mean:
+// pairs) bins, and a round finds what that many bins hold.  That has to be 120 bins (in
+// a narrow group fewer), 500 with intervis.  Local dominance takes these shares of the global order's time in the mean:
 //   bins                         to 70   120   200   350   600   1200   3000   more
 //   jobs, blocks of 8 to 600^2           0.9   0.7   0.65  0.56  0.31 (246)
 //   candidates in 1 to 60 heaps   2.0    1.5   1.24  1.06  0.87  0.56 (6150)
@@ -1286,8 +1294,8 @@ double site_local_limit(int nrows, int nsheds, int roi, int intervis, int nblock
 //   with intervis, in heaps                          1.23  1.07  0.87   0.74   0.50 (380)
 // (1016^2, radius 11, 18 576 in blocks of 84^2, intervis: 4775 bins, 2.5 ms against 20.4;
 // 312^2, radius 41, 400 in blocks of 32^2, without: the job 0.39 ms against 0.46).
-unsigned long long site_max_near(int nsheds, int intervis) {
-  const double least = intervis ? 500 : 120;
+unsigned long long site_max_near(int nsheds, int intervis, int nctas) {
+  const double least = intervis ? 500 : 120 * site_narrow(nctas);
   return (unsigned long long)(nsheds * std::max(0.0, nsheds / least - 1));
 }
 
@@ -1295,9 +1303,9 @@ unsigned long long site_max_near(int nsheds, int intervis) {
 
 bool site_may_be_local(int roi) { return local_width(roi); }
 
-bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks) {
+bool site_is_local(int nrows, int nsheds, int roi, int intervis, int nblocks, int nctas) {
   const double circle = 3.14159 * roi * roi / ((double)nrows * nrows) * nsheds;
-  return circle <= site_local_limit(nrows, nsheds, roi, intervis, nblocks);
+  return circle <= site_local_limit(nrows, nsheds, roi, intervis, nblocks, nctas);
 }
 
 namespace {
@@ -1516,7 +1524,7 @@ SiteArgs make_site_args(const SiteJob &j, int block0) {
   a.local = j.scratch.local;
   a.use_local = j.local != 0;
   a.max_near = j.local == 2 ? kBeyond - 1
-                            : site_max_near(j.nsheds, j.intervis);
+                            : site_max_near(j.nsheds, j.intervis, j.nctas);
   a.local_words = (int)((kLocalSmem - sizeof(LocalShared)) / 8);
   return a;
 }
@@ -1697,7 +1705,7 @@ extern "C" int siting_site_it_noalloc(int nrows, int roi, int intervis, int nshe
   auto need_of = [&](bool local) {  // + error flag
     return site_scratch_bytes(nrows, nsheds, G, roi, intervis, local) + 256;
   };
-  const bool local = site_is_local(nrows, nsheds, roi, intervis, 1) && need_of(true) <= kNoAllocScratchBytes;
+  const bool local = site_is_local(nrows, nsheds, roi, intervis, 1, G) && need_of(true) <= kNoAllocScratchBytes;
   const size_t need = need_of(local);
   if (need > kNoAllocScratchBytes) return SITING_ENOMEM;  // beyond the 16 MiB array
   void *base = nullptr;

@@ -143,7 +143,7 @@ extern "C" int siting_autotune(siting_ctx *ctx, const siting_params *p, const ui
               220 * 1024)
         continue;
       void *sp;
-      int local = site_is_local(n, g.nwanted, p->roi, p->intervis, g.nblocks);
+      int local = site_is_local(n, g.nwanted, p->roi, p->intervis, g.nblocks, G);
       SiteScratch s;
       if ((rc = site_scratch_get(ctx, n, g.nwanted, G, p->roi, p->intervis, &local, &sp, &s))) return rc;
       float t;

@@ -98,3 +98,19 @@ def test_the_order_of_many_picks(native, oracle, n, roi, count, top, intervis):
             assert np.array_equal(ctx.last_pick_order(count), order), f"{ctas} CTAs"
         assert np.array_equal(sel, want)
         assert (res.nusedsheds, res.cumarea) == (used, area)
+
+
+@pytest.mark.parametrize("ctas, local", [(4, True), (8, True), (32, False), (0, False)])
+def test_the_line_for_narrow_groups(native, oracle, ctas, local):
+    """Two circles on the raster: a group of few CTAs goes by local dominance."""
+    n, roi, count = 300, 120, 1100
+    dem = native.fbm_dem(n, seed=5, octaves=7, range_max=9000)
+    obs = np.random.default_rng(5).integers(0, n * n, count).astype(np.int32)
+    sheds = oracle.sheds(dem, n, roi, 20, 20, obs)
+    want, used, area, order = oracle.site(n, roi, 0, obs, sheds, want_order=True)
+    with native.Context(0) as ctx:
+        ctx.set_site_ctas(ctas)
+        sel, res = ctx.site_it(n, roi, 0, obs, sheds)
+        assert np.array_equal(ctx.last_pick_order(count), order)
+        assert (ctx.last_site_phase_cycles()[12] == 0) == local
+    assert np.array_equal(sel, want) and (res.nusedsheds, res.cumarea) == (used, area)
