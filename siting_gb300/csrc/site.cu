@@ -65,7 +65,7 @@ constexpr int kMaxSlots = 4096;  // candidates owned by one CTA
 // rounds with 3, 4, 6 or 8), and fewer keys make each merge cheaper.
 constexpr int kTopK = 3;
 constexpr int kFewKeys = 256;     // published keys that one warp orders
-constexpr int kFewPicks = 4;      // where the round before took at most so many picks
+constexpr int kFewPicks = 8;      // where the round before took at most so many picks
 constexpr int kMaxPicks = 64;    // picks accepted in one round at most
 constexpr int kSmallRecip = 128; // reciprocals tabled in shared memory (>= kMaxPicks)
 constexpr int kMaxPairs = 8192;  // (candidate, pick) pairs one CTA updates per round
@@ -223,7 +223,9 @@ __global__ void __launch_bounds__(256) site_score_kernel(const uint64_t *sheds, 
 // 1741^2, 23 762 3.33, 3.16).  A pick costs a turn, so rounds of many are ranked: sparse
 // candidates give 30 and more (of 140 jobs, the 65 with more than 100 circles on the raster
 // took 1.01 times their time before this form where every round took it by turns up to 12
-// picks, 1.07 with no such limit, and 1.00 with a limit of 4; the other 75 0.96 in each).
+// picks, 1.07 with no such limit, and 1.00 with a limit of 4; the other 75 0.96 in each.
+// With limits of 4 and 8, intervis: 256^2, radius 20, 146 picks 0.633, 0.628; 512^2, 38, 206
+// 1.012, 1.005; 300^2, 10, 801 2.267, 2.281).
 // A function of its own: inside the round's loop its code
 // costs the larger jobs 2-4%.  Returns the number of picks and, from bit 8 on, that at
 // the 95% stop plus one.
